@@ -55,23 +55,23 @@ MAX_REQUESTS = 64
 def listed() -> list[dict]:
     return [
         # A chat turn for one user: a short prompt, an answer token by token.  Latency and launches are all there is.
-        _case("chat, one request", "generate", "tinyllama", requests=1, shortest=57, longest=57, new=32),
+        _case("chat", "generate", "tinyllama", requests=1, shortest=57, longest=57, new=32),
         # The benchmark's headline: eight requests of 1,024 tokens each decode together.
         _case("eight requests", "generate", "tinyllama", requests=8, shortest=1024, longest=1024, new=64),
         # A full batch of short dialogues, sampled with the usual temperature and top-p.
-        _case("full batch, sampled", "generate", "tinyllama", requests=64, shortest=90, longest=310, new=32, temperature=0.8, top_p=0.95),
+        _case("full batch sampled", "generate", "tinyllama", requests=64, shortest=90, longest=310, new=32, temperature=0.8, top_p=0.95),
         # A wider model with a cache entry per head, two users.
-        _case("two requests, 7B widths", "generate", "llama2-7b", requests=2, shortest=333, longest=500, new=32),
+        _case("two requests at 7B", "generate", "llama2-7b", requests=2, shortest=333, longest=500, new=32),
         # A server's middling batch on the widest model, texts of different lengths.
-        _case("batch of 24, 8B widths", "generate", "llama3-8b", requests=24, shortest=150, longest=1100, new=24),
+        _case("batch of 24 at 8B", "generate", "llama3-8b", requests=24, shortest=150, longest=1100, new=24),
         # Questions over long documents: the cache is a large part of what a decode step reads.
-        _case("long documents, 8B widths", "generate", "llama3-8b", requests=4, shortest=3500, longest=4001, new=48, temperature=0.7, top_p=0.9),
+        _case("long documents at 8B", "generate", "llama3-8b", requests=4, shortest=3500, longest=4001, new=48, temperature=0.7, top_p=0.9),
         # The first token of a short question: the smallest call, mostly launches.
         _case("short prompt", "prompt", "tinyllama", requests=1, shortest=150, longest=150),
         # The first token after a whole context of prompt.
-        _case("prompt of 2,048", "prompt", "tinyllama", requests=1, shortest=2048, longest=2048),
+        _case("prompt of 2048", "prompt", "tinyllama", requests=1, shortest=2048, longest=2048),
         # A whole context of prompt on the widest model: the largest call.
-        _case("prompt of 8,192, 8B widths", "prompt", "llama3-8b", requests=1, shortest=8192, longest=8192),
+        _case("prompt of 8192 at 8B", "prompt", "llama3-8b", requests=1, shortest=8192, longest=8192),
         # How well a few texts are predicted: logits at every place.
         _case("scored texts", "score", "tinyllama", requests=3, shortest=201, longest=420),
         # A serving run through the engine's own scheduler.
