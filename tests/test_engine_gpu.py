@@ -10,6 +10,7 @@ import tiny_configs
 import trace_tools
 from tinyllama_inference_engine_b200 import EngineConfig
 from tinyllama_inference_engine_b200.engine.api import Engine
+from tinyllama_inference_engine_b200.engine.batch import StepEntry
 from tinyllama_inference_engine_b200.engine.request import SamplingParams
 from tinyllama_inference_engine_b200.engine.runner import ModelRunner
 
@@ -276,3 +277,25 @@ def test_step_shapes_that_repeat_are_replayed_as_graphs(model_folders, dtype, fr
     assert worst <= fraction, worst
     graphs = [slot for slot in runner._step_graphs.values() if slot.graph is not None]
     assert len(graphs) == 3 and all(slot.uses >= 4 for slot in graphs)
+
+
+def test_steps_of_one_shape_queued_without_waiting_keep_their_own_descriptions(model_folders):
+    """A program that reads no logits runs ahead of the device; the pinned description of a replayed shape must not be overwritten under a queued copy."""
+    runner = _engine(model_folders["b"], use_cuda_graphs=True).runner
+    prompts = _prompts(runner.spec.vocab_size, [40] * 7, seed=9)
+
+    def logits(wait):
+        got = []
+        for index, prompt in enumerate(prompts):
+            got.append(runner.step([StepEntry(f"r{index}", prompt, [39])]))
+            if wait:
+                torch.cuda.synchronize()
+        for index in range(len(prompts)):
+            runner.finish(f"r{index}")
+        return got
+
+    want = logits(wait=True)      # from the third on these are replays of one graph
+    torch.cuda._sleep(200_000_000)   # about a tenth of a second: the device is behind the host for the whole run
+    got = logits(wait=False)
+    for index, (a, b) in enumerate(zip(got, want)):
+        assert torch.equal(a, b), index

@@ -33,6 +33,7 @@ class GraphedStep:
         self.uses = 0
         self.host: torch.Tensor | None = None
         self.device: torch.Tensor | None = None
+        self.copied: torch.cuda.Event | None = None   # the description's last copy to the device
         self.graph: torch.cuda.CUDAGraph | None = None
         self.logits: torch.Tensor | None = None
 
@@ -41,7 +42,12 @@ class GraphedStep:
             words = len(lay_out_step(entries, firsts, slots, table_rows)["flat"])
             self.host = torch.zeros(words, dtype=torch.int32).pin_memory()
             self.device = torch.zeros(words, dtype=torch.int32, device=runner.device)
+            self.copied = torch.cuda.Event()
+        # The host may be steps ahead of the device (nothing reads a prompt portion without wanted logits): the pinned buffer
+        # is written again only once the copy that a step before this one queued from it has been done.
+        self.copied.synchronize()
         ctx = pack_step(entries, firsts, slots, table_rows, runner.device, into=(self.host, self.device))
+        self.copied.record()
         # launch shapes chosen from the context length must hold for every later step of this shape
         ctx.max_seq_len = runner.spec.max_positions
         if self.graph is not None:
