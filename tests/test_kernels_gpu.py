@@ -127,6 +127,27 @@ def test_gemm_fp32_is_true_32_bit(ops, M, N, K):
     assert torch.equal(alone[0], got[M - 1])
 
 
+@pytest.mark.parametrize("N,K", [(64, 128), (130, 516), (2049, 260), (16, 4)])
+def test_gemm_fp32_gives_a_row_the_same_bits_in_every_kernel(ops, N, K):
+    """The streaming kernels (1, 2, 4, 8, 16 rows), the three register tiles and the plain one (an unaligned operand) around their edges."""
+    torch.manual_seed(33)
+    x, w = torch.randn(900, K).cuda(), torch.randn(N, K).cuda()
+    full = torch.empty(900, N, device="cuda")
+    ops.linear(x, w, full)
+    # one rounding per multiply-add of a sum of K terms
+    bound = K * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    assert bool(((full.double() - x.double() @ w.double().T).abs() <= bound).all())
+    for M in (1, 2, 3, 4, 5, 8, 9, 16, 17, 31, 33, 64, 65, 129, 300):
+        got = torch.full((M, N), float("nan"), device="cuda")
+        ops.linear(x[7 : 7 + M], w, got)
+        assert torch.equal(got, full[7 : 7 + M]), M
+    wide = torch.randn(40, K + 1).cuda()   # rows one element apart from 16-byte alignment: the plain kernel
+    wide[:, :K] = x[:40]
+    got = torch.empty(40, N, device="cuda")
+    ops.linear(wide[:, :K], w, got)
+    assert torch.equal(got, full[:40])
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 256, 64), (37, 136, 80), (130, 72, 520), (64, 2048, 2048)])
 def test_linear_bf16(ops, M, N, K):
     torch.manual_seed(4)
