@@ -294,6 +294,33 @@ def test_argmax_and_sampling(ops):
     assert float((freq - expect).abs().max()) < 0.03
 
 
+@pytest.mark.parametrize("q_heads,kv_heads,head_dim,page_size", [(8, 1, 64, 64), (4, 4, 64, 16), (6, 2, 128, 32), (24, 2, 64, 16), (32, 1, 128, 16)])
+def test_paged_attention_f32_over_shared_keys(ops, q_heads, kv_heads, head_dim, page_size):
+    """Rows of one request and of several in a tile, lengths around 32 keys, NaN where no row looks; a row has the same bits alone and among others."""
+    torch.manual_seed(34)
+    rng = np.random.default_rng(34)
+    seq_lens, q_lens = [1, 31, 32, 33, 64, 97, 200], [1, 31, 2, 33, 1, 40, 3]
+    qkv, pages, positions, token_seq, table = _paged_case(rng, torch.float32, seq_lens, q_lens, kv_heads, head_dim, page_size, q_heads)
+    want = torch.empty(len(positions), q_heads * head_dim)
+    plain_ops.paged_attention(qkv, pages, positions, token_seq, table, want, q_heads, kv_heads, head_dim, page_size)
+    for entry, length in enumerate(seq_lens):
+        if length % page_size:
+            pages[int(table[entry, length // page_size]), :, :, length % page_size :] = float("nan")
+    args = (pages.cuda(), positions.cuda(), token_seq.cuda(), table.cuda())
+    got = torch.empty(want.shape, device="cuda")
+    ops.paged_attention(qkv.cuda(), *args, got, q_heads, kv_heads, head_dim, page_size)
+    assert torch.allclose(got.cpu(), want, atol=4e-6), float((got.cpu() - want).abs().max())
+
+    class Single:
+        decode_only = True
+
+    lasts = torch.tensor(np.cumsum(q_lens) - 1)
+    alone = torch.empty(len(lasts), want.shape[1], device="cuda")
+    ops.paged_attention(qkv[lasts].cuda(), args[0], positions[lasts].cuda(), torch.arange(len(lasts), dtype=torch.int32).cuda(), args[3], alone,
+                        q_heads, kv_heads, head_dim, page_size, batch=Single())
+    assert torch.equal(alone, got[lasts.cuda()])
+
+
 @pytest.mark.parametrize("q_heads,kv_heads,head_dim,page_size,window", [
     (32, 4, 64, 64, 0), (8, 8, 128, 64, 0), (32, 8, 128, 16, 0), (4, 2, 16, 16, 0), (6, 2, 32, 32, 0), (3, 3, 48, 16, 0),
     (16, 1, 64, 64, 0), (8, 2, 64, 32, 100), (10, 2, 80, 16, 33),

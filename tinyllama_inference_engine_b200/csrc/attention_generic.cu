@@ -13,7 +13,12 @@
 // time, with a running maximum and sum in 32-bit.  The order of operations for a row
 // depends only on the row's own position, never on the batch, so the 32-bit path gives
 // bit-identical rows however the tokens were cut into steps.
+//
+// 32-bit rows of head size 64 or 128 without a window run on a second kernel with the same order of operations: a CTA owns one
+// kv head and a run of rows, so that the query heads of the group and the neighbouring rows share every key and value,
+// which the CTA copies to shared memory 32 keys at a time while it works on the 32 before.
 #include "common.cuh"
+#include "mma_utils.cuh"
 
 namespace tlie {
 
@@ -93,6 +98,168 @@ __global__ void paged_attention_generic_kernel(const T* __restrict__ q, int q_ro
   }
 }
 
+
+// --- the 32-bit kernel over shared keys and values ------------------------------------------------------
+constexpr int kSharedWarps = 8;
+constexpr int kSharedKeys = 32;
+constexpr int kSharedStages = 3;
+
+template <int HEAD_DIM, int SLOTS>
+struct SharedAttention {
+  static constexpr int kStride = HEAD_DIM + 4;   // eight rows' 16-byte reads fall into different banks
+  static constexpr int kPlane = kSharedKeys * kStride;
+  static constexpr int kSmem = (kSharedStages * 2 * kPlane + kSharedWarps * SLOTS * HEAD_DIM) * (int)sizeof(float);
+};
+
+// A warp owns SLOTS (row, head) pairs: pair slot * 8 + warp of the CTA's `rows_per_tile` rows x group heads.  Rounding is spelled out
+// (no contraction left to the compiler), so that every build of the kernel gives a row the same bits.
+template <int HEAD_DIM, int SLOTS>
+__global__ void __launch_bounds__(kSharedWarps * 32) paged_attention_shared_f32_kernel(
+    const float* __restrict__ q, int q_row_stride, const float* __restrict__ pages, const int* __restrict__ positions, const int* __restrict__ token_seq,
+    const int* __restrict__ block_table, int table_stride, float* __restrict__ out, int tokens, int q_heads, int kv_heads, int page_size, float scale,
+    int rows_per_tile) {
+  using Shape = SharedAttention<HEAD_DIM, SLOTS>;
+  extern __shared__ __align__(16) float smem[];
+  float* qs = smem + kSharedStages * 2 * Shape::kPlane;   // [slot * 8 + warp][HEAD_DIM]
+  constexpr int kQuads = HEAD_DIM / 4, kDims = HEAD_DIM / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int group = q_heads / kv_heads;
+  const int g = blockIdx.y;
+  const int t0 = blockIdx.x * rows_per_tile, t1 = min(tokens, t0 + rows_per_tile);
+  const size_t plane = (size_t)kv_heads * page_size * HEAD_DIM;
+  const float* head_pages = pages + (size_t)g * page_size * HEAD_DIM;
+
+  int row[SLOTS], head[SLOTS], pos[SLOTS];
+#pragma unroll
+  for (int s = 0; s < SLOTS; ++s) {
+    const int pair = s * kSharedWarps + warp;
+    row[s] = t0 + pair / group;
+    head[s] = g * group + pair % group;
+    const bool live = row[s] < t1;
+    pos[s] = live ? positions[row[s]] : -1;
+    float* mine = qs + pair * HEAD_DIM;
+    for (int d = lane; d < HEAD_DIM; d += 32) mine[d] = live ? q[(size_t)row[s] * q_row_stride + (size_t)head[s] * HEAD_DIM + d] : 0.0f;
+  }
+
+  // the rows of one request at a time (a tile may reach into the next request's rows)
+  for (int first = t0; first < t1;) {
+    const int entry = token_seq[first];
+    int last = first, longest = positions[first];
+    while (last + 1 < t1 && token_seq[last + 1] == entry) longest = max(longest, positions[++last]);
+    const int* table = block_table + (size_t)entry * table_stride;
+    const int chunks = longest / kSharedKeys + 1;
+    auto copy = [&](int chunk) {
+      float* stage = smem + (chunk % kSharedStages) * 2 * Shape::kPlane;
+      for (int i = threadIdx.x; i < kSharedKeys * kQuads; i += kSharedWarps * 32) {
+        const int key = i / kQuads, d = (i % kQuads) * 4;
+        const int at = chunk * kSharedKeys + key;
+        const bool seen = at <= longest;   // keys past the last one are zeros: nobody wrote them
+        const float* source = seen ? head_pages + (size_t)table[at / page_size] * 2 * plane + (size_t)(at % page_size) * HEAD_DIM + d : pages;
+        cp_async_16(stage + key * Shape::kStride + d, source, seen);
+        cp_async_16(stage + Shape::kPlane + key * Shape::kStride + d, seen ? source + plane : pages, seen);
+      }
+    };
+    __syncthreads();   // everyone is done with the last request's stages
+    for (int c = 0; c < kSharedStages - 1; ++c) {
+      if (c < chunks) copy(c);
+      cp_async_commit();
+    }
+    bool active[SLOTS];
+    bool any = false;
+    float running_max[SLOTS], running_sum[SLOTS], acc[SLOTS][kDims];
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      active[s] = row[s] >= first && row[s] <= last;
+      any = any || active[s];
+      running_max[s] = -INFINITY;
+      running_sum[s] = 0.0f;
+#pragma unroll
+      for (int i = 0; i < kDims; ++i) acc[s][i] = 0.0f;
+    }
+    for (int c = 0; c < chunks; ++c) {
+      cp_async_wait<kSharedStages - 2>();
+      __syncthreads();
+      if (c + kSharedStages - 1 < chunks) copy(c + kSharedStages - 1);
+      cp_async_commit();
+      if (!any) continue;
+      const float* ks = smem + (c % kSharedStages) * 2 * Shape::kPlane + lane * Shape::kStride;
+      const float* vs = smem + (c % kSharedStages) * 2 * Shape::kPlane + Shape::kPlane + lane;
+      float dot[SLOTS];
+#pragma unroll
+      for (int s = 0; s < SLOTS; ++s) dot[s] = 0.0f;
+#pragma unroll 8
+      for (int i = 0; i < kQuads; ++i) {
+        const float4 k = *reinterpret_cast<const float4*>(ks + 4 * i);
+#pragma unroll
+        for (int s = 0; s < SLOTS; ++s) {
+          const float4 v = *reinterpret_cast<const float4*>(qs + (s * kSharedWarps + warp) * HEAD_DIM + 4 * i);
+          dot[s] = fmaf(v.w, k.w, fmaf(v.z, k.z, fmaf(v.y, k.y, fmaf(v.x, k.x, dot[s]))));
+        }
+      }
+      const int base = c * kSharedKeys;
+      float p[SLOTS];
+      int count = kSharedKeys;   // keys of this chunk that all of the warp's rows see
+#pragma unroll
+      for (int s = 0; s < SLOTS; ++s) {
+        const bool seen = active[s] && base + lane <= pos[s];
+        const float score = seen ? __fmul_rn(dot[s], scale) : -INFINITY;
+        const float new_max = fmaxf(running_max[s], warp_max(score));
+        const float rescale = (active[s] && base <= pos[s]) ? expf(__fsub_rn(running_max[s], new_max)) : 1.0f;
+        p[s] = seen ? expf(__fsub_rn(score, new_max)) : 0.0f;
+        running_sum[s] = __fadd_rn(__fmul_rn(running_sum[s], rescale), warp_sum(p[s]));
+        running_max[s] = new_max;
+#pragma unroll
+        for (int i = 0; i < kDims; ++i) acc[s][i] = __fmul_rn(acc[s][i], rescale);
+        count = min(count, active[s] ? pos[s] - base + 1 : 0);
+      }
+      if (count == kSharedKeys) {
+#pragma unroll 8
+        for (int j = 0; j < kSharedKeys; ++j) {
+          float v[kDims];
+#pragma unroll
+          for (int i = 0; i < kDims; ++i) v[i] = vs[j * Shape::kStride + 32 * i];
+#pragma unroll
+          for (int s = 0; s < SLOTS; ++s) {
+            const float pj = __shfl_sync(0xffffffffu, p[s], j);
+#pragma unroll
+            for (int i = 0; i < kDims; ++i) acc[s][i] = fmaf(pj, v[i], acc[s][i]);
+          }
+        }
+      } else {   // a row takes only the values it sees: what lies past it may be anything, and 0 times that is not always 0
+#pragma unroll
+        for (int s = 0; s < SLOTS; ++s) {
+          const int mine = active[s] ? min(kSharedKeys, pos[s] - base + 1) : 0;   // the same for the whole warp
+          for (int j = 0; j < mine; ++j) {
+            const float pj = __shfl_sync(0xffffffffu, p[s], j);
+#pragma unroll
+            for (int i = 0; i < kDims; ++i) acc[s][i] = fmaf(pj, vs[j * Shape::kStride + 32 * i], acc[s][i]);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      if (!active[s]) continue;
+      const float inv = 1.0f / running_sum[s];
+#pragma unroll
+      for (int i = 0; i < kDims; ++i)
+        out[(size_t)row[s] * q_heads * HEAD_DIM + (size_t)head[s] * HEAD_DIM + lane + 32 * i] = acc[s][i] * inv;
+    }
+    first = last + 1;
+  }
+}
+
+template <int HEAD_DIM, int SLOTS>
+static int launch_shared(const float* q, int q_row_stride, const float* pages, const int* positions, const int* token_seq, const int* block_table,
+                         int table_stride, float* out, int tokens, int q_heads, int kv_heads, int page_size, float scale, int rows_per_tile, cudaStream_t stream) {
+  constexpr int smem = SharedAttention<HEAD_DIM, SLOTS>::kSmem;
+  static const cudaError_t configured = cudaFuncSetAttribute(paged_attention_shared_f32_kernel<HEAD_DIM, SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (configured != cudaSuccess) return (int)configured;
+  paged_attention_shared_f32_kernel<HEAD_DIM, SLOTS><<<dim3((tokens + rows_per_tile - 1) / rows_per_tile, kv_heads), kSharedWarps * 32, smem, stream>>>(
+      q, q_row_stride, pages, positions, token_seq, block_table, table_stride, out, tokens, q_heads, kv_heads, page_size, scale, rows_per_tile);
+  return (int)cudaGetLastError();
+}
+
 }  // namespace tlie
 
 using namespace tlie;
@@ -116,4 +283,22 @@ TLIE_EXPORT int tlie_paged_attention_generic(int dtype, const void* q, int q_row
         (const __nv_bfloat16*)q, q_row_stride, (const __nv_bfloat16*)pages, positions, token_seq, block_table,
         table_stride, (__nv_bfloat16*)out, tokens, q_heads, kv_heads, head_dim, page_size, window, scale);
   return (int)cudaGetLastError();
+}
+
+// The same for 32-bit rows of head size 64 or 128 without a window, 16-byte aligned rows and pages, at most 32 query heads per kv head.  single_rows: every
+// row is of another request (a decode step), so a CTA takes one row.
+TLIE_EXPORT int tlie_paged_attention_shared_f32(const float* q, int q_row_stride, const float* pages, const int* positions, const int* token_seq,
+                                                const int* block_table, int table_stride, float* out, int tokens, int q_heads, int kv_heads, int head_dim,
+                                                int page_size, float scale, int single_rows, cudaStream_t stream) {
+  if (tokens <= 0) return 0;
+  if ((head_dim != 64 && head_dim != 128) || kv_heads <= 0 || kv_heads > 65535 || q_heads % kv_heads != 0 || q_heads / kv_heads > 4 * kSharedWarps ||
+      (reinterpret_cast<uintptr_t>(pages) & 15) != 0)
+    return (int)cudaErrorInvalidValue;
+  const int group = q_heads / kv_heads;
+  if (single_rows && group <= kSharedWarps)
+    return head_dim == 64 ? launch_shared<64, 1>(q, q_row_stride, pages, positions, token_seq, block_table, table_stride, out, tokens, q_heads, kv_heads, page_size, scale, 1, stream)
+                          : launch_shared<128, 1>(q, q_row_stride, pages, positions, token_seq, block_table, table_stride, out, tokens, q_heads, kv_heads, page_size, scale, 1, stream);
+  const int rows = single_rows ? 1 : 4 * kSharedWarps / group;
+  return head_dim == 64 ? launch_shared<64, 4>(q, q_row_stride, pages, positions, token_seq, block_table, table_stride, out, tokens, q_heads, kv_heads, page_size, scale, rows, stream)
+                        : launch_shared<128, 4>(q, q_row_stride, pages, positions, token_seq, block_table, table_stride, out, tokens, q_heads, kv_heads, page_size, scale, rows, stream);
 }
