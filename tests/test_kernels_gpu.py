@@ -244,6 +244,40 @@ def test_sampling_non_finite_logits_still_gives_a_token_of_the_vocabulary(ops):
     assert all(0 <= t < vocab for t in out.cpu().tolist())
 
 
+@pytest.mark.parametrize("vocab", [1, 3, 32000, 32767, 32768, 32769, 65537, 128256, 131073, 262145])
+def test_sampling_over_blocks_keeps_the_set_and_the_order_of_tokens(ops, vocab):
+    """Rows of one block, of clusters of 2, 4 and 8 and of the long kernel, vocabularies at their edges; against sums in 64 bits."""
+    torch.manual_seed(35)
+    rows = 24
+    logits = torch.randn(rows, vocab) * 2
+    if vocab > 3:
+        logits[:, vocab - 1] = logits[:, vocab // 2] = 9.0   # ties at the top, one of them the last token
+        logits[0] = 0.0                                       # every token as probable as every other
+    temperature = torch.tensor([0.8, 1.3, 0.0])[torch.arange(rows) % 3]
+    top_p = torch.tensor([0.95, 0.5, 1.0, 1e-6])[torch.arange(rows) % 4]
+    seeds, counters = torch.arange(rows, dtype=torch.int64) * 3 + 5, torch.arange(rows, dtype=torch.int64)
+    got = torch.full((rows,), -7, dtype=torch.int32, device="cuda")
+    ops.sample(logits.cuda(), temperature.cuda(), top_p.cuda(), seeds.cuda(), counters.cuda(), got)
+    for r, token in enumerate(got.tolist()):
+        if float(temperature[r]) == 0.0:
+            assert token == int((logits[r] == logits[r].max()).nonzero()[0]), r
+            continue
+        p = torch.exp((logits[r] - logits[r].max()).double() / float(temperature[r]))
+        order = p.sort(descending=True).values
+        sums = order.cumsum(0)
+        # 32-bit sums of up to 2^18 terms in blocks: a few units of 2^-24 times the depth of the tree (32 per thread, then halving)
+        slack = 64 * 2.0 ** -24 * float(sums[-1])
+        crossing = min(int((sums < float(top_p[r]) * sums[-1] - slack).sum()), vocab - 1)
+        last = min(int((sums < float(top_p[r]) * sums[-1] + slack).sum()), vocab - 1)
+        # the threshold is the probability of the token that crosses the line; rounding may move the line by the slack
+        assert float(p[token]) >= float(order[last]) * (1 - 1e-5), (r, token)
+        if float(top_p[r]) == 1.0 or float(order[crossing]) == float(order[last]):
+            kept = torch.where(p >= float(order[crossing]) * (1 - 1e-6) if float(top_p[r]) < 1.0 else p > 0, p, 0.0).cumsum(0)
+            target = ops.uniform_from(int(seeds[r]), int(counters[r])) * float(kept[-1])
+            before = float(kept[token]) - float(p[token])
+            assert before - slack <= target <= float(kept[token]) + slack, (r, token)
+
+
 def test_argmax_and_sampling(ops):
     torch.manual_seed(7)
     logits = torch.randn(6, 1000)

@@ -9,7 +9,9 @@
 // mt19937; here the kept set is found by bisecting on the probability threshold (no sort),
 // the walk is in token-id order, and the uniform number comes from a counter-based hash
 // of (seed, draw index), so a request's draws do not depend on what else is in the batch.
-// All arithmetic is 32-bit; one block owns one row.
+// All arithmetic is 32-bit; one block owns one row, or a cluster of blocks a long one (see sample_kernel).
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace tlie {
@@ -97,9 +99,9 @@ __host__ __device__ inline float uniform_from(unsigned long long seed, unsigned 
   return (float)(z >> 40) * (1.0f / 16777216.0f);  // 24 bits -> [0, 1)
 }
 
-// One block per row.  temperature <= 0 means greedy for that row.
+// Rows too long for sample_kernel: one block per row that works every probability out again in each pass.  temperature <= 0 means greedy for that row.
 __global__ void __launch_bounds__(kSampleThreads)
-    sample_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
+    sample_long_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
                   const float* __restrict__ top_p, const long long* __restrict__ seeds,
                   const long long* __restrict__ counters, int* __restrict__ out) {
   __shared__ float scratch[32];
@@ -200,6 +202,264 @@ __global__ void __launch_bounds__(kSampleThreads)
   }
 }
 
+// A cluster of CTAS blocks per row (one block up to 32,768 tokens, up to eight), temperature <= 0 means greedy for that row.
+//
+// The bisection asks some thirty times how much probability lies above a threshold.  Bound by those questions' chain of sums, not by bytes: the row's
+// probabilities stay in registers, 32 per thread, so a question is 32 comparisons and one sum over the block (and over the cluster through
+// distributed shared memory).  Read and exponentiated again for every question by one block, 64 rows of 32,000 took 550 us and 4 rows of
+// 128,256 took 800.
+// A block owns a run of token ids; its thread t holds the quads t, t + 1024, ... of the run, so that loads are whole lines; token-id order is
+// block, then round of quads, then thread.
+template <int CTAS>
+__global__ void __launch_bounds__(kSampleThreads)
+    sample_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature, const float* __restrict__ top_p,
+                  const long long* __restrict__ seeds, const long long* __restrict__ counters, int* __restrict__ out) {
+  namespace cg = cooperative_groups;
+  constexpr int kRounds = 8, kWarps = kSampleThreads / 32;
+  __shared__ float scratch[32];
+  __shared__ float exchange[2][8];          // the blocks' partial results, double buffered: one cluster barrier per exchange
+  __shared__ int exchanged_index[8];
+  __shared__ float rounds[kRounds][kWarps];
+  __shared__ int found;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = CTAS > 1 ? (int)cluster.block_rank() : 0;
+  const int row_index = blockIdx.x / CTAS;
+  const float* row = logits + (size_t)row_index * vocab;
+  const float temp = temperature[row_index];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int quads = (vocab + 3) / 4, quads_each = (quads + CTAS - 1) / CTAS;
+  const int first_id = min(vocab, rank * quads_each * 4), end_id = min(vocab, (rank + 1) * quads_each * 4);   // this block's token ids
+
+  if (CTAS > 1) cluster.sync();   // a block's shared memory may be written once the block runs
+  int parity = 0;
+  // every block's value in every block, in block order
+  auto all_values = [&](float mine, float (&values)[CTAS]) {
+    if (CTAS == 1) {
+      values[0] = mine;
+      return;
+    }
+    if (threadIdx.x < CTAS) *cluster.map_shared_rank(&exchange[parity][rank], threadIdx.x) = mine;
+    cluster.sync();
+#pragma unroll
+    for (int c = 0; c < CTAS; ++c) values[c] = exchange[parity][c];
+    parity ^= 1;
+  };
+  auto sum_of_all = [&](float v) {
+    float values[CTAS];
+    all_values(block_sum(v, scratch), values);
+    float sum = values[0];
+#pragma unroll
+    for (int c = 1; c < CTAS; ++c) sum += values[c];
+    return sum;
+  };
+
+  if (!(temp > 0.0f)) {
+    // greedy: lowest id among the maxima
+    float local_max = -INFINITY;
+    int local_arg = 0x7fffffff;
+    row_max_and_arg(row + first_id, end_id - first_id, local_max, local_arg);
+    const float block_best = block_max(local_max, scratch);
+    if (threadIdx.x == 0) found = 0x7fffffff;
+    __syncthreads();
+    if (local_max == block_best && local_arg != 0x7fffffff) atomicMin(&found, first_id + local_arg);
+    __syncthreads();
+    int best_id = found;
+    if (CTAS > 1) {
+      if (threadIdx.x < CTAS) *cluster.map_shared_rank(&exchanged_index[rank], threadIdx.x) = best_id;
+      float values[CTAS];
+      all_values(block_best, values);
+      float best = -INFINITY;
+      best_id = 0x7fffffff;
+#pragma unroll
+      for (int c = 0; c < CTAS; ++c)
+        if (exchanged_index[c] != 0x7fffffff && (values[c] > best || best_id == 0x7fffffff)) {   // blocks are in id order: a tie stays with the first
+          best = values[c];
+          best_id = exchanged_index[c];
+        }
+    }
+    // a row without any comparable value (all NaN) leaves no maximum: token 0, as argmax_kernel answers
+    if (rank == 0 && threadIdx.x == 0) out[row_index] = (best_id < 0 || best_id >= vocab) ? 0 : best_id;
+    return;
+  }
+
+  float p[kRounds][4];   // logits first, then probabilities; -inf (so 0) past the end
+  const bool whole = (vocab & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0;
+  float local_max = -INFINITY;
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) {
+    const int id = first_id + (r * kSampleThreads + (int)threadIdx.x) * 4;
+    if (whole) {
+      const float4 v = id < end_id ? *reinterpret_cast<const float4*>(row + id) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+      p[r][0] = v.x, p[r][1] = v.y, p[r][2] = v.z, p[r][3] = v.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) p[r][i] = id + i < end_id ? row[id + i] : -INFINITY;
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) local_max = fmaxf(local_max, p[r][i]);
+  float row_max;
+  {
+    float values[CTAS];
+    all_values(block_max(local_max, scratch), values);
+    row_max = values[0];
+#pragma unroll
+    for (int c = 1; c < CTAS; ++c) row_max = fmaxf(row_max, values[c]);
+  }
+  const float inv_temp = 1.0f / temp;
+  float sum = 0.0f;
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) {
+    const int id = first_id + (r * kSampleThreads + (int)threadIdx.x) * 4;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      p[r][i] = id + i < end_id ? expf((p[r][i] - row_max) * inv_temp) : -1.0f;   // -1: no token, never kept
+      sum += id + i < end_id ? p[r][i] : 0.0f;
+    }
+  }
+  const float total = sum_of_all(sum);
+
+  // Largest threshold tau with mass{p >= tau} >= top_p * total, by bisection on the bit
+  // pattern of positive floats (monotone in value).  The kept set is {p >= tau}.
+  float tau = 0.0f;
+  if (top_p[row_index] < 1.0f) {
+    const float want = top_p[row_index] * total;
+    unsigned lo = 0u;                    // mass{p >= 0} = total >= want
+    unsigned hi = __float_as_uint(1.0f) + 1u;  // p <= 1, so mass{p >= hi} = 0 < want
+    while (hi - lo > 1u) {
+      const unsigned mid = lo + (hi - lo) / 2u;
+      const float threshold = __uint_as_float(mid);
+      float mass[2] = {0.0f, 0.0f};
+#pragma unroll
+      for (int r = 0; r < kRounds; ++r)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (p[r][i] >= threshold) mass[i & 1] += p[r][i];
+      if (sum_of_all(mass[0] + mass[1]) >= want) lo = mid; else hi = mid;
+    }
+    tau = __uint_as_float(lo);
+  }
+
+  // what is kept, per round and warp, then per block
+  float kept[kRounds];
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) {
+    kept[r] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (p[r][i] >= tau) kept[r] += p[r][i];
+    const float of_warp = warp_sum(kept[r]);
+    if (lane == 0) rounds[r][warp] = of_warp;
+  }
+  if (threadIdx.x == 0) found = -1;
+  __syncthreads();
+  float of_round[kRounds], of_block = 0.0f;
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) {
+    of_round[r] = warp_sum(rounds[r][lane]);
+    of_block += of_round[r];
+  }
+  float blocks[CTAS];
+  all_values(of_block, blocks);
+  float kept_total = blocks[0];
+#pragma unroll
+  for (int c = 1; c < CTAS; ++c) kept_total += blocks[c];
+  const float target = uniform_from((unsigned long long)seeds[row_index], (unsigned long long)counters[row_index]) * kept_total;
+
+  // The last block, round and thread with something kept that starts at or before the target holds it (whatever rounding does to the starts), and of its
+  // quad the first token that reaches past the target, or the last kept one.
+  int block_of = -1;
+  float start = 0.0f, running = 0.0f;
+#pragma unroll
+  for (int c = 0; c < CTAS; ++c) {
+    if (blocks[c] > 0.0f && running <= target) {
+      block_of = c;
+      start = running;
+    }
+    running += blocks[c];
+  }
+  if (block_of == rank) {   // the same for the whole block
+    int round_of = -1;
+    running = start;
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      if (of_round[r] > 0.0f && running <= target) {
+        round_of = r;
+        start = running;
+      }
+      running += of_round[r];
+    }
+    if (round_of >= 0) {
+      float mine = 0.0f, quad[4];
+#pragma unroll
+      for (int r = 0; r < kRounds; ++r)
+        if (r == round_of) {
+          mine = kept[r];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) quad[i] = p[r][i];
+        }
+      float inclusive = mine;   // over the warp's lanes, then the warps before it
+#pragma unroll
+      for (int offset = 1; offset < 32; offset <<= 1) {
+        const float before = __shfl_up_sync(0xffffffffu, inclusive, offset);
+        if (lane >= offset) inclusive += before;
+      }
+      float cursor = start + warp_sum(lane < warp ? rounds[round_of][lane] : 0.0f) + (inclusive - mine);
+      const bool here = mine > 0.0f && cursor <= target;
+      if (here) atomicMax(&found, (int)threadIdx.x);
+      __syncthreads();
+      const int holder = found;
+      __syncthreads();
+      // rounding can put the first kept thread's start past the target: then it is that one
+      if (holder < 0 && threadIdx.x == 0) found = kSampleThreads;
+      __syncthreads();
+      if (holder < 0 && mine > 0.0f) atomicMin(&found, (int)threadIdx.x);
+      __syncthreads();
+      if (found == (int)threadIdx.x) {
+        int pick = -1;
+        const int id = first_id + (round_of * kSampleThreads + (int)threadIdx.x) * 4;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (quad[i] >= tau && !(pick >= 0 && target < cursor)) {
+            cursor += quad[i];
+            pick = id + i;
+          }
+        out[row_index] = (pick < 0 || pick >= vocab) ? 0 : pick;
+      }
+      if (found >= kSampleThreads && threadIdx.x == 0) out[row_index] = 0;
+    } else if (threadIdx.x == 0) {
+      out[row_index] = 0;
+    }
+  } else if (block_of < 0 && rank == 0) {
+    // non-finite logits: nothing kept, or no comparable target: the last kept token of the row, and at any rate one of the vocabulary
+    int last = 0;
+    for (int i = threadIdx.x; i < vocab; i += kSampleThreads)
+      if (expf((row[i] - row_max) * inv_temp) >= tau) last = max(last, i);
+    atomicMax(&found, last);
+    __syncthreads();
+    if (threadIdx.x == 0) out[row_index] = max(found, 0);
+  }
+  // no block leaves while another may still write its part of an exchange: the last exchange ended in a barrier that follows all writes
+}
+
+template <int CTAS>
+static int launch_sample(const float* logits, int rows, int vocab, const float* temperature, const float* top_p, const long long* seeds, const long long* counters,
+                         int* out, cudaStream_t stream) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(rows * CTAS);
+  config.blockDim = dim3(kSampleThreads);
+  config.stream = stream;
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeClusterDimension;
+  attribute[0].val.clusterDim.x = CTAS;
+  attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
+  config.attrs = attribute;
+  config.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&config, sample_kernel<CTAS>, logits, vocab, temperature, top_p, seeds, counters, out);
+}
+
 }  // namespace tlie
 
 using namespace tlie;
@@ -213,7 +473,13 @@ TLIE_EXPORT int tlie_argmax(const float* logits, int rows, int vocab, int* out, 
 TLIE_EXPORT int tlie_sample(const float* logits, int rows, int vocab, const float* temperature, const float* top_p,
                             const long long* seeds, const long long* counters, int* out, cudaStream_t stream) {
   if (rows <= 0) return 0;
-  sample_kernel<<<rows, kSampleThreads, 0, stream>>>(logits, vocab, temperature, top_p, seeds, counters, out);
+  // a block holds 32 probabilities per thread
+  constexpr int kHeld = 32 * kSampleThreads;
+  if (vocab <= kHeld) return launch_sample<1>(logits, rows, vocab, temperature, top_p, seeds, counters, out, stream);
+  if (vocab <= 2 * kHeld) return launch_sample<2>(logits, rows, vocab, temperature, top_p, seeds, counters, out, stream);
+  if (vocab <= 4 * kHeld) return launch_sample<4>(logits, rows, vocab, temperature, top_p, seeds, counters, out, stream);
+  if (vocab <= 8 * kHeld) return launch_sample<8>(logits, rows, vocab, temperature, top_p, seeds, counters, out, stream);
+  sample_long_kernel<<<rows, kSampleThreads, 0, stream>>>(logits, vocab, temperature, top_p, seeds, counters, out);
   return (int)cudaGetLastError();
 }
 
