@@ -202,124 +202,112 @@ __global__ void __launch_bounds__(kSampleThreads)
   }
 }
 
-// A cluster of CTAS blocks per row (one block up to 32,768 tokens, up to eight), temperature <= 0 means greedy for that row.
+// A cluster of CTAS blocks per row (one block up to 32,768 tokens, up to four), temperature <= 0 means greedy for that row.
 //
 // The bisection asks some thirty times how much probability lies above a threshold.  Bound by those questions' chain of sums, not by bytes: the row's
-// probabilities stay in registers, 32 per thread, so a question is 32 comparisons and one sum over the block (and over the cluster through
+// probabilities stay in registers, 32 * CTAS per thread, so a question is that many comparisons and one sum over the block (and over the cluster through
 // distributed shared memory).  Read and exponentiated again for every question by one block, 64 rows of 32,000 took 550 us and 4 rows of
 // 128,256 took 800.
-// A block owns a run of token ids; its thread t holds the quads t, t + 1024, ... of the run, so that loads are whole lines; token-id order is
-// block, then round of quads, then thread.
+// Every sum keeps the long kernel's order: 1,024 runs of consecutive tokens, one per thread of the cluster, added run by run, then 32 runs at a time, then
+// those.  A token far down the tail has a probability near the rounding of the sums before it, so in another order one draw in a hundred that falls
+// into a flat tail would be another token.
 template <int CTAS>
-__global__ void __launch_bounds__(kSampleThreads)
+__global__ void __launch_bounds__(kSampleThreads / CTAS)
     sample_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature, const float* __restrict__ top_p,
                   const long long* __restrict__ seeds, const long long* __restrict__ counters, int* __restrict__ out) {
   namespace cg = cooperative_groups;
-  constexpr int kRounds = 8, kWarps = kSampleThreads / 32;
-  __shared__ float scratch[32];
-  __shared__ float exchange[2][8];          // the blocks' partial results, double buffered: one cluster barrier per exchange
-  __shared__ int exchanged_index[8];
-  __shared__ float rounds[kRounds][kWarps];
-  __shared__ int found;
+  constexpr int kThreads = kSampleThreads / CTAS, kWarps = kThreads / 32, kHeld = 32 * CTAS;
+  __shared__ float exchange[2][32];         // the warps' partial results of the whole cluster, double buffered: one barrier per exchange
+  __shared__ int arg_exchange[32];
+  __shared__ __align__(16) float prefix[kSampleThreads];
+  __shared__ float kept_total_smem;
+  __shared__ int chosen, last_kept;         // the first block's are the row's
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = CTAS > 1 ? (int)cluster.block_rank() : 0;
   const int row_index = blockIdx.x / CTAS;
   const float* row = logits + (size_t)row_index * vocab;
   const float temp = temperature[row_index];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int quads = (vocab + 3) / 4, quads_each = (quads + CTAS - 1) / CTAS;
-  const int first_id = min(vocab, rank * quads_each * 4), end_id = min(vocab, (rank + 1) * quads_each * 4);   // this block's token ids
-
-  if (CTAS > 1) cluster.sync();   // a block's shared memory may be written once the block runs
-  int parity = 0;
-  // every block's value in every block, in block order
-  auto all_values = [&](float mine, float (&values)[CTAS]) {
-    if (CTAS == 1) {
-      values[0] = mine;
-      return;
-    }
-    if (threadIdx.x < CTAS) *cluster.map_shared_rank(&exchange[parity][rank], threadIdx.x) = mine;
-    cluster.sync();
-#pragma unroll
-    for (int c = 0; c < CTAS; ++c) values[c] = exchange[parity][c];
-    parity ^= 1;
+  const int run = rank * kThreads + (int)threadIdx.x;    // which of the 1,024 runs is this thread's
+  auto sync_all = [&] {
+    if (CTAS > 1) cluster.sync();
+    else __syncthreads();
   };
-  auto sum_of_all = [&](float v) {
-    float values[CTAS];
-    all_values(block_sum(v, scratch), values);
-    float sum = values[0];
-#pragma unroll
-    for (int c = 1; c < CTAS; ++c) sum += values[c];
-    return sum;
+  if (CTAS > 1) cluster.sync();   // a block's shared memory may be written once the block runs
+
+  int parity = 0;
+  // this thread's view of all 32 warps' values, lane w holds warp w's
+  auto all_warps = [&](float mine) {
+    if (lane < CTAS) *(CTAS > 1 ? cluster.map_shared_rank(&exchange[parity][rank * kWarps + warp], lane) : &exchange[0][warp] + parity * 32) = mine;
+    sync_all();
+    const float value = exchange[parity][lane];
+    parity ^= 1;
+    return value;
   };
 
   if (!(temp > 0.0f)) {
-    // greedy: lowest id among the maxima
-    float local_max = -INFINITY;
-    int local_arg = 0x7fffffff;
-    row_max_and_arg(row + first_id, end_id - first_id, local_max, local_arg);
-    const float block_best = block_max(local_max, scratch);
-    if (threadIdx.x == 0) found = 0x7fffffff;
-    __syncthreads();
-    if (local_max == block_best && local_arg != 0x7fffffff) atomicMin(&found, first_id + local_arg);
-    __syncthreads();
-    int best_id = found;
-    if (CTAS > 1) {
-      if (threadIdx.x < CTAS) *cluster.map_shared_rank(&exchanged_index[rank], threadIdx.x) = best_id;
-      float values[CTAS];
-      all_values(block_best, values);
-      float best = -INFINITY;
-      best_id = 0x7fffffff;
+    // greedy: lowest id among the maxima.  Each block takes a quarter (or all) of the row in whole lines.
+    const int each = ((vocab + CTAS - 1) / CTAS + 3) & ~3;
+    const int first_id = min(vocab, rank * each), end_id = min(vocab, first_id + each);
+    float value = -INFINITY;
+    int index = 0x7fffffff;
+    row_max_and_arg(row + first_id, end_id - first_id, value, index);
+    if (index != 0x7fffffff) index += first_id;
 #pragma unroll
-      for (int c = 0; c < CTAS; ++c)
-        if (exchanged_index[c] != 0x7fffffff && (values[c] > best || best_id == 0x7fffffff)) {   // blocks are in id order: a tie stays with the first
-          best = values[c];
-          best_id = exchanged_index[c];
-        }
+    for (int offset = 16; offset > 0; offset >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, value, offset);
+      const int oi = __shfl_xor_sync(0xffffffffu, index, offset);
+      if (ov > value || (ov == value && oi < index)) {
+        value = ov;
+        index = oi;
+      }
+    }
+    if (lane < CTAS) *(CTAS > 1 ? cluster.map_shared_rank(&arg_exchange[rank * kWarps + warp], lane) : &arg_exchange[warp]) = index;
+    value = all_warps(value);
+    index = arg_exchange[lane];
+#pragma unroll
+    for (int offset = 16; offset > 0; offset >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, value, offset);
+      const int oi = __shfl_xor_sync(0xffffffffu, index, offset);
+      if (ov > value || (ov == value && oi < index)) {
+        value = ov;
+        index = oi;
+      }
     }
     // a row without any comparable value (all NaN) leaves no maximum: token 0, as argmax_kernel answers
-    if (rank == 0 && threadIdx.x == 0) out[row_index] = (best_id < 0 || best_id >= vocab) ? 0 : best_id;
+    if (rank == 0 && threadIdx.x == 0) out[row_index] = (index < 0 || index >= vocab) ? 0 : index;
     return;
   }
 
-  float p[kRounds][4];   // logits first, then probabilities; -inf (so 0) past the end
-  const bool whole = (vocab & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0;
+  const int per_run = (vocab + kSampleThreads - 1) / kSampleThreads;   // at most kHeld
+  const int begin = min(vocab, run * per_run), count = min(vocab, begin + per_run) - begin;
+  float p[kHeld];   // logits first, then probabilities
   float local_max = -INFINITY;
+  if ((per_run & 3) == 0 && (vocab & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
 #pragma unroll
-  for (int r = 0; r < kRounds; ++r) {
-    const int id = first_id + (r * kSampleThreads + (int)threadIdx.x) * 4;
-    if (whole) {
-      const float4 v = id < end_id ? *reinterpret_cast<const float4*>(row + id) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
-      p[r][0] = v.x, p[r][1] = v.y, p[r][2] = v.z, p[r][3] = v.w;
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) p[r][i] = id + i < end_id ? row[id + i] : -INFINITY;
+    for (int i = 0; i < kHeld; i += 4) {
+      const float4 v = i < count ? *reinterpret_cast<const float4*>(row + begin + i) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+      p[i] = v.x, p[i + 1] = v.y, p[i + 2] = v.z, p[i + 3] = v.w;
     }
+  } else {
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) p[i] = i < count ? row[begin + i] : -INFINITY;
   }
 #pragma unroll
-  for (int r = 0; r < kRounds; ++r)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) local_max = fmaxf(local_max, p[r][i]);
-  float row_max;
-  {
-    float values[CTAS];
-    all_values(block_max(local_max, scratch), values);
-    row_max = values[0];
-#pragma unroll
-    for (int c = 1; c < CTAS; ++c) row_max = fmaxf(row_max, values[c]);
-  }
+  for (int i = 0; i < kHeld; ++i)
+    if (i < count && p[i] > local_max) local_max = p[i];
+  const float row_max = warp_max(all_warps(warp_max(local_max)));
   const float inv_temp = 1.0f / temp;
   float sum = 0.0f;
 #pragma unroll
-  for (int r = 0; r < kRounds; ++r) {
-    const int id = first_id + (r * kSampleThreads + (int)threadIdx.x) * 4;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      p[r][i] = id + i < end_id ? expf((p[r][i] - row_max) * inv_temp) : -1.0f;   // -1: no token, never kept
-      sum += id + i < end_id ? p[r][i] : 0.0f;
+  for (int i = 0; i < kHeld; ++i)
+    if (i < count) {
+      p[i] = expf((p[i] - row_max) * inv_temp);
+      sum += p[i];
+    } else {
+      p[i] = -1.0f;   // no token: never kept
     }
-  }
-  const float total = sum_of_all(sum);
+  const float total = warp_sum(all_warps(warp_sum(sum)));
 
   // Largest threshold tau with mass{p >= tau} >= top_p * total, by bisection on the bit
   // pattern of positive floats (monotone in value).  The kept set is {p >= tau}.
@@ -331,117 +319,72 @@ __global__ void __launch_bounds__(kSampleThreads)
     while (hi - lo > 1u) {
       const unsigned mid = lo + (hi - lo) / 2u;
       const float threshold = __uint_as_float(mid);
-      float mass[2] = {0.0f, 0.0f};
+      float mass = 0.0f;
 #pragma unroll
-      for (int r = 0; r < kRounds; ++r)
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (p[r][i] >= threshold) mass[i & 1] += p[r][i];
-      if (sum_of_all(mass[0] + mass[1]) >= want) lo = mid; else hi = mid;
+      for (int i = 0; i < kHeld; ++i)
+        if (p[i] >= threshold) mass += p[i];
+      if (warp_sum(all_warps(warp_sum(mass))) >= want) lo = mid; else hi = mid;
     }
     tau = __uint_as_float(lo);
   }
-
-  // what is kept, per round and warp, then per block
-  float kept[kRounds];
+  float kept = 0.0f;
+  int last = -1;
 #pragma unroll
-  for (int r = 0; r < kRounds; ++r) {
-    kept[r] = 0.0f;
+  for (int i = 0; i < kHeld; ++i)
+    if (p[i] >= tau) {
+      kept += p[i];
+      last = begin + i;
+    }
+  if (threadIdx.x == 0) chosen = last_kept = -1;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (p[r][i] >= tau) kept[r] += p[r][i];
-    const float of_warp = warp_sum(kept[r]);
-    if (lane == 0) rounds[r][warp] = of_warp;
+  for (int c = 0; c < CTAS; ++c) *(CTAS > 1 ? cluster.map_shared_rank(&prefix[run], c) : &prefix[run]) = kept;
+  sync_all();
+  if (threadIdx.x == 0) {   // exclusive scan in run order, in every block
+    float running = 0.0f;
+#pragma unroll 8
+    for (int i = 0; i < kSampleThreads; i += 4) {
+      const float4 v = *reinterpret_cast<const float4*>(prefix + i);
+      float4 start;
+      start.x = running;
+      running += v.x;
+      start.y = running;
+      running += v.y;
+      start.z = running;
+      running += v.z;
+      start.w = running;
+      running += v.w;
+      *reinterpret_cast<float4*>(prefix + i) = start;
+    }
+    kept_total_smem = running;
   }
-  if (threadIdx.x == 0) found = -1;
   __syncthreads();
-  float of_round[kRounds], of_block = 0.0f;
+  const float target = uniform_from((unsigned long long)seeds[row_index], (unsigned long long)counters[row_index]) * kept_total_smem;
+  // the run whose [start, start + kept) holds the target walks its tokens
+  const float start = prefix[run];
+  int* row_chosen = CTAS > 1 ? cluster.map_shared_rank(&chosen, 0) : &chosen;
+  int* row_last = CTAS > 1 ? cluster.map_shared_rank(&last_kept, 0) : &last_kept;
+  if (kept > 0.0f && target >= start && target < start + kept) {
+    float cursor = start;
+    int pick = -1;
+    bool reached = false;
 #pragma unroll
-  for (int r = 0; r < kRounds; ++r) {
-    of_round[r] = warp_sum(rounds[r][lane]);
-    of_block += of_round[r];
-  }
-  float blocks[CTAS];
-  all_values(of_block, blocks);
-  float kept_total = blocks[0];
-#pragma unroll
-  for (int c = 1; c < CTAS; ++c) kept_total += blocks[c];
-  const float target = uniform_from((unsigned long long)seeds[row_index], (unsigned long long)counters[row_index]) * kept_total;
-
-  // The last block, round and thread with something kept that starts at or before the target holds it (whatever rounding does to the starts), and of its
-  // quad the first token that reaches past the target, or the last kept one.
-  int block_of = -1;
-  float start = 0.0f, running = 0.0f;
-#pragma unroll
-  for (int c = 0; c < CTAS; ++c) {
-    if (blocks[c] > 0.0f && running <= target) {
-      block_of = c;
-      start = running;
-    }
-    running += blocks[c];
-  }
-  if (block_of == rank) {   // the same for the whole block
-    int round_of = -1;
-    running = start;
-#pragma unroll
-    for (int r = 0; r < kRounds; ++r) {
-      if (of_round[r] > 0.0f && running <= target) {
-        round_of = r;
-        start = running;
+    for (int i = 0; i < kHeld; ++i)
+      if (!reached && p[i] >= tau) {
+        cursor += p[i];
+        pick = begin + i;
+        reached = target < cursor;
       }
-      running += of_round[r];
-    }
-    if (round_of >= 0) {
-      float mine = 0.0f, quad[4];
-#pragma unroll
-      for (int r = 0; r < kRounds; ++r)
-        if (r == round_of) {
-          mine = kept[r];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) quad[i] = p[r][i];
-        }
-      float inclusive = mine;   // over the warp's lanes, then the warps before it
-#pragma unroll
-      for (int offset = 1; offset < 32; offset <<= 1) {
-        const float before = __shfl_up_sync(0xffffffffu, inclusive, offset);
-        if (lane >= offset) inclusive += before;
-      }
-      float cursor = start + warp_sum(lane < warp ? rounds[round_of][lane] : 0.0f) + (inclusive - mine);
-      const bool here = mine > 0.0f && cursor <= target;
-      if (here) atomicMax(&found, (int)threadIdx.x);
-      __syncthreads();
-      const int holder = found;
-      __syncthreads();
-      // rounding can put the first kept thread's start past the target: then it is that one
-      if (holder < 0 && threadIdx.x == 0) found = kSampleThreads;
-      __syncthreads();
-      if (holder < 0 && mine > 0.0f) atomicMin(&found, (int)threadIdx.x);
-      __syncthreads();
-      if (found == (int)threadIdx.x) {
-        int pick = -1;
-        const int id = first_id + (round_of * kSampleThreads + (int)threadIdx.x) * 4;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (quad[i] >= tau && !(pick >= 0 && target < cursor)) {
-            cursor += quad[i];
-            pick = id + i;
-          }
-        out[row_index] = (pick < 0 || pick >= vocab) ? 0 : pick;
-      }
-      if (found >= kSampleThreads && threadIdx.x == 0) out[row_index] = 0;
-    } else if (threadIdx.x == 0) {
-      out[row_index] = 0;
-    }
-  } else if (block_of < 0 && rank == 0) {
-    // non-finite logits: nothing kept, or no comparable target: the last kept token of the row, and at any rate one of the vocabulary
-    int last = 0;
-    for (int i = threadIdx.x; i < vocab; i += kSampleThreads)
-      if (expf((row[i] - row_max) * inv_temp) >= tau) last = max(last, i);
-    atomicMax(&found, last);
-    __syncthreads();
-    if (threadIdx.x == 0) out[row_index] = max(found, 0);
+    atomicMax(row_chosen, pick);
   }
-  // no block leaves while another may still write its part of an exchange: the last exchange ended in a barrier that follows all writes
+  last = __reduce_max_sync(0xffffffffu, last);
+  if (lane == 0) atomicMax(row_last, last);
+  sync_all();
+  if (rank == 0 && threadIdx.x == 0) {
+    // rounding can put the target past the last kept token: take the last kept one; non-finite logits can leave nothing kept at all: the answer must
+    // still be a token of the vocabulary
+    const int pick = chosen < 0 ? last_kept : chosen;
+    out[row_index] = (pick < 0 || pick >= vocab) ? 0 : pick;
+  }
 }
 
 template <int CTAS>
@@ -449,7 +392,7 @@ static int launch_sample(const float* logits, int rows, int vocab, const float* 
                          int* out, cudaStream_t stream) {
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(rows * CTAS);
-  config.blockDim = dim3(kSampleThreads);
+  config.blockDim = dim3(kSampleThreads / CTAS);
   config.stream = stream;
   cudaLaunchAttribute attribute[1];
   attribute[0].id = cudaLaunchAttributeClusterDimension;
@@ -473,12 +416,10 @@ TLIE_EXPORT int tlie_argmax(const float* logits, int rows, int vocab, int* out, 
 TLIE_EXPORT int tlie_sample(const float* logits, int rows, int vocab, const float* temperature, const float* top_p,
                             const long long* seeds, const long long* counters, int* out, cudaStream_t stream) {
   if (rows <= 0) return 0;
-  // a block holds 32 probabilities per thread
-  constexpr int kHeld = 32 * kSampleThreads;
+  constexpr int kHeld = 32 * kSampleThreads;   // what a block's registers hold
   if (vocab <= kHeld) return launch_sample<1>(logits, rows, vocab, temperature, top_p, seeds, counters, out, stream);
   if (vocab <= 2 * kHeld) return launch_sample<2>(logits, rows, vocab, temperature, top_p, seeds, counters, out, stream);
   if (vocab <= 4 * kHeld) return launch_sample<4>(logits, rows, vocab, temperature, top_p, seeds, counters, out, stream);
-  if (vocab <= 8 * kHeld) return launch_sample<8>(logits, rows, vocab, temperature, top_p, seeds, counters, out, stream);
   sample_long_kernel<<<rows, kSampleThreads, 0, stream>>>(logits, vocab, temperature, top_p, seeds, counters, out);
   return (int)cudaGetLastError();
 }
