@@ -23,6 +23,10 @@ constexpr int kTileKeys = 32;
 #endif
 constexpr int kWarps = DECODE_WARPS;
 constexpr int kStages = DECODE_STAGES;
+#ifndef DECODE_TILES_PER_WARP
+#define DECODE_TILES_PER_WARP 1
+#endif
+constexpr int kTilesPerWarp = DECODE_TILES_PER_WARP;   // what a part holds at least, per warp
 constexpr int kRow = kD + 8;                       // padded row, in elements (16 bytes of padding)
 constexpr int kTileElems = kTileKeys * kRow;       // one K or V tile
 constexpr int kChunks = kD / 8;                    // 16-byte chunks per row
@@ -128,6 +132,7 @@ struct DecodeAttnParams {
 struct DecodeAttnItem {
   int seq, kvh, split;
   int pos, n_keys, lo, tile_begin, tile_end, next_load;
+  int parts;   // into how many of the launch's `splits` the keys of this request are cut: CTAs past them have nothing to do
   const int* table;
   bool patch_new;
   // cos (first half) and sin (second half) of this position's rotation angles, in shared memory: worked out in the first
@@ -149,7 +154,11 @@ __device__ __forceinline__ void decode_attn_prologue(const DecodeAttnParams& p, 
   // this CTA's tiles: [it.tile_begin, it.tile_end)
   const int first_tile = it.lo / kTileKeys;
   const int all_tiles = (it.n_keys + kTileKeys - 1) / kTileKeys - first_tile;
-  const int per_split = (all_tiles + p.splits - 1) / p.splits;
+  // A part is worth its merge (a trip to L2 for the partial results, one for the ticket, one back) only where the warps of the parts before it
+  // have a tile each: 57 to 89 keys in one part of three tiles instead of three parts of one.
+  it.parts = min(p.splits, (all_tiles + kWarps * kTilesPerWarp - 1) / (kWarps * kTilesPerWarp));
+  if (it.split >= it.parts) return;
+  const int per_split = (all_tiles + it.parts - 1) / it.parts;
   it.tile_begin = first_tile + it.split * per_split;
   it.tile_end = min(first_tile + all_tiles, it.tile_begin + per_split);
 
@@ -407,6 +416,7 @@ __device__ __forceinline__ void decode_attn_main(const DecodeAttnParams& p, Deco
     row_sum[r] += __shfl_xor_sync(0xffffffffu, row_sum[r], 2);
   }
   __syncthreads();  // every warp is done with its stage buffers: reuse them to merge the warps
+  const int live = min(kWarps, it.tile_end - it.tile_begin);   // warps that had a tile
 
   float* merge_o = reinterpret_cast<float*>(smem_raw);                   // [warp][16][kD]
   float* merge_ml = merge_o + kWarps * 16 * kD;                          // [warp][16][2]
@@ -429,18 +439,16 @@ __device__ __forceinline__ void decode_attn_main(const DecodeAttnParams& p, Deco
     const int r = idx / kD;
     const int d = idx - r * kD;
     float m = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) m = fmaxf(m, merge_ml[(w * 16 + r) * 2]);
+    for (int w = 0; w < live; ++w) m = fmaxf(m, merge_ml[(w * 16 + r) * 2]);
     float acc = 0.0f, sum = 0.0f;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
+    for (int w = 0; w < live; ++w) {
       const float wm = merge_ml[(w * 16 + r) * 2];
       const float f = (wm == -INFINITY) ? 0.0f : exp2f(wm - m);
       acc += f * merge_o[((size_t)w * 16 + r) * kD + d];
       sum += f * merge_ml[(w * 16 + r) * 2 + 1];
     }
     const int head = it.kvh * group + r;
-    if (p.splits == 1) {
+    if (it.parts == 1) {
       p.out[((size_t)it.seq * p.q_heads + head) * kD + d] = __float2bfloat16_rn(acc / sum);
     } else {
       const size_t slot = ((size_t)it.seq * p.q_heads + head) * p.splits + it.split;
@@ -451,18 +459,18 @@ __device__ __forceinline__ void decode_attn_main(const DecodeAttnParams& p, Deco
       }
     }
   }
-  if (p.splits == 1) return;
+  if (it.parts == 1) return;
   // The CTA of this (request, kv head) that arrives last merges all parts.  No CTA waits for another.
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
     const int ticket = atomicAdd(&p.tickets[it.seq * p.kv_heads + it.kvh], 1);
-    *last_arrival = (ticket == p.splits - 1);
+    *last_arrival = (ticket == it.parts - 1);
   }
   __syncthreads();
   if (!*last_arrival) return;
   __threadfence();
-  // One warp per query head, lane sp holds part sp's maximum and sum (p.splits <= 32).  The parts' outputs do not depend
+  // One warp per query head, lane sp holds part sp's maximum and sum (at most 32 parts).  The parts' outputs do not depend
   // on those, so their loads go out first, eight parts at a time, and everything is one trip to L2 and back.
   for (int r = warp; r < group; r += kWarps) {
     const size_t pair = (size_t)it.seq * p.q_heads + it.kvh * group + r;
@@ -472,17 +480,17 @@ __device__ __forceinline__ void decode_attn_main(const DecodeAttnParams& p, Deco
 #pragma unroll
     for (int i = 0; i < kPerLane; ++i) acc[i] = 0.0f;
     float part_max = -INFINITY, part_sum = 0.0f, m = 0.0f, f = 0.0f, sum = 0.0f;
-    for (int sp0 = 0; sp0 < p.splits; sp0 += 8) {
+    for (int sp0 = 0; sp0 < it.parts; sp0 += 8) {
       float part[8][kPerLane];
 #pragma unroll
       for (int j = 0; j < 8; ++j)
 #pragma unroll
         for (int i = 0; i < kPerLane; ++i) {
           const int d = lane + 32 * i;
-          part[j][i] = (sp0 + j < p.splits && d < kD) ? __ldcg(p.partial_o + (pair * p.splits + sp0 + j) * kD + d) : 0.0f;
+          part[j][i] = (sp0 + j < it.parts && d < kD) ? __ldcg(p.partial_o + (pair * p.splits + sp0 + j) * kD + d) : 0.0f;
         }
       if (sp0 == 0) {
-        if (lane < p.splits) {
+        if (lane < it.parts) {
           part_max = __ldcg(ml + lane * 2);
           part_sum = __ldcg(ml + lane * 2 + 1);
         }
@@ -494,7 +502,7 @@ __device__ __forceinline__ void decode_attn_main(const DecodeAttnParams& p, Deco
       for (int j = 0; j < 8; ++j) {
         const float fs = __shfl_sync(0xffffffffu, f, (sp0 + j) & 31);
 #pragma unroll
-        for (int i = 0; i < kPerLane; ++i) acc[i] += fs * part[j][i];   // parts past p.splits were loaded as zeros
+        for (int i = 0; i < kPerLane; ++i) acc[i] += fs * part[j][i];   // parts past the last were loaded as zeros
       }
     }
 #pragma unroll
