@@ -584,6 +584,24 @@ def test_decode_attention_with_rotation_and_cache_write(ops, q_heads, kv_heads, 
             assert torch.equal(pages_gpu.cpu(), pages)
 
 
+@pytest.mark.parametrize("q_heads,kv_heads,head_dim", [(32, 4, 64), (8, 2, 128)])
+@pytest.mark.parametrize("splits", [2, 4, 8, 18])
+def test_decode_attention_parts_that_are_warps(ops, q_heads, kv_heads, head_dim, splits):
+    """Keys around whole tiles and around as many tiles as a CTA has warps: parts in one CTA, in several, and launched parts without keys."""
+    from tinyllama_inference_engine_b200.ops import fast
+
+    rng = np.random.default_rng(36)
+    torch.manual_seed(36)
+    seq_lens = [1, 31, 32, 33, 64, 65, 96, 97, 128, 129, 255, 256, 257, 288, 577]
+    qkv, pages, positions, token_seq, table = _paged_case(rng, torch.bfloat16, seq_lens, [1] * len(seq_lens), kv_heads, head_dim, 64, q_heads)
+    want = torch.empty(len(seq_lens), q_heads * head_dim, dtype=torch.bfloat16)
+    plain_ops.paged_attention(qkv, pages, positions, token_seq, table, want, q_heads, kv_heads, head_dim, 64)
+    for _ in range(2):   # the tickets are left as they were found
+        got = torch.empty(want.shape, dtype=torch.bfloat16, device="cuda")
+        fast.decode_attention(qkv.cuda(), pages.cuda(), positions.cuda(), table.cuda(), got, q_heads, kv_heads, head_dim, 64, 0, head_dim ** -0.5, splits)
+        assert float((got.cpu().float() - want.float()).abs().max()) <= 1.6e-2
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 128, 64), (128, 256, 128), (2048, 2560, 2048), (300, 200, 136), (2048, 2048, 5632), (129, 1000, 2048), (1000, 131, 80),
                                    (4200, 2500, 72)])
 @pytest.mark.parametrize("tile_n,pair", [(width, pair) for width in (128, 160, 192, 256) for pair in (False, True)] + [(288, False), (320, False), (288, True), (384, True), (480, True)])   # the wide tiles: two for single SMs, three for pairs

@@ -8,8 +8,8 @@
 //   * one CTA per (request, kv head, split of the key range); the query heads that share the
 //     kv head (the group, up to 16) are the rows of one tensor-core tile, so every key and value
 //     is read from HBM once per group, not once per head;
-//   * the key range of a request is cut into up to SPLITS parts, as many as give every warp a tile, so that small
-//     batches still fill the 148 SMs;
+//   * the key range of a request is cut into SPLITS parts so that small batches still fill the 148 SMs (none is needed when
+//     SPLITS == 1; parts of a single tile are warps of one CTA where they fit it);
 //   * each of the four warps of a CTA walks its own 32-key tiles with a private multi-stage
 //     cp.async pipeline (no block-wide barrier in the loop); rows in shared memory are padded
 //     by 16 bytes so that ldmatrix reads are free of bank conflicts for any head size;

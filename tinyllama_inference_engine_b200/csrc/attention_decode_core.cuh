@@ -23,10 +23,6 @@ constexpr int kTileKeys = 32;
 #endif
 constexpr int kWarps = DECODE_WARPS;
 constexpr int kStages = DECODE_STAGES;
-#ifndef DECODE_TILES_PER_WARP
-#define DECODE_TILES_PER_WARP 1
-#endif
-constexpr int kTilesPerWarp = DECODE_TILES_PER_WARP;   // what a part holds at least, per warp
 constexpr int kRow = kD + 8;                       // padded row, in elements (16 bytes of padding)
 constexpr int kTileElems = kTileKeys * kRow;       // one K or V tile
 constexpr int kChunks = kD / 8;                    // 16-byte chunks per row
@@ -132,7 +128,8 @@ struct DecodeAttnParams {
 struct DecodeAttnItem {
   int seq, kvh, split;
   int pos, n_keys, lo, tile_begin, tile_end, next_load;
-  int parts;   // into how many of the launch's `splits` the keys of this request are cut: CTAs past them have nothing to do
+  int parts;   // how many of the launch's `splits` have keys of this request: CTAs past them have nothing to do
+  bool warps_are_parts;
   const int* table;
   bool patch_new;
   // cos (first half) and sin (second half) of this position's rotation angles, in shared memory: worked out in the first
@@ -154,11 +151,17 @@ __device__ __forceinline__ void decode_attn_prologue(const DecodeAttnParams& p, 
   // this CTA's tiles: [it.tile_begin, it.tile_end)
   const int first_tile = it.lo / kTileKeys;
   const int all_tiles = (it.n_keys + kTileKeys - 1) / kTileKeys - first_tile;
-  // A part is worth its merge (a trip to L2 for the partial results, one for the ticket, one back) only where the warps of the parts before it
-  // have a tile each: 57 to 89 keys in one part of three tiles instead of three parts of one.
-  it.parts = min(p.splits, (all_tiles + kWarps * kTilesPerWarp - 1) / (kWarps * kTilesPerWarp));
+  // What a request's keys are cut into decides the order its sums are taken in: parts of per_split tiles, merged in part order.  Parts of one tile each
+  // that fit the warps of one CTA are its warps (57 to 89 keys: three tiles, where eight CTAs merged through global memory and a ticket, five of them empty);
+  // the merge below adds them as it would have added parts.  Otherwise every part that has a tile is a CTA.
+  int per_split = (all_tiles + p.splits - 1) / p.splits;
+  it.parts = (all_tiles + per_split - 1) / per_split;
+  it.warps_are_parts = p.splits > 1 && per_split == 1 && all_tiles <= kWarps;
+  if (it.warps_are_parts) {
+    it.parts = 1;
+    per_split = all_tiles;
+  }
   if (it.split >= it.parts) return;
-  const int per_split = (all_tiles + it.parts - 1) / it.parts;
   it.tile_begin = first_tile + it.split * per_split;
   it.tile_end = min(first_tile + all_tiles, it.tile_begin + per_split);
 
@@ -438,14 +441,36 @@ __device__ __forceinline__ void decode_attn_main(const DecodeAttnParams& p, Deco
   for (int idx = threadIdx.x; idx < group * kD; idx += kWarps * 32) {
     const int r = idx / kD;
     const int d = idx - r * kD;
-    float m = -INFINITY;
-    for (int w = 0; w < live; ++w) m = fmaxf(m, merge_ml[(w * 16 + r) * 2]);
-    float acc = 0.0f, sum = 0.0f;
-    for (int w = 0; w < live; ++w) {
-      const float wm = merge_ml[(w * 16 + r) * 2];
-      const float f = (wm == -INFINITY) ? 0.0f : exp2f(wm - m);
-      acc += f * merge_o[((size_t)w * 16 + r) * kD + d];
-      sum += f * merge_ml[(w * 16 + r) * 2 + 1];
+    float m = -INFINITY, acc = 0.0f, sum = 0.0f;
+    if (live == kWarps && !it.warps_are_parts) {   // every warp, nothing asked per warp: a CTA in the middle of long keys waits for this
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) m = fmaxf(m, merge_ml[(w * 16 + r) * 2]);
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        const float wm = merge_ml[(w * 16 + r) * 2];
+        const float f = (wm == -INFINITY) ? 0.0f : exp2f(wm - m);
+        acc += f * merge_o[((size_t)w * 16 + r) * kD + d];
+        sum += f * merge_ml[(w * 16 + r) * 2 + 1];
+      }
+    } else {
+      float of_part[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+      static_assert(kWarps <= 8, "a part per warp");
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w)
+        if (w < live) m = fmaxf(m, merge_ml[(w * 16 + r) * 2]);
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        if (w >= live) break;
+        const float wm = merge_ml[(w * 16 + r) * 2];
+        const float f = (wm == -INFINITY) ? 0.0f : exp2f(wm - m);
+        acc += f * merge_o[((size_t)w * 16 + r) * kD + d];
+        if (it.warps_are_parts) of_part[w] = __fmul_rn(f, merge_ml[(w * 16 + r) * 2 + 1]);
+        else sum += f * merge_ml[(w * 16 + r) * 2 + 1];
+      }
+      // as a warp adds the parts' sums, a lane each (warp_sum)
+      if (it.warps_are_parts)
+        sum = __fadd_rn(__fadd_rn(__fadd_rn(of_part[0], of_part[4]), __fadd_rn(of_part[2], of_part[6])),
+                        __fadd_rn(__fadd_rn(of_part[1], of_part[5]), __fadd_rn(of_part[3], of_part[7])));
     }
     const int head = it.kvh * group + r;
     if (it.parts == 1) {

@@ -36,7 +36,6 @@ _scratch: dict[torch.device, list[torch.Tensor]] = {}
 def build_all() -> list:
     built = [build_library(f"tlie_attn_decode_d{d}", ["attention_decode.cu"], {"HEAD_DIM": d}) for d in DEFAULT_HEAD_DIMS]
     built.append(build_library("tlie_attn_decode_d64_w4", ["attention_decode.cu"], {"HEAD_DIM": 64, "DECODE_WARPS": 4, "DECODE_STAGES": 3}))
-    built.append(build_library("tlie_attn_decode_d128_w3", ["attention_decode.cu"], {"HEAD_DIM": 128, **NARROW_WIDE_HEADS}))
     built += [build_library(f"tlie_attn_prefill_d{d}", ["attention_prefill.cu"], {"HEAD_DIM": d}) for d in DEFAULT_HEAD_DIMS]
     built.append(build_library("tlie_gemv_fused", ["gemv_fused.cu"]))
     built.append(build_library("tlie_gemm_skinny", ["gemm_skinny.cu"]))
@@ -498,22 +497,15 @@ def linear_bf16(x, weight, out) -> None:
 
 
 # --- decode attention -------------------------------------------------------------------------
-NARROW_WIDE_HEADS = {"DECODE_WARPS": 3, "DECODE_STAGES": 2, "DECODE_TILES_PER_WARP": 8}   # the narrow build of head size 128
-
-
 def decode_attention_library(head_dim: int, narrow: bool = False):
     """The decode attention library of a head size.
 
-    Default build: eight warps and two stages per CTA for head sizes up to 64, four warps and two stages above (one CTA per SM
-    pulls enough bandwidth when there are few (request, kv head) pairs).  ``narrow``: two CTAs per SM, for steps with more pairs
-    than SMs, where the wide CTAs would run in two uneven waves: four warps and three stages (64 requests at 1.1B widths: 13.7 -> 9.8 us),
-    above 64 three warps and two stages (head size 128; 8 requests of 500 keys at 7B widths, 256 pairs: 20.5 -> 17.5 us; 48 of 300 to 900
-    at 8B widths, 384 pairs: 41.3 -> 36.2).
+    Default build: eight warps and two stages per CTA for head sizes up to 64 (one CTA per SM pulls enough bandwidth when
+    there are few (request, kv head) pairs).  ``narrow``: four warps and three stages, two CTAs per SM, for steps with
+    more pairs than SMs, where the wide CTAs would run in two uneven waves.
     """
     if narrow and head_dim <= 64:
         lib = load_library(f"tlie_attn_decode_d{head_dim}_w4", ["attention_decode.cu"], {"HEAD_DIM": head_dim, "DECODE_WARPS": 4, "DECODE_STAGES": 3})
-    elif narrow and head_dim == 128:
-        lib = load_library(f"tlie_attn_decode_d{head_dim}_w3", ["attention_decode.cu"], {"HEAD_DIM": head_dim, **NARROW_WIDE_HEADS})
     else:
         lib = load_library(f"tlie_attn_decode_d{head_dim}", ["attention_decode.cu"], {"HEAD_DIM": head_dim})
     if not getattr(lib, "_tlie_typed", False):
@@ -546,12 +538,7 @@ def decode_attention(qkv, pages, positions, block_table, out, q_heads: int, kv_h
     """
     ops = _ops()
     requests = qkv.shape[0]
-    narrow = requests * kv_heads > sm_count()
-    lib = decode_attention_library(head_dim, narrow=narrow)
-    if narrow and head_dim == 128 and 2 * requests * kv_heads <= 16384:
-        # requests of more than 768 keys in two parts (the kernel cuts a request into as many of the launch's parts as are worth it): 24 requests of
-        # 150 to 1,124 keys at 8B widths 25.5 -> 21.7 us (27.0 in wide CTAs)
-        splits = max(splits, 2)
+    lib = decode_attention_library(head_dim, narrow=requests * kv_heads > sm_count())
     floats = lib.tlie_decode_attention_scratch_floats(c_int(requests), c_int(q_heads), c_int(splits))
     buffer = scratch(qkv.device, floats)
     ops._check(
