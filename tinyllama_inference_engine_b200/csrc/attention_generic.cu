@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kSharedWarps * 32) paged_attention_shared_f32_
         const float new_max = fmaxf(running_max[s], warp_max(score));
         const float rescale = (active[s] && base <= pos[s]) ? expf(__fsub_rn(running_max[s], new_max)) : 1.0f;
         p[s] = seen ? expf(__fsub_rn(score, new_max)) : 0.0f;
-        running_sum[s] = __fadd_rn(__fmul_rn(running_sum[s], rescale), warp_sum(p[s]));
+        running_sum[s] = fmaf(running_sum[s], rescale, warp_sum(p[s]));
         running_max[s] = new_max;
 #pragma unroll
         for (int i = 0; i < kDims; ++i) acc[s][i] = __fmul_rn(acc[s][i], rescale);

@@ -2,8 +2,7 @@
 //
 // The reference's 32-bit model computes each output as one dot product over K in index
 // order (src/model.cpp:53-78).  These kernels keep that property on the GPU: every output
-// element is accumulated by one thread with fused multiply-adds in ascending k, one sum over the even k and one over the odd
-// k that are added at the end (a packed multiply-add advances both), so its
+// element is accumulated by one thread with fused multiply-adds in ascending k, so its
 // value depends on neither M nor N nor the kernel or tile it falls in, and no reduced-precision
 // tensor-core mode can be involved.  Three kernels, the same bits:
 //   * up to 16 rows (decoding): bound by the weights' bytes, or, for narrow products of long rows, by the chain of K dependent
@@ -19,10 +18,11 @@ namespace tlie {
 constexpr int kTile = 64;
 constexpr int kTileK = 16;
 
-// The sums over even and odd k of one output, side by side in a register pair.
-typedef unsigned long long Sums;
-__device__ __forceinline__ void multiply_add(Sums& acc, Sums a, Sums b) { asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(acc) : "l"(a), "l"(b)); }
-__device__ __forceinline__ float total(Sums acc) { return __fadd_rn(__uint_as_float((unsigned)acc), __uint_as_float((unsigned)(acc >> 32))); }
+__device__ __forceinline__ float4 read_four(unsigned addr) {   // k .. k + 3
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
+}
 
 __global__ void __launch_bounds__(256) gemm_nt_f32_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                           float* __restrict__ out, int M, int N, int K, long long lda) {
@@ -32,11 +32,11 @@ __global__ void __launch_bounds__(256) gemm_nt_f32_kernel(const float* __restric
   const int ty = threadIdx.x / 16;
   const int row0 = blockIdx.y * kTile;
   const int col0 = blockIdx.x * kTile;
-  float acc[2][4][4];   // even k, odd k
+  float acc[4][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[0][i][j] = acc[1][i][j] = 0.0f;
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
 
   for (int k0 = 0; k0 < K; k0 += kTileK) {
     for (int idx = threadIdx.x; idx < kTile * kTileK; idx += 256) {
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(256) gemm_nt_f32_kernel(const float* __restric
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[k & 1][i][j] = fmaf(a[i], b[j], acc[k & 1][i][j]);
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
     }
     __syncthreads();
   }
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(256) gemm_nt_f32_kernel(const float* __restric
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int gc = col0 + tx * 4 + j;
-      if (gc < N) out[(size_t)gr * N + gc] = __fadd_rn(acc[0][i][j], acc[1][i][j]);
+      if (gc < N) out[(size_t)gr * N + gc] = acc[i][j];
     }
   }
 }
@@ -82,7 +82,7 @@ constexpr int kStreamK = 128;        // columns of a ring stage
 constexpr int kStreamStride = kStreamK + 4;   // shared-memory row stride: 8 rows' 16-byte reads fall into different banks
 constexpr int kStreamAhead = 4;      // operands are in registers this many steps before they are used
 
-// Inside a 1.1B-shaped decode step of 4 rows (K = 2,048): 2,560 / 2,048 / 11,264 columns 15 / 14 / 29 us back to back, the plain kernel 336 / 331 / 388.
+// Back to back in a graph, K = 2,048, 4 rows: 2,560 / 2,048 / 11,264 columns 11.8 / 9.4 / 27 us, K = 5,632: 25 us (the plain kernel 336 / 331 / 388 / 901).
 // MP: rows of x, rounded up to a power of two.  One or two warps own the outputs, a thread one weight row and MM rows of x; the others only
 // copy.  STAGES: what the CTA keeps in flight.  With at most one CTA per SM that has to cover the trip to HBM by itself.
 template <int MP, int MM, int STAGES>
@@ -94,6 +94,9 @@ __global__ void __launch_bounds__(128) gemm_stream_f32_kernel(const float* __res
   constexpr int kQuads = kStreamK / 4;
   constexpr int kRows = MP / MM;
   static_assert(kRows == 1 || kRows == 2 || kRows == 4, "");
+  struct Operands {
+    float4 w[kStreamAhead], x[kStreamAhead][MM];
+  };
   const int n0 = blockIdx.x * kStreamN;
   const int chunks = (K + kStreamK - 1) / kStreamK;
   // rows past N or M repeat the last one (their outputs are not stored); columns past K are zeros.  A warp copies whole rows of a stage.
@@ -126,9 +129,9 @@ __global__ void __launch_bounds__(128) gemm_stream_f32_kernel(const float* __res
   const bool computes = turn < kWarpsNeeded && (kRows > 1 || lane < 16);
   const int n = kRows == 4 ? turn * 8 + (lane & 7) : lane & 15;
   const int m = kRows == 4 ? lane >> 3 : (kRows == 2 ? lane >> 4 : 0);
-  Sums acc[MM];
+  float acc[MM];
 #pragma unroll
-  for (int j = 0; j < MM; ++j) acc[j] = 0;
+  for (int j = 0; j < MM; ++j) acc[j] = 0.0f;
   for (int c = 0; c < chunks; ++c) {
     cp_async_wait<STAGES - 2>();
     __syncthreads();   // stage c is here for every thread, and everyone is done with the stage that is filled next
@@ -138,35 +141,47 @@ __global__ void __launch_bounds__(128) gemm_stream_f32_kernel(const float* __res
     }
     cp_async_commit();
     if (computes) {
-      const float* stage = ring + (c % STAGES) * kStageFloats;
-      const float* ws = stage + n * kStreamStride;
-      const float* xs = stage + (kStreamN + m) * kStreamStride;
-      ulonglong2 wv[kStreamAhead], xv[kStreamAhead][MM];
-      auto fetch = [&](int q) {
-        wv[q % kStreamAhead] = *reinterpret_cast<const ulonglong2*>(ws + 4 * q);
+      const unsigned stage = (unsigned)__cvta_generic_to_shared(ring + (c % STAGES) * kStageFloats);
+      const unsigned ws = stage + n * kStreamStride * 4, xs = stage + (kStreamN + m) * kStreamStride * 4;
+      // Two sets of operands in a rolled loop, one read while the other is used: what one pass of a loop reads for the next cannot be moved down to its use
+      // (unrolled, the reads are, whatever their order in the source, and every step waited for shared memory).
+      Operands even, odd;
+      auto fetch = [&](Operands& to, int group) {
 #pragma unroll
-        for (int j = 0; j < MM; ++j) xv[q % kStreamAhead][j] = *reinterpret_cast<const ulonglong2*>(xs + j * kRows * kStreamStride + 4 * q);
+        for (int i = 0; i < kStreamAhead; ++i) {
+          to.w[i] = read_four(ws + 16 * (group * kStreamAhead + i));
+#pragma unroll
+          for (int j = 0; j < MM; ++j) to.x[i][j] = read_four(xs + j * kRows * kStreamStride * 4 + 16 * (group * kStreamAhead + i));
+        }
       };
+      auto use = [&](const Operands& from) {
 #pragma unroll
-      for (int q = 0; q < kStreamAhead; ++q) fetch(q);
+        for (int i = 0; i < kStreamAhead; ++i) {
 #pragma unroll
-      for (int q = 0; q < kQuads; ++q) {
-        const ulonglong2 wq = wv[q % kStreamAhead];
-        ulonglong2 xq[MM];
+          for (int j = 0; j < MM; ++j) acc[j] = fmaf(from.x[i][j].x, from.w[i].x, acc[j]);
 #pragma unroll
-        for (int j = 0; j < MM; ++j) xq[j] = xv[q % kStreamAhead][j];
-        if (q + kStreamAhead < kQuads) fetch(q + kStreamAhead);
+          for (int j = 0; j < MM; ++j) acc[j] = fmaf(from.x[i][j].y, from.w[i].y, acc[j]);
 #pragma unroll
-        for (int j = 0; j < MM; ++j) multiply_add(acc[j], xq[j].x, wq.x);
+          for (int j = 0; j < MM; ++j) acc[j] = fmaf(from.x[i][j].z, from.w[i].z, acc[j]);
 #pragma unroll
-        for (int j = 0; j < MM; ++j) multiply_add(acc[j], xq[j].y, wq.y);
+          for (int j = 0; j < MM; ++j) acc[j] = fmaf(from.x[i][j].w, from.w[i].w, acc[j]);
+        }
+      };
+      constexpr int kGroups = kQuads / kStreamAhead;
+      fetch(even, 0);
+#pragma unroll 1
+      for (int group = 0; group < kGroups; group += 2) {
+        fetch(odd, group + 1);
+        use(even);
+        fetch(even, group + 2 < kGroups ? group + 2 : 0);   // (the last pass reads something it has)
+        use(odd);
       }
     }
   }
   if (!computes || n0 + n >= N) return;
 #pragma unroll
   for (int j = 0; j < MM; ++j)
-    if (m + j * kRows < M) out[(size_t)(m + j * kRows) * N + n0 + n] = total(acc[j]);
+    if (m + j * kRows < M) out[(size_t)(m + j * kRows) * N + n0 + n] = acc[j];
 }
 
 template <int MP, int MM, int STAGES>
@@ -190,7 +205,8 @@ constexpr int kWideStride = kWideK + 4;   // as above: 8 rows' 16-byte reads in 
 
 // A warp is 4 x 8 lanes, a lane TM x TN outputs: rows lane / 8 + 4 i, columns lane % 8 + 8 j (the eight lanes of one pass over the banks read eight
 // neighbouring weight rows, and one row of x).  Held back by what shared memory delivers, 16 values of four bytes per lane and k in the time of 64
-// multiply-adds: 45 TFLOP/s at 2,048 rows with 8 x 8 outputs per lane, of 72 (the plain kernel: 22; 8 x 16 outputs in twice the registers: 44).
+// multiply-adds: 45 TFLOP/s at 2,048 rows with 8 x 8 outputs per lane, of 72 (the plain kernel: 22; 8 x 16 outputs in twice the registers: 44; the next step's
+// operands read into a second set of registers: 43).
 template <int TM, int TN, int WM, int WN>
 __global__ void __launch_bounds__(WM * WN * 32) gemm_wide_f32_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                      float* __restrict__ out, int M, int N, int K, long long lda) {
@@ -228,11 +244,11 @@ __global__ void __launch_bounds__(WM * WN * 32) gemm_wide_f32_kernel(const float
   }
   const int m_of = (warp % WM) * TM * LM + (lane >> 3);
   const int n_of = (warp / WM) * TN * LN + (lane & 7);
-  Sums acc[TM][TN];
+  float acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0;
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
   for (int c = 0; c < chunks; ++c) {
     cp_async_wait<kTileStages - 2>();
     __syncthreads();
@@ -242,16 +258,20 @@ __global__ void __launch_bounds__(WM * WN * 32) gemm_wide_f32_kernel(const float
     const float* ws = ring + (c % kTileStages) * kStageFloats + (BM + n_of) * kWideStride;
 #pragma unroll
     for (int q = 0; q < kWideK / 4; ++q) {
-      ulonglong2 a[TM];
+      float4 a[TM];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xs + LM * i * kWideStride + 4 * q);
+      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(xs + LM * i * kWideStride + 4 * q);
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
-        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(ws + LN * j * kWideStride + 4 * q);
+        const float4 b = *reinterpret_cast<const float4*>(ws + LN * j * kWideStride + 4 * q);
 #pragma unroll
-        for (int i = 0; i < TM; ++i) multiply_add(acc[i][j], a[i].x, b.x);
+        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].x, b.x, acc[i][j]);
 #pragma unroll
-        for (int i = 0; i < TM; ++i) multiply_add(acc[i][j], a[i].y, b.y);
+        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].y, b.y, acc[i][j]);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].z, b.z, acc[i][j]);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].w, b.w, acc[i][j]);
       }
     }
   }
@@ -261,7 +281,7 @@ __global__ void __launch_bounds__(WM * WN * 32) gemm_wide_f32_kernel(const float
     if (row >= M) break;
 #pragma unroll
     for (int j = 0; j < TN; ++j)
-      if (col0 + n_of + LN * j < N) out[(size_t)row * N + col0 + n_of + LN * j] = total(acc[i][j]);
+      if (col0 + n_of + LN * j < N) out[(size_t)row * N + col0 + n_of + LN * j] = acc[i][j];
   }
 }
 
