@@ -224,6 +224,31 @@ def test_embedding_survives_an_id_outside_the_table_and_reports_it(ops):
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("rows", [1, 3, 1023, 1024, 1027])
+def test_rows_of_eight_at_a_time(ops, rows):
+    """Embedding, gate and rotation in pieces of eight elements: widths of whole pieces and others, rotation with one token per block and with four."""
+    torch.manual_seed(37)
+    for width in (8, 2048, 2056, 2052, 131):
+        table, ids = torch.randn(50, width).bfloat16(), torch.randint(0, 50, (rows,), dtype=torch.int32)
+        got = torch.empty(rows, width, device="cuda")
+        ops.embedding(table.cuda(), ids.cuda(), got)
+        assert torch.equal(got.cpu(), table.float()[ids.long()])
+        gate_up = torch.randn(rows, 2 * width).bfloat16()
+        want, got = torch.empty(rows, width, dtype=torch.bfloat16), torch.empty(rows, width, dtype=torch.bfloat16, device="cuda")
+        plain_ops.silu_mul(gate_up, want)
+        ops.silu_mul(gate_up.cuda(), got)
+        assert torch.allclose(got.cpu().float(), want.float(), atol=_tol(torch.bfloat16, 4), rtol=_tol(torch.bfloat16))
+    rng = np.random.default_rng(37)
+    qkv, pages, positions, token_seq, table = _paged_case(rng, torch.bfloat16, [rows], [rows], 2, 64, 64, 6)
+    inv_freq = torch.from_numpy(np.power(np.float32(1e4), np.float32(-2.0) * np.arange(16, dtype=np.float32) / np.float32(32)))
+    qkv_plain, pages_plain = qkv.clone(), pages.clone()
+    plain_ops.rope_store(qkv_plain, positions, token_seq, table, inv_freq, 32, pages_plain, 6, 2, 64, 64, True)
+    qkv_gpu, pages_gpu = qkv.clone().cuda(), pages.clone().cuda()
+    ops.rope_store(qkv_gpu, positions.cuda(), token_seq.cuda(), table.cuda(), inv_freq.cuda(), 32, pages_gpu, 6, 2, 64, 64, True)
+    assert torch.allclose(qkv_gpu.cpu().float(), qkv_plain.float(), atol=_tol(torch.bfloat16, 4) + 2e-4)
+    assert torch.allclose(pages_gpu.cpu().float(), pages_plain.float(), atol=_tol(torch.bfloat16, 4) + 2e-4)
+
+
 def test_sampling_non_finite_logits_still_gives_a_token_of_the_vocabulary(ops):
     vocab = 131
     logits = torch.randn(6, vocab)

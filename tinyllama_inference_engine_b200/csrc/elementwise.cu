@@ -24,6 +24,37 @@ __global__ void embedding_kernel(const T* __restrict__ table, const int* __restr
   for (int i = threadIdx.x; i < hidden; i += blockDim.x) dst[i] = to_float(src[i]);
 }
 
+// The same eight elements at a time (hidden % 8 == 0, 16-byte aligned): 8,192 rows of 4,096 took 68 us element by element, 38 so, ncu; a step of one
+// row 6.6 us and 3.1.
+__device__ __forceinline__ void load8(const float* p, float4& a, float4& b) {
+  a = reinterpret_cast<const float4*>(p)[0];
+  b = reinterpret_cast<const float4*>(p)[1];
+}
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float4& a, float4& b) {
+  const uint4 raw = *reinterpret_cast<const uint4*>(p);
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  a = make_float4(__bfloat162float(h[0].x), __bfloat162float(h[0].y), __bfloat162float(h[1].x), __bfloat162float(h[1].y));
+  b = make_float4(__bfloat162float(h[2].x), __bfloat162float(h[2].y), __bfloat162float(h[3].x), __bfloat162float(h[3].y));
+}
+template <typename T>
+__global__ void __launch_bounds__(256) embedding_vec_kernel(const T* __restrict__ table, const int* __restrict__ ids, float* __restrict__ residual, int hidden,
+                                                            int vocab, int* __restrict__ error_flag) {
+  const int row = blockIdx.x;
+  int id = ids[row];
+  if (id < 0 || id >= vocab) {
+    if (threadIdx.x == 0 && error_flag != nullptr) atomicOr(error_flag, 2);
+    id = 0;
+  }
+  const T* src = table + (size_t)id * hidden;
+  float* dst = residual + (size_t)row * hidden;
+  for (int i = threadIdx.x * 8; i < hidden; i += 256 * 8) {
+    float4 a, b;
+    load8(src + i, a, b);
+    reinterpret_cast<float4*>(dst + i)[0] = a;
+    reinterpret_cast<float4*>(dst + i)[1] = b;
+  }
+}
+
 // Optional add, then RMSNorm.  For output row r the source row is rows ? rows[r] : r.
 //   if delta:  residual[src, :] += float(delta[src, :])        (32-bit sum, stored back)
 //   scale = 1 / sqrt(mean(residual[src]^2) + eps);  out[r, :] = (x * scale) * weight
@@ -206,6 +237,26 @@ __global__ void silu_mul_vec_kernel(const T* __restrict__ gate_up, T* __restrict
   }
 }
 
+// The same for bfloat16, eight neighbours per thread (inter % 8 == 0, 16-byte aligned), a block a run of one row's columns: no division per element,
+// wide accesses, and a programmatic launch.  (931 rows of 5,632: 11.0 us with the kernel above and its 64-bit division per four elements, 9.6 with this one, ncu.)
+__global__ void __launch_bounds__(256) gate_mul_rows_kernel(const __nv_bfloat16* __restrict__ gate_up, __nv_bfloat16* __restrict__ out, int inter, int blocks_per_row,
+                                                            int kind) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int row = blockIdx.x / blocks_per_row;
+  const int col = ((blockIdx.x - row * blocks_per_row) * 256 + threadIdx.x) * 8;
+  if (col >= inter) return;
+  float4 g0, g1, u0, u1;
+  load8(gate_up + (size_t)row * 2 * inter + col, g0, g1);
+  load8(gate_up + (size_t)row * 2 * inter + inter + col, u0, u1);
+  __nv_bfloat162 packed[4];
+  packed[0] = __floats2bfloat162_rn(gate_act(g0.x, kind) * u0.x, gate_act(g0.y, kind) * u0.y);
+  packed[1] = __floats2bfloat162_rn(gate_act(g0.z, kind) * u0.z, gate_act(g0.w, kind) * u0.w);
+  packed[2] = __floats2bfloat162_rn(gate_act(g1.x, kind) * u1.x, gate_act(g1.y, kind) * u1.y);
+  packed[3] = __floats2bfloat162_rn(gate_act(g1.z, kind) * u1.z, gate_act(g1.w, kind) * u1.w);
+  *reinterpret_cast<uint4*>(out + (size_t)row * inter + col) = *reinterpret_cast<uint4*>(packed);
+}
+
 // residual[t, :] += float(delta[t, :]) without a norm (the last add when no norm follows).
 template <typename T>
 __global__ void add_kernel(float* __restrict__ residual, const T* __restrict__ delta, size_t count) {
@@ -362,6 +413,13 @@ TLIE_EXPORT int tlie_embedding(int dtype, const void* table, const int* ids, flo
                                int* error_flag, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (vocab <= 0) return (int)cudaErrorInvalidValue;
+  if (hidden % 8 == 0 && ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(residual)) & 15) == 0) {
+    if (dtype == TLIE_F32)
+      embedding_vec_kernel<float><<<rows, 256, 0, stream>>>((const float*)table, ids, residual, hidden, vocab, error_flag);
+    else
+      embedding_vec_kernel<__nv_bfloat16><<<rows, 256, 0, stream>>>((const __nv_bfloat16*)table, ids, residual, hidden, vocab, error_flag);
+    return (int)cudaGetLastError();
+  }
   if (dtype == TLIE_F32)
     embedding_kernel<float><<<rows, 256, 0, stream>>>((const float*)table, ids, residual, hidden, vocab, error_flag);
   else
@@ -436,6 +494,11 @@ TLIE_EXPORT int tlie_gate_mul(int dtype, const void* gate_up, void* out, int row
   if (kind < 0 || kind > 1) return (int)cudaErrorInvalidValue;
   const size_t total = (size_t)rows * inter;
   if (total == 0) return 0;
+  const int blocks_per_row = (inter / 8 + 255) / 256;
+  if (dtype == TLIE_BF16 && inter % 8 == 0 && ((reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 &&
+      (long long)rows * blocks_per_row <= 0x7fffffff)
+    return (int)launch_pdl(gate_mul_rows_kernel, dim3((unsigned)(rows * blocks_per_row)), dim3(256), 0, stream, (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)out, inter,
+                           blocks_per_row, kind);
   if (inter % 4 == 0) {
     const size_t total4 = total / 4;
     const size_t most = (size_t)device_sm_count() * 32;
