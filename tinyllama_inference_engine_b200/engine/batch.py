@@ -1,6 +1,7 @@
 """One step's batch: requests' next tokens, flattened, with everything a kernel needs to find the cache."""
 from __future__ import annotations
 
+from array import array
 from dataclasses import dataclass, field
 from itertools import chain
 
@@ -90,17 +91,33 @@ class StepContext:
         return self.plans.get(name)
 
 
-def lay_out_step(entries: list[StepEntry], first_positions: list[int], slots: list[int], table_rows: list[list[list[int]]]) -> dict:
+def token_array(tokens) -> np.ndarray | None:
+    """The tokens as int32 (None: something only a Python loop can make sense of).  A prompt is read once so: its range check and its place in the
+    step's description work on the array."""
+    if isinstance(tokens, (bytes, bytearray)):
+        return None   # array() would take those for the words themselves
+    try:
+        return np.frombuffer(array("i", tokens), dtype=np.int32)
+    except (TypeError, OverflowError):
+        return None
+
+
+def lay_out_step(entries: list[StepEntry], first_positions: list[int], slots: list[int], table_rows: list[list[list[int]]],
+                 arrays: list | None = None) -> dict:
     """The step as one flat array of int32 words and where its sections lie (host work only).
 
-    Sections that have a word per token are made with numpy (a 2,048-token portion costs 0.1 ms so, 0.3 ms as Python lists)."""
+    Sections that have a word per token are made with numpy (a 2,048-token portion costs 0.1 ms so, 0.3 ms as Python lists).
+    ``arrays``: the entries' tokens as ``token_array`` gives them, where the caller has them."""
     q_lens = [len(e.tokens) for e in entries]
     num_tokens, num_seqs = sum(q_lens), len(entries)
     lens = np.asarray(q_lens, dtype=np.int32)
     starts = np.zeros(num_seqs + 1, dtype=np.int32)
     np.cumsum(lens, out=starts[1:])
     seq_starts = starts.tolist()
-    token_ids = np.fromiter(chain.from_iterable(e.tokens for e in entries), dtype=np.int32, count=num_tokens)
+    if arrays is not None and all(a is not None for a in arrays):
+        token_ids = arrays[0] if num_seqs == 1 else np.concatenate(arrays)
+    else:
+        token_ids = np.fromiter(chain.from_iterable(e.tokens for e in entries), dtype=np.int32, count=num_tokens)
     shift = np.asarray(first_positions, dtype=np.int32) - starts[:-1]           # position of a row = its index + its entry's shift
     positions = np.arange(num_tokens, dtype=np.int32) + np.repeat(shift, lens)
     token_seq = np.repeat(np.arange(num_seqs, dtype=np.int32), lens)
@@ -124,13 +141,22 @@ def lay_out_step(entries: list[StepEntry], first_positions: list[int], slots: li
             "num_tokens": num_tokens, "num_seqs": num_seqs, "want_rows": want_rows}
 
 
+def refresh_step(layout: dict, into: tuple) -> None:
+    """Write a step's layout into (pinned host tensor, device tensor): all that a replay of its captured kernels needs."""
+    flat = layout["flat"]
+    host, buffer = into
+    host.numpy()[: len(flat)] = flat
+    buffer[: len(flat)].copy_(host[: len(flat)], non_blocking=True)
+
+
 def pack_step(entries: list[StepEntry], first_positions: list[int], slots: list[int], table_rows: list[list[list[int]]],
-              device: torch.device, into: tuple | None = None) -> StepContext:
+              device: torch.device, into: tuple | None = None, arrays: list | None = None) -> StepContext:
     """Flatten the entries into one int32 buffer, copy it once, and slice the views.
 
     ``into``: (pinned host tensor, device tensor) of fixed address to write and copy into, for a step whose kernels were captured
-    in a CUDA graph and read their description from there; they must be at least as long as the step's layout."""
-    layout = lay_out_step(entries, first_positions, slots, table_rows)
+    in a CUDA graph and read their description from there; they must be at least as long as the step's layout.
+    ``arrays``: see ``lay_out_step``."""
+    layout = lay_out_step(entries, first_positions, slots, table_rows, arrays)
     flat, offsets, table_offsets, plans = layout["flat"], layout["offsets"], layout["table_offsets"], layout["plans"]
     if into is None:
         host = torch.from_numpy(flat)
@@ -138,9 +164,8 @@ def pack_step(entries: list[StepEntry], first_positions: list[int], slots: list[
             host = host.pin_memory()
         buffer = host.to(device, non_blocking=True)
     else:
-        host, buffer = into
-        host.numpy()[: len(flat)] = flat
-        buffer[: len(flat)].copy_(host[: len(flat)], non_blocking=True)
+        refresh_step(layout, into)
+        buffer = into[1]
     views = [buffer[o : o + n] for o, n in offsets]
     tables = [buffer[o : o + b * w].view(b, w) for o, b, w in table_offsets]
     want_rows, num_tokens = layout["want_rows"], layout["num_tokens"]
@@ -159,7 +184,7 @@ def step_shape(entries: list[StepEntry], first_positions: list[int]) -> tuple:
     """What of a step decides its kernels, their launch shapes and its buffer's layout: every entry's number of tokens and of wanted
     places, whether all rows are wanted in order, and whether every entry begins its request.  Everything else about it is data the
     kernels read on the device."""
-    in_order = all(entry.want == list(range(len(entry.tokens))) for entry in entries)
+    in_order = all(len(entry.want) == len(entry.tokens) and entry.want == list(range(len(entry.tokens))) for entry in entries)
     return tuple((len(entry.tokens), len(entry.want)) for entry in entries) + (in_order, not any(first_positions))
 
 

@@ -18,7 +18,7 @@ from ..errors import BatchError, KernelError
 from ..models import DecoderModel, expected_tensors
 from ..parts.base import Runtime, Workspace
 from ..weights import WeightStore
-from .batch import StepContext, StepEntry, lay_out_step, pack_step, step_shape
+from .batch import StepContext, StepEntry, lay_out_step, pack_step, refresh_step, step_shape, token_array
 from .timing import StepClock, StepTimings
 
 _TORCH_DTYPES = {"bfloat16": torch.bfloat16, "float32": torch.float32}
@@ -37,22 +37,26 @@ class GraphedStep:
         self.graph: torch.cuda.CUDAGraph | None = None
         self.logits: torch.Tensor | None = None
 
-    def run(self, runner: "ModelRunner", entries, firsts, slots, table_rows) -> torch.Tensor | None:
+    def run(self, runner: "ModelRunner", entries, firsts, slots, table_rows, arrays) -> torch.Tensor | None:
+        if self.graph is not None:
+            # the kernels know their views of the description: it only has to be written anew
+            layout = lay_out_step(entries, firsts, slots, table_rows, arrays)
+            # The host may be steps ahead of the device (nothing reads a prompt portion without wanted logits): the pinned buffer
+            # is written again only once the copy that a step before this one queued from it has been done.
+            self.copied.synchronize()
+            refresh_step(layout, (self.host, self.device))
+            self.copied.record()
+            self.graph.replay()
+            return None if self.logits is None else self.logits.clone()   # the graph's own memory is written again by the next replay
         if self.host is None:
-            words = len(lay_out_step(entries, firsts, slots, table_rows)["flat"])
+            words = len(lay_out_step(entries, firsts, slots, table_rows, arrays)["flat"])
             self.host = torch.zeros(words, dtype=torch.int32).pin_memory()
             self.device = torch.zeros(words, dtype=torch.int32, device=runner.device)
             self.copied = torch.cuda.Event()
-        # The host may be steps ahead of the device (nothing reads a prompt portion without wanted logits): the pinned buffer
-        # is written again only once the copy that a step before this one queued from it has been done.
-        self.copied.synchronize()
-        ctx = pack_step(entries, firsts, slots, table_rows, runner.device, into=(self.host, self.device))
+        ctx = pack_step(entries, firsts, slots, table_rows, runner.device, into=(self.host, self.device), arrays=arrays)
         self.copied.record()
         # launch shapes chosen from the context length must hold for every later step of this shape
         ctx.max_seq_len = runner.spec.max_positions
-        if self.graph is not None:
-            self.graph.replay()
-            return None if self.logits is None else self.logits.clone()   # the graph's own memory is written again by the next replay
         # This use runs kernel by kernel (with the settings the capture will have, so that every library and buffer it needs
         # exists), then the same launches are recorded for the uses to come.
         logits = runner.run(ctx)
@@ -100,10 +104,14 @@ class ModelRunner:
     # --- the step --------------------------------------------------------------------------
     def validate(self, entries: list[StepEntry]) -> list[int]:
         """Check a batch without changing anything; returns each entry's first position."""
+        return self._validate(entries)[0]
+
+    def _validate(self, entries: list[StepEntry]) -> tuple[list[int], list]:
+        """Each entry's first position, and its tokens as an array (None for a few tokens, where a list is as quick)."""
         if not entries:
             raise BatchError("a step needs at least one entry")
         seen = set()
-        firsts = []
+        firsts, arrays = [], []
         vocab = self.spec.vocab_size
         new_requests = 0
         for entry in entries:
@@ -112,7 +120,10 @@ class ModelRunner:
             seen.add(entry.request_id)
             if not entry.tokens:
                 raise BatchError(f"request {entry.request_id!r} brings no tokens")
-            if min(entry.tokens) < 0 or max(entry.tokens) >= vocab:
+            tokens = token_array(entry.tokens) if len(entry.tokens) > 16 else None
+            arrays.append(tokens)
+            lowest, highest = (min(entry.tokens), max(entry.tokens)) if tokens is None else (tokens.min(), tokens.max())
+            if lowest < 0 or highest >= vocab:
                 token = next(token for token in entry.tokens if not 0 <= token < vocab)
                 raise BatchError(f"token {token} of request {entry.request_id!r} is outside the vocabulary of {vocab}")
             for place in entry.want:
@@ -130,7 +141,7 @@ class ModelRunner:
             raise BatchError(f"the step brings {total} tokens; max_batch_tokens is {self.engine_config.max_batch_tokens}")
         if len(self.cache.records) + new_requests > self.cache.max_requests:
             raise BatchError(f"more than {self.cache.max_requests} live requests")
-        return firsts
+        return firsts, arrays
 
     def step(self, entries: list[StepEntry], timings: StepTimings | None = None, trace: dict | None = None) -> torch.Tensor | None:
         """Run the entries as one batch; returns 32-bit logits [wanted, vocab] (None if nothing is wanted).
@@ -139,7 +150,7 @@ class ModelRunner:
         state after every run of a layer, ``trace["layer<i>.output"]`` [rows, hidden] in 32-bit, as the reference's traced
         forward keeps them (src/model.cpp:98-100, 200-206), so that a wrong logit can be followed back to its layer."""
         clock = StepClock(self.device, timings is not None)
-        firsts = self.validate(entries)
+        firsts, arrays = self._validate(entries)
         wanted = [(e.request_id if self.cache.has(e.request_id) else None, f + len(e.tokens)) for e, f in zip(entries, firsts)]
         if not self.cache.can_reserve(wanted):
             from ..errors import OutOfPages
@@ -155,9 +166,9 @@ class ModelRunner:
         table_rows = [self.cache.block_table_rows(group, ids) for group in self.cache.page_groups]
         graphed = self._graphed_step(entries, firsts) if timings is None and trace is None else None
         if graphed is not None:
-            logits = graphed.run(self, entries, firsts, slots, table_rows)
+            logits = graphed.run(self, entries, firsts, slots, table_rows, arrays)
         else:
-            ctx = pack_step(entries, firsts, slots, table_rows, self.device)
+            ctx = pack_step(entries, firsts, slots, table_rows, self.device, arrays=arrays)
             clock.mark()
             logits = self.run(ctx, trace)
             clock.mark()

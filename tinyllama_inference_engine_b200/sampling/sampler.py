@@ -20,7 +20,8 @@ class Sampler:
     def select(self, logits: torch.Tensor, params: list, draw_indices: list[int]) -> list[int]:
         """One token per row of ``logits`` (32-bit, [rows, vocab]); ``params[i]`` has temperature, top_p, seed."""
         rows = logits.shape[0]
-        out = torch.empty(rows, dtype=torch.int32, device=logits.device)
+        both = torch.empty(rows + 1, dtype=torch.int32, device=logits.device)   # the tokens, and behind them the device error word: one trip to the host
+        out = both[:rows]
         if all(not p.temperature > 0.0 for p in params):
             ops.argmax(logits, out)
         else:
@@ -28,6 +29,7 @@ class Sampler:
             seeds = torch.tensor([[p.seed, k] for p, k in zip(params, draw_indices)], dtype=torch.int64)
             host, seeds = host.to(logits.device), seeds.to(logits.device)
             ops.sample(logits, host[:, 0].contiguous(), host[:, 1].contiguous(), seeds[:, 0].contiguous(), seeds[:, 1].contiguous(), out)
-        tokens = out.cpu().tolist()                 # the host waits for the step here,
-        ops.check_device_errors(logits.device)      # so this is where a fault a kernel recorded on the device surfaces
+        both[rows:].copy_(ops.error_flag(logits.device))
+        *tokens, word = both.cpu().tolist()              # the host waits for the step here,
+        ops.raise_for_error_word(word, logits.device)    # so this is where a fault a kernel recorded on the device surfaces
         return tokens
