@@ -299,3 +299,28 @@ def test_steps_of_one_shape_queued_without_waiting_keep_their_own_descriptions(m
     got = logits(wait=False)
     for index, (a, b) in enumerate(zip(got, want)):
         assert torch.equal(a, b), index
+
+
+@pytest.mark.parametrize("dtype,lengths", [("float32", [200, 17, 90]), ("bfloat16", [1200, 17, 831])])
+def test_last_layer_of_the_wanted_rows_alone_gives_their_logits(tmp_path, dtype, lengths):
+    """Few wanted rows of many (one, several of an entry out of order, one twice, up to half of the step): the bits of a step that shows every row of every layer."""
+    from tinyllama_inference_engine_b200.weights import write_random_model
+
+    folder = write_random_model(tmp_path / "m", dict(tiny_configs.TINY_B, hidden_size=2048, intermediate_size=5632, num_hidden_layers=2, num_attention_heads=32,
+                                                     num_key_value_heads=4, head_dim=64, vocab_size=512, max_position_embeddings=2048), seed=3)
+    runner = ModelRunner(folder, EngineConfig(dtype=dtype, page_size=64, max_cache_tokens=4096, max_requests=8, max_batch_tokens=2048, use_cuda_graphs=False))
+    prompts = _prompts(runner.spec.vocab_size, lengths, seed=41)
+    assert runner.model.blocks[-1].keeps_wanted_rows(sum(lengths)) and (dtype == "float32" or not runner.model.blocks[-1].keeps_wanted_rows(300))
+
+    def logits(wants, trace=None):
+        got = runner.step([StepEntry(f"r{i}", p, w) for i, (p, w) in enumerate(zip(prompts, wants))], trace=trace)
+        for i in range(len(prompts)):
+            runner.finish(f"r{i}")
+        return got
+
+    a, b, c = lengths
+    for wants in ([[a - 1], [], []], [[a - 1], [b - 1], [c - 1]], [[5, 3, a - 1, 3], [], [0]], [list(range(40, 60)), [b - 1, 0], [1]], [list(range(b * 8)), [], list(range(13))]):
+        trace = {}
+        want = logits(wants, trace)
+        assert all(value.shape[0] == sum(lengths) for value in trace.values())
+        assert torch.equal(logits(wants), want), wants

@@ -249,6 +249,16 @@ def test_rows_of_eight_at_a_time(ops, rows):
     assert torch.allclose(pages_gpu.cpu().float(), pages_plain.float(), atol=_tol(torch.bfloat16, 4) + 2e-4)
 
 
+@pytest.mark.parametrize("dtype,width", [(torch.float32, 2048), (torch.bfloat16, 4096), (torch.bfloat16, 131), (torch.float32, 3)])
+def test_gather_rows(ops, dtype, width):
+    x = torch.randn(40, width).to(dtype).cuda()
+    for rows in ([39], [0, 7, 7, 3], list(range(39, -1, -1))):
+        index = torch.tensor(rows, dtype=torch.int32).cuda()
+        out = torch.empty(len(rows), width, dtype=dtype, device="cuda")
+        ops.gather_rows(x, index, out)
+        assert torch.equal(out, x[index.long()])
+
+
 def test_sampling_non_finite_logits_still_gives_a_token_of_the_vocabulary(ops):
     vocab = 131
     logits = torch.randn(6, vocab)

@@ -427,10 +427,11 @@ TLIE_EXPORT int tlie_embedding(int dtype, const void* table, const int* ids, flo
   return (int)cudaGetLastError();
 }
 
+// many_rows: take the kernel for many rows whatever their number (a few rows of a prompt portion, with the bits they have among all of it).
 TLIE_EXPORT int tlie_add_rmsnorm(int dtype, float* residual, const void* delta, const int* rows, const float* weight,
-                                 float eps, void* out, int out_rows, int hidden, cudaStream_t stream) {
+                                 float eps, void* out, int out_rows, int hidden, int many_rows, cudaStream_t stream) {
   if (out_rows <= 0) return 0;
-  if (dtype == TLIE_BF16 && hidden % 4 == 0 && hidden <= 32 * kRowChunks * 4 && out_rows >= 256) {
+  if (dtype == TLIE_BF16 && hidden % 4 == 0 && hidden <= 32 * kRowChunks * 4 && (out_rows >= 256 || many_rows)) {
     // many rows (a prompt portion): a warp per row
     const dim3 grid((out_rows + kRowWarps - 1) / kRowWarps), block(kRowWarps * 32);
     if (hidden <= 32 * 16 * 4)

@@ -9,11 +9,22 @@
 //   head_linear         out[t, h, :] = W[h] . x[t, h, :]  per head, operands with strides of their own, 32-bit sums in a fixed order; optionally gated
 //   sigmoid_gate        x[t, i] *= sigmoid(gate[t, i])
 //   add_bias            x[t, i] += bias[i]
+//   gather_rows         out[t, :] = x[rows[t], :]                                      the rows of a step that are still read
 // Storage float or bfloat16, arithmetic 32-bit.
 #include "common.cuh"
 #include "mma_utils.cuh"
 
 namespace tlie {
+
+// A block per row, in units of 16 bytes where rows allow it, else of 2.
+template <typename U>
+__global__ void __launch_bounds__(256) gather_rows_kernel(const U* __restrict__ x, const int* __restrict__ rows, U* __restrict__ out, int units) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const U* src = x + (size_t)rows[blockIdx.x] * units;
+  U* dst = out + (size_t)blockIdx.x * units;
+  for (int i = threadIdx.x; i < units; i += 256) dst[i] = src[i];
+}
 
 template <typename T>
 __global__ void add_row_vector_kernel(float* __restrict__ residual, const T* __restrict__ delta, const float* __restrict__ vector, int hidden, size_t total) {
@@ -334,4 +345,13 @@ TLIE_EXPORT int tlie_sigmoid_gate(int dtype, void* x, long long x_row, const voi
   }
   TLIE_BY_TYPE(dtype, (sigmoid_gate_kernel<T><<<blocks_for(total, 256), 256, 0, stream>>>((T*)x, x_row, (const T*)gate, gate_row, width, total)));
   return (int)cudaGetLastError();
+}
+
+// Rows of row_bytes bytes (an even number).
+TLIE_EXPORT int tlie_gather_rows(const void* x, const int* rows, void* out, int count, int row_bytes, cudaStream_t stream) {
+  if (count <= 0 || row_bytes <= 0) return 0;
+  if (row_bytes & 1) return (int)cudaErrorInvalidValue;
+  if (row_bytes % 16 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) == 0)
+    return (int)launch_pdl(gather_rows_kernel<uint4>, dim3(count), dim3(256), 0, stream, (const uint4*)x, rows, (uint4*)out, row_bytes / 16);
+  return (int)launch_pdl(gather_rows_kernel<unsigned short>, dim3(count), dim3(256), 0, stream, (const unsigned short*)x, rows, (unsigned short*)out, row_bytes / 2);
 }

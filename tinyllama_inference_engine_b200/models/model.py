@@ -50,14 +50,15 @@ class DecoderModel:
         """Logits (32-bit, [len(want_rows), vocab]) of the rows ``ctx.want_rows``.
 
         ``trace``: a dictionary that receives the hidden state of all rows after every run of a layer (32-bit copies)."""
-        hidden, pending = self._run_blocks(ctx, caches, trace)
-        return self.logits(hidden, ctx.want_rows, pending if ctx.wants_every_row_in_order else None)
+        hidden, pending, wanted_only = self._run_blocks(ctx, caches, trace, wanted=True)
+        return self.logits(hidden, ctx.want_rows, pending if ctx.wants_every_row_in_order else None, wanted_only)
 
     def forward_hidden(self, ctx, caches: dict[int, LayerCache]):
         return self._run_blocks(ctx, caches)[0]
 
-    def _run_blocks(self, ctx, caches: dict[int, LayerCache], trace: dict | None = None):
-        """The complete residual stream of the step's rows, and a lazy final norm of it if the last block left one prepared."""
+    def _run_blocks(self, ctx, caches: dict[int, LayerCache], trace: dict | None = None, wanted: bool = False):
+        """The complete residual stream of the step's rows, a lazy final norm of it if the last block left one prepared, and whether the rows are
+        the wanted ones alone (only with ``wanted``, and not in a trace, which shows every row of every layer)."""
         from .. import ops
 
         if EMBEDDING_STREAM in self.cache_needs:
@@ -65,13 +66,20 @@ class DecoderModel:
         else:
             residual = self.embedding.forward(ctx.token_ids, ctx)
         pending = None
+        wanted_only = False
         order = self.spec.order
+        want_rows = ctx.want_rows
         for index, entry in enumerate(order):
             cache = caches[entry.cache]
             if cache.writes != entry.writes_cache:
                 cache = LayerCache(cache.need, entry.writes_cache, cache.pages, cache.block_table, cache.page_size, cache.state, cache.plane_pages)
             block = self.blocks[entry.layer]
-            if block.accepts_next_norm:
+            if (wanted and trace is None and index + 1 == len(order) and want_rows is not None and want_rows.shape[0] > 0
+                    and ops.wanted_rows_pay(residual.shape[0], want_rows.shape[0], residual.device)
+                    and hasattr(block, "keeps_wanted_rows") and block.keeps_wanted_rows(residual.shape[0])):
+                residual, pending = block.forward_wanted(residual, pending, ctx, cache, want_rows)
+                wanted_only = True
+            elif block.accepts_next_norm:
                 # the norm that reads this block's result: the next block's first one (if it names one), or the final norm
                 following = self.blocks[order[index + 1].layer].first_norm if index + 1 < len(order) else self.final_norm
                 residual, pending = block.forward(residual, pending, ctx, cache, next_norm=following)
@@ -84,13 +92,14 @@ class DecoderModel:
                 complete = residual if pending is None or isinstance(pending, ops.LazyNorm) else residual + pending.float()
                 trace[f"layer{len(trace)}.output"] = complete.float().clone()
         if isinstance(pending, ops.LazyNorm):
-            return residual, pending
+            return residual, pending, wanted_only
         if pending is not None:
             ops.add_(residual, pending)
-        return residual, None
+        return residual, None, wanted_only
 
-    def logits(self, residual, want_rows, prepared=None):
-        """``prepared``: a lazy final norm of all rows that the last block left ready, usable when every row is wanted in order."""
+    def logits(self, residual, want_rows, prepared=None, wanted_only: bool = False):
+        """``prepared``: a lazy final norm of all rows that the last block left ready, usable when every row is wanted in order.
+        ``wanted_only``: ``residual`` holds the wanted rows and no others."""
         if want_rows is None or want_rows.shape[0] == 0:
             return None
         from .. import ops
@@ -99,8 +108,9 @@ class DecoderModel:
             if prepared.norm is self.final_norm and prepared.finished is not None and want_rows.shape[0] == prepared.shape[0]:
                 return self.head.forward(prepared.finished)
             prepared = None
+        rows = None if wanted_only else want_rows
         if self.final_norm.supports_lazy and want_rows.shape[0] <= ops.fused_rows_limit(self.runtime.dtype, residual.device):
             if prepared is not None and prepared.weight is self.final_norm.weight and prepared.shape[0] == want_rows.shape[0]:
                 return self.head.forward(prepared)
-            return self.head.forward(self.final_norm.forward(residual, None, rows=want_rows, lazy=True))
-        return self.head.forward(self.final_norm.forward(residual, None, rows=want_rows))
+            return self.head.forward(self.final_norm.forward(residual, None, rows=rows, lazy=True))
+        return self.head.forward(self.final_norm.forward(residual, None, rows=rows))

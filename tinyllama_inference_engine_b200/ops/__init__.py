@@ -165,10 +165,11 @@ def activation(kind: str, x, out, constants=(0.0, 0.0)) -> None:
                                    c_float(constants[1]), _stream()), "activation")
 
 
-def add_rmsnorm(residual, delta, weight, eps: float, out, rows=None) -> None:
+def add_rmsnorm(residual, delta, weight, eps: float, out, rows=None, many_rows: bool = False) -> None:
     """Optional ``residual += delta`` in 32-bit, then ``out = rmsnorm(residual) * weight``.
 
     With ``rows`` (int32) only those rows are normalised (and ``delta`` must be None).
+    ``many_rows``: as in a step of many rows, whose kernel adds a row's squares in another order, whatever the number of rows here.
     """
     if residual.dtype != torch.float32 or weight.dtype != torch.float32:
         raise KernelError("the residual stream and norm weights are 32-bit", code="invalid_dtype")
@@ -180,7 +181,7 @@ def add_rmsnorm(residual, delta, weight, eps: float, out, rows=None) -> None:
     if delta is not None and (delta.shape != residual.shape or delta.dtype != out.dtype):
         raise KernelError("add_rmsnorm: delta must match the residual's shape and the output's dtype", code="invalid_shape")
     _check(
-        core().tlie_add_rmsnorm(_code(out), _ptr(residual), _ptr(delta), _i32(rows, "rows"), _ptr(weight), c_float(eps), _ptr(out), c_int(out_rows), c_int(hidden), _stream()),
+        core().tlie_add_rmsnorm(_code(out), _ptr(residual), _ptr(delta), _i32(rows, "rows"), _ptr(weight), c_float(eps), _ptr(out), c_int(out_rows), c_int(hidden), c_int(1 if many_rows else 0), _stream()),
         "add_rmsnorm",
     )
 
@@ -291,6 +292,30 @@ def scale_rows(x, factor: float) -> None:
     if x.dtype != torch.float32:
         raise KernelError("scale_rows takes a 32-bit tensor", code="invalid_dtype")
     _check(core().tlie_scale_rows(_ptr(x), c_float(factor), c_longlong(x.numel()), _stream()), "scale_rows")
+
+
+def wanted_rows_pay(tokens: int, wanted: int, device: torch.device) -> bool:
+    """Whether a step's last layer goes on with the wanted rows alone once its keys and values are stored: where they are at most half of
+    the rows, of a step of more rows than the small-step kernels take (which read the same weights for one row as for sixteen)."""
+    return device.type == "cuda" and 2 * wanted <= tokens and tokens > fast.GEMV_KERNEL_MAX_ROWS
+
+
+def rows_keep_their_bits(tokens: int, weight, gated: bool = False) -> bool:
+    """Whether the product that a step of this many rows runs (``gated``: the gated one, else the one that adds into the residual) can be run for a few of
+    the rows and give them the same bits: in 32-bit, where an output is one thread's sum in order, and where the step's product
+    is this engine's tcgen05 kernel, whose tiles all add along k alike.  The library cuts k by the number of rows."""
+    if weight.dtype == torch.float32:
+        return True
+    if gated:
+        return fast.use_tcgen05 and weight.dtype == torch.bfloat16 and weight.shape[1] % 8 == 0 and fast.gated_takes(tokens, weight.shape[0], weight.shape[1])
+    return fast.can_accumulate(tokens, weight)
+
+
+def gather_rows(x, rows, out) -> None:
+    """out[t, :] = x[rows[t], :]."""
+    if x.dtype != out.dtype or x.dim() != 2 or out.shape != (rows.shape[0], x.shape[1]):
+        raise KernelError("gather_rows: out is [rows, width] of x's dtype", code="invalid_shape")
+    _check(core().tlie_gather_rows(_ptr(x), _i32(rows, "rows"), _ptr(out), c_int(rows.shape[0]), c_int(x.shape[1] * x.element_size()), _stream()), "gather_rows")
 
 
 def gather_gated(z, table, ids, out, offset: int) -> None:
@@ -478,12 +503,16 @@ def can_accumulate(rows: int, weight) -> bool:
     return fast.can_accumulate(rows, weight)
 
 
-def linear_accumulate(x, weight, residual, prepare: "LazyNorm | None" = None) -> None:
+def linear_accumulate(x, weight, residual, prepare: "LazyNorm | None" = None, like_rows: int | None = None) -> None:
     """residual += x . weight^T, the sum in 32-bit, in one kernel (bfloat16 x; up to 16 rows in the register-fed weight-streaming
     kernel, up to 127 in the tensor-core one, for prompt portions in the tensor-core product's epilogue).
 
     ``prepare``: the lazy norm of this residual (all rows) that the next product will consume; the kernel then leaves that
-    norm's input beside the residual (``prepare.prepared``), written by the threads that hold the finished sums."""
+    norm's input beside the residual (``prepare.prepared``), written by the threads that hold the finished sums.
+    ``like_rows``: x holds a few rows of a step of that many, whose kernel they get (see ``rows_keep_their_bits``)."""
+    if like_rows is not None and x.dtype == torch.bfloat16 and fast.can_accumulate(like_rows, weight):
+        fast.gemm_tcgen05_accumulate(x, weight, residual)
+        return
     rows = x.shape[0]
     if isinstance(prepare, FinishedNorm):
         # the next layer's input in full, where one kernel completes the stream; otherwise it stays unfinished and the block norms the stream itself
@@ -522,10 +551,13 @@ def linear_accumulate(x, weight, residual, prepare: "LazyNorm | None" = None) ->
         add_(residual, delta)
 
 
-def linear_gated(x, weight, out, clamp=None, activation: str = "silu") -> None:
+def linear_gated(x, weight, out, clamp=None, activation: str = "silu", like_rows: int | None = None) -> None:
     """out = act(x . gate^T) * (x . up^T) for weight = [gate rows | up rows], in one kernel where one takes the shape (``clamp``: see
     ``norm_linear``; ``activation``: "silu", or "gelu_tanh", which the small-step kernel has in its epilogue and larger steps run
-    as a kernel behind the product)."""
+    as a kernel behind the product; ``like_rows``: see ``linear_accumulate``)."""
+    if like_rows is not None and x.dtype == torch.bfloat16 and clamp is None and activation == "silu" and rows_keep_their_bits(like_rows, weight, gated=True):
+        fast.gemm_tcgen05_gated(x, weight, out)
+        return
     if activation != "silu":
         if activation not in GATE_KINDS or clamp is not None:
             raise KernelError(f"linear_gated: no gate {activation!r} (with a clamp: silu only)", code="invalid_argument")

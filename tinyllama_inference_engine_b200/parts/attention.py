@@ -66,6 +66,14 @@ class Attention(Mixer):
         return ops.can_accumulate(rows, self.w_o)
 
     def forward(self, x, ctx, cache: LayerCache, accumulate_into=None, prepare=None):
+        return self.project(self.mix(x, ctx, cache), accumulate_into, prepare)
+
+    def rows_alone(self, rows: int) -> bool:
+        """Whether ``project`` of a step of this many rows can be run for a few of them with the same result."""
+        return ops.rows_keep_their_bits(rows, self.w_o)
+
+    def mix(self, x, ctx, cache: LayerCache):
+        """The rows' heads side by side, before the output projection; the step's keys and values are in the cache."""
         ws, dtype, tokens = self.runtime.workspace, self.runtime.dtype, x.shape[0]
         qkv = ws.get("qkv", tokens, self.qkv_width, dtype)
         if isinstance(x, ops.LazyNorm):
@@ -82,10 +90,14 @@ class Attention(Mixer):
         ops.attention_step(qkv, ctx.positions, ctx.token_seq, cache.block_table, inv_freq, rotary_dim, cache.pages, mixed,
                            self.q_heads, self.kv_heads, self.head_dim, cache.page_size, self.window, self.scale,
                            write_cache=cache.writes, batch=ctx)
+        return mixed
+
+    def project(self, mixed, accumulate_into=None, prepare=None, like_rows: int | None = None):
+        """``like_rows``: ``mixed`` holds a few rows of a step of that many, and they get the bits they have among all of them."""
         if accumulate_into is not None:
-            ops.linear_accumulate(mixed, self.w_o, accumulate_into, prepare)
+            ops.linear_accumulate(mixed, self.w_o, accumulate_into, prepare, like_rows)
             return None
-        out = ws.get("mixer_out", tokens, self.hidden, dtype)
+        out = self.runtime.workspace.get("mixer_out", mixed.shape[0], self.hidden, self.runtime.dtype)
         ops.linear(mixed, self.w_o, out)
         return out
 

@@ -56,10 +56,16 @@ class GatedMLP(FeedForward):
     def adds_to_residual(self, rows: int) -> bool:
         return ops.can_accumulate(rows, self.w_down)
 
-    def forward(self, x, ctx, accumulate_into=None, prepare=None):
+    def rows_alone(self, rows: int) -> bool:
+        """Whether ``forward`` of a step of this many rows can be run for a few of them (``like_rows``) with the same result."""
+        return self.activation == "silu" and ops.rows_keep_their_bits(rows, self.w_gate_up, gated=True) and ops.rows_keep_their_bits(rows, self.w_down)
+
+    def forward(self, x, ctx, accumulate_into=None, prepare=None, like_rows: int | None = None):
         ws, dtype, tokens = self.runtime.workspace, self.runtime.dtype, x.shape[0]
         act = ws.get("activated", tokens, self.inter, dtype)
-        if self.activation == "clamped_sigmoid" and tokens <= ops.fused_rows_limit(dtype, act.device):
+        if like_rows is not None and dtype == torch.bfloat16:
+            ops.linear_gated(x, self.w_gate_up, act, like_rows=like_rows)
+        elif self.activation == "clamped_sigmoid" and tokens <= ops.fused_rows_limit(dtype, act.device):
             # few rows: the clamps, the gate and the shift are applied in the stacked product's epilogue
             clamp = (self.limit, self.alpha, self.shift)
             if isinstance(x, ops.LazyNorm):
@@ -92,7 +98,7 @@ class GatedMLP(FeedForward):
             ops.linear(x, self.w_gate_up, gate_up)
             ops.silu_mul(gate_up, act)
         if accumulate_into is not None:
-            ops.linear_accumulate(act, self.w_down, accumulate_into, prepare)
+            ops.linear_accumulate(act, self.w_down, accumulate_into, prepare, like_rows)
             return None
         out = ws.get("ff_out", tokens, self.hidden, dtype)
         ops.linear(act, self.w_down, out)

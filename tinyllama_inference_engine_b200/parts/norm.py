@@ -36,8 +36,8 @@ class RMSNorm(Norm):
         if offset != 0.0:
             self.weight = (self.weight + offset).contiguous()
 
-    def forward(self, residual, delta=None, rows=None, lazy: bool = False):
-        """``lazy`` (and nothing to add): hand the norm on to the product that consumes it (ops.LazyNorm)."""
+    def forward(self, residual, delta=None, rows=None, lazy: bool = False, many_rows: bool = False):
+        """``lazy`` (and nothing to add): hand the norm on to the product that consumes it (ops.LazyNorm).  ``many_rows``: see ``ops.add_rmsnorm``."""
         if lazy and delta is None:
             handle = ops.LazyNorm(residual, self.weight, self.eps, rows, lambda: self.forward(residual, None, rows))
             if rows is None and self.runtime.dtype == torch.bfloat16:
@@ -48,7 +48,7 @@ class RMSNorm(Norm):
             return handle
         count = residual.shape[0] if rows is None else rows.shape[0]
         out = self.runtime.workspace.get("normed" if rows is None else "normed_rows", count, self.size, self.runtime.dtype)
-        ops.add_rmsnorm(residual, delta, self.weight, self.eps, out, rows)
+        ops.add_rmsnorm(residual, delta, self.weight, self.eps, out, rows, **({"many_rows": True} if many_rows else {}))
         return out
 
 
