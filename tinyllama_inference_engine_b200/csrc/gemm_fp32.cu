@@ -192,10 +192,12 @@ static int launch_stream_stages(const float* x, const float* w, float* out, int 
   return (int)launch_pdl(gemm_stream_f32_kernel<MP, MM, STAGES>, dim3((N + kStreamN - 1) / kStreamN), dim3(128), smem, stream, x, w, out, M, N, K, lda, device_sm_count());
 }
 
-template <int MP, int MM>
+// MM rows per thread where a CTA has an SM (nearly) to itself and a sum's own chain is the time; MANY where there are more tiles than that and shared
+// memory's bandwidth is (4 rows x 11,264 columns, K = 2,048: 27.4 us with one row per thread, 26 with two; x 32,000: 69 and 58; 8 rows x 11,264: 47 with two, 37 with four).
+template <int MP, int MM, int MANY>
 static int launch_stream(const float* x, const float* w, float* out, int M, int N, int K, long long lda, cudaStream_t stream) {
   if ((N + kStreamN - 1) / kStreamN <= 2 * device_sm_count()) return launch_stream_stages<MP, MM, 10>(x, w, out, M, N, K, lda, stream);
-  return launch_stream_stages<MP, MM, 4>(x, w, out, M, N, K, lda, stream);
+  return launch_stream_stages<MP, MANY, 4>(x, w, out, M, N, K, lda, stream);
 }
 
 // --- more rows ---------------------------------------------------------------------------------------
@@ -324,11 +326,11 @@ TLIE_EXPORT int tlie_gemm_nt_f32(const float* x, const float* w, float* out, int
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || lda < K) return (int)cudaErrorInvalidValue;
   if (K % 4 == 0 && lda % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0) {
-    if (M == 1) return launch_stream<1, 1>(x, w, out, M, N, K, lda, stream);
-    if (M == 2) return launch_stream<2, 1>(x, w, out, M, N, K, lda, stream);
-    if (M <= 4) return launch_stream<4, 1>(x, w, out, M, N, K, lda, stream);
-    if (M <= 8) return launch_stream<8, 2>(x, w, out, M, N, K, lda, stream);
-    if (M <= 16) return launch_stream<16, 4>(x, w, out, M, N, K, lda, stream);
+    if (M == 1) return launch_stream<1, 1, 1>(x, w, out, M, N, K, lda, stream);
+    if (M == 2) return launch_stream<2, 1, 1>(x, w, out, M, N, K, lda, stream);
+    if (M <= 4) return launch_stream<4, 1, 2>(x, w, out, M, N, K, lda, stream);
+    if (M <= 8) return launch_stream<8, 2, 4>(x, w, out, M, N, K, lda, stream);
+    if (M <= 16) return launch_stream<16, 4, 4>(x, w, out, M, N, K, lda, stream);
     switch (wide_choice(M, N)) {
       case 0: return launch_wide<8, 8, 2, 1>(x, w, out, M, N, K, lda, stream);    // 64 x 64
       case 1: return launch_wide<4, 8, 2, 2>(x, w, out, M, N, K, lda, stream);    // 32 x 128
