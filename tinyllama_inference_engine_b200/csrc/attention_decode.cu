@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(kWarps * 32) decode_attention_kernel(const Dec
   if (!p.fuse_rope) grid_dependency_wait();
   decode_attn_prologue(p, it, smem_raw);
   if (p.fuse_rope) grid_dependency_wait();
-  if (it.split >= it.parts) return;   // after the wait: this kernel's end says that everything before it has ended too
+  if (it.warps_are_parts && it.split > 0) return;   // after the wait: this kernel's end says that everything before it has ended too
   decode_attn_main(p, it, smem_raw, &last_arrival);
 }
 

@@ -128,8 +128,7 @@ struct DecodeAttnParams {
 struct DecodeAttnItem {
   int seq, kvh, split;
   int pos, n_keys, lo, tile_begin, tile_end, next_load;
-  int parts;   // how many of the launch's `splits` have keys of this request: CTAs past them have nothing to do
-  bool warps_are_parts;
+  bool warps_are_parts;   // see the first step: the launch's other parts of this request have nothing to do
   const int* table;
   bool patch_new;
   // cos (first half) and sin (second half) of this position's rotation angles, in shared memory: worked out in the first
@@ -151,17 +150,15 @@ __device__ __forceinline__ void decode_attn_prologue(const DecodeAttnParams& p, 
   // this CTA's tiles: [it.tile_begin, it.tile_end)
   const int first_tile = it.lo / kTileKeys;
   const int all_tiles = (it.n_keys + kTileKeys - 1) / kTileKeys - first_tile;
-  // What a request's keys are cut into decides the order its sums are taken in: parts of per_split tiles, merged in part order.  Parts of one tile each
-  // that fit the warps of one CTA are its warps (57 to 89 keys: three tiles, where eight CTAs merged through global memory and a ticket, five of them empty);
-  // the merge below adds them as it would have added parts.  Otherwise every part that has a tile is a CTA.
   int per_split = (all_tiles + p.splits - 1) / p.splits;
-  it.parts = (all_tiles + per_split - 1) / per_split;
+  // What a request's keys are cut into decides the order its sums are taken in: parts of per_split tiles, merged in part order.  Parts of one tile each
+  // that fit the warps of one CTA are its warps (57 to 89 keys at 1.1B shapes, three tiles: 8.9 -> 6.6 us, where eight CTAs merged through global
+  // memory and a ticket, five of them empty); merge_warps_as_parts adds them as the parts would have been added.
   it.warps_are_parts = p.splits > 1 && per_split == 1 && all_tiles <= kWarps;
   if (it.warps_are_parts) {
-    it.parts = 1;
+    if (it.split > 0) return;
     per_split = all_tiles;
   }
-  if (it.split >= it.parts) return;
   it.tile_begin = first_tile + it.split * per_split;
   it.tile_end = min(first_tile + all_tiles, it.tile_begin + per_split);
 
@@ -194,6 +191,32 @@ __device__ __forceinline__ void decode_attn_prologue(const DecodeAttnParams& p, 
     }
     cp_async_commit();
     it.next_load += kWarps;
+  }
+}
+
+// The end of a request whose parts are the warps of this CTA (merge_o, merge_ml: what the first `live` warps brought): a part's maximum, factor and output
+// as the merge of parts below takes them, the sums added as a warp of it adds them (warp_sum).  A function of its own, so that the code of all other
+// requests is what it would be without it.
+__device__ __noinline__ void merge_warps_as_parts(const float* merge_o, const float* merge_ml, int live, int group, __nv_bfloat16* out) {
+  static_assert(kWarps <= 8, "a part per warp");
+  for (int idx = threadIdx.x; idx < group * kD; idx += kWarps * 32) {
+    const int r = idx / kD, d = idx - r * kD;
+    float m = -INFINITY, acc = 0.0f;
+    float sums[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w)
+      if (w < live) m = fmaxf(m, merge_ml[(w * 16 + r) * 2]);
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      if (w >= live) break;
+      const float wm = merge_ml[(w * 16 + r) * 2];
+      const float f = (wm == -INFINITY) ? 0.0f : exp2f(wm - m);
+      acc += f * merge_o[((size_t)w * 16 + r) * kD + d];
+      sums[w] = __fmul_rn(f, merge_ml[(w * 16 + r) * 2 + 1]);
+    }
+    const float sum = __fadd_rn(__fadd_rn(__fadd_rn(sums[0], sums[4]), __fadd_rn(sums[2], sums[6])),
+                                __fadd_rn(__fadd_rn(sums[1], sums[5]), __fadd_rn(sums[3], sums[7])));
+    out[(size_t)r * kD + d] = __float2bfloat16_rn(acc / sum);
   }
 }
 
@@ -419,7 +442,6 @@ __device__ __forceinline__ void decode_attn_main(const DecodeAttnParams& p, Deco
     row_sum[r] += __shfl_xor_sync(0xffffffffu, row_sum[r], 2);
   }
   __syncthreads();  // every warp is done with its stage buffers: reuse them to merge the warps
-  const int live = min(kWarps, it.tile_end - it.tile_begin);   // warps that had a tile
 
   float* merge_o = reinterpret_cast<float*>(smem_raw);                   // [warp][16][kD]
   float* merge_ml = merge_o + kWarps * 16 * kD;                          // [warp][16][2]
@@ -438,42 +460,26 @@ __device__ __forceinline__ void decode_attn_main(const DecodeAttnParams& p, Deco
     merge_ml[(warp * 16 + g + 8) * 2 + 1] = row_sum[1];
   }
   __syncthreads();
+  if (it.warps_are_parts) {
+    merge_warps_as_parts(merge_o, merge_ml, it.tile_end - it.tile_begin, group, p.out + ((size_t)it.seq * p.q_heads + it.kvh * group) * kD);
+    return;
+  }
   for (int idx = threadIdx.x; idx < group * kD; idx += kWarps * 32) {
     const int r = idx / kD;
     const int d = idx - r * kD;
-    float m = -INFINITY, acc = 0.0f, sum = 0.0f;
-    if (live == kWarps && !it.warps_are_parts) {   // every warp, nothing asked per warp: a CTA in the middle of long keys waits for this
+    float m = -INFINITY;
 #pragma unroll
-      for (int w = 0; w < kWarps; ++w) m = fmaxf(m, merge_ml[(w * 16 + r) * 2]);
+    for (int w = 0; w < kWarps; ++w) m = fmaxf(m, merge_ml[(w * 16 + r) * 2]);
+    float acc = 0.0f, sum = 0.0f;
 #pragma unroll
-      for (int w = 0; w < kWarps; ++w) {
-        const float wm = merge_ml[(w * 16 + r) * 2];
-        const float f = (wm == -INFINITY) ? 0.0f : exp2f(wm - m);
-        acc += f * merge_o[((size_t)w * 16 + r) * kD + d];
-        sum += f * merge_ml[(w * 16 + r) * 2 + 1];
-      }
-    } else {
-      float of_part[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-      static_assert(kWarps <= 8, "a part per warp");
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w)
-        if (w < live) m = fmaxf(m, merge_ml[(w * 16 + r) * 2]);
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) {
-        if (w >= live) break;
-        const float wm = merge_ml[(w * 16 + r) * 2];
-        const float f = (wm == -INFINITY) ? 0.0f : exp2f(wm - m);
-        acc += f * merge_o[((size_t)w * 16 + r) * kD + d];
-        if (it.warps_are_parts) of_part[w] = __fmul_rn(f, merge_ml[(w * 16 + r) * 2 + 1]);
-        else sum += f * merge_ml[(w * 16 + r) * 2 + 1];
-      }
-      // as a warp adds the parts' sums, a lane each (warp_sum)
-      if (it.warps_are_parts)
-        sum = __fadd_rn(__fadd_rn(__fadd_rn(of_part[0], of_part[4]), __fadd_rn(of_part[2], of_part[6])),
-                        __fadd_rn(__fadd_rn(of_part[1], of_part[5]), __fadd_rn(of_part[3], of_part[7])));
+    for (int w = 0; w < kWarps; ++w) {
+      const float wm = merge_ml[(w * 16 + r) * 2];
+      const float f = (wm == -INFINITY) ? 0.0f : exp2f(wm - m);
+      acc += f * merge_o[((size_t)w * 16 + r) * kD + d];
+      sum += f * merge_ml[(w * 16 + r) * 2 + 1];
     }
     const int head = it.kvh * group + r;
-    if (it.parts == 1) {
+    if (p.splits == 1) {
       p.out[((size_t)it.seq * p.q_heads + head) * kD + d] = __float2bfloat16_rn(acc / sum);
     } else {
       const size_t slot = ((size_t)it.seq * p.q_heads + head) * p.splits + it.split;
@@ -484,18 +490,18 @@ __device__ __forceinline__ void decode_attn_main(const DecodeAttnParams& p, Deco
       }
     }
   }
-  if (it.parts == 1) return;
+  if (p.splits == 1) return;
   // The CTA of this (request, kv head) that arrives last merges all parts.  No CTA waits for another.
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
     const int ticket = atomicAdd(&p.tickets[it.seq * p.kv_heads + it.kvh], 1);
-    *last_arrival = (ticket == it.parts - 1);
+    *last_arrival = (ticket == p.splits - 1);
   }
   __syncthreads();
   if (!*last_arrival) return;
   __threadfence();
-  // One warp per query head, lane sp holds part sp's maximum and sum (at most 32 parts).  The parts' outputs do not depend
+  // One warp per query head, lane sp holds part sp's maximum and sum (p.splits <= 32).  The parts' outputs do not depend
   // on those, so their loads go out first, eight parts at a time, and everything is one trip to L2 and back.
   for (int r = warp; r < group; r += kWarps) {
     const size_t pair = (size_t)it.seq * p.q_heads + it.kvh * group + r;
@@ -505,17 +511,17 @@ __device__ __forceinline__ void decode_attn_main(const DecodeAttnParams& p, Deco
 #pragma unroll
     for (int i = 0; i < kPerLane; ++i) acc[i] = 0.0f;
     float part_max = -INFINITY, part_sum = 0.0f, m = 0.0f, f = 0.0f, sum = 0.0f;
-    for (int sp0 = 0; sp0 < it.parts; sp0 += 8) {
+    for (int sp0 = 0; sp0 < p.splits; sp0 += 8) {
       float part[8][kPerLane];
 #pragma unroll
       for (int j = 0; j < 8; ++j)
 #pragma unroll
         for (int i = 0; i < kPerLane; ++i) {
           const int d = lane + 32 * i;
-          part[j][i] = (sp0 + j < it.parts && d < kD) ? __ldcg(p.partial_o + (pair * p.splits + sp0 + j) * kD + d) : 0.0f;
+          part[j][i] = (sp0 + j < p.splits && d < kD) ? __ldcg(p.partial_o + (pair * p.splits + sp0 + j) * kD + d) : 0.0f;
         }
       if (sp0 == 0) {
-        if (lane < it.parts) {
+        if (lane < p.splits) {
           part_max = __ldcg(ml + lane * 2);
           part_sum = __ldcg(ml + lane * 2 + 1);
         }
@@ -527,7 +533,7 @@ __device__ __forceinline__ void decode_attn_main(const DecodeAttnParams& p, Deco
       for (int j = 0; j < 8; ++j) {
         const float fs = __shfl_sync(0xffffffffu, f, (sp0 + j) & 31);
 #pragma unroll
-        for (int i = 0; i < kPerLane; ++i) acc[i] += fs * part[j][i];   // parts past the last were loaded as zeros
+        for (int i = 0; i < kPerLane; ++i) acc[i] += fs * part[j][i];   // parts past p.splits were loaded as zeros
       }
     }
 #pragma unroll
