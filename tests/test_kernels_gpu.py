@@ -279,6 +279,30 @@ def test_sampling_non_finite_logits_still_gives_a_token_of_the_vocabulary(ops):
     assert all(0 <= t < vocab for t in out.cpu().tolist())
 
 
+@pytest.mark.parametrize("vocab", [131, 4, 32000, 32772, 50304, 128256, 131076])
+def test_greedy_rows_with_little_to_compare(ops, vocab):
+    """Rows of NaN (token 0) and rows with one comparable value among NaN, read whole and in slices whose last loads are not full; both greedy kernels."""
+    places = sorted({0, vocab // 4, vocab // 2 + 1, vocab - 1})
+    logits = torch.full((1 + 2 * len(places) + 1, vocab), float("nan"))
+    want = [0]
+    for place in places:
+        for value in (float("-inf"), -3.0):
+            logits[len(want), place] = value
+            want.append(place)
+    logits[-1] = float("-inf")   # every token as likely as every other: the first
+    want.append(0)
+    rows, logits = len(want), logits.cuda()
+    got = torch.full((rows,), -7, dtype=torch.int32, device="cuda")
+    ops.argmax(logits, got)
+    assert got.tolist() == want
+    got.fill_(-7)
+    zeros = torch.zeros(rows, dtype=torch.int64, device="cuda")
+    ops.sample(logits, torch.zeros(rows, device="cuda"), torch.ones(rows, device="cuda"), zeros, zeros, got)
+    assert got.tolist() == want
+    ops.sample(logits, torch.ones(rows, device="cuda"), torch.full((rows,), 0.9, device="cuda"), zeros, zeros, got)
+    assert all(0 <= token < vocab for token in got.tolist()) and got[0].item() == 0
+
+
 @pytest.mark.parametrize("vocab", [1, 3, 32000, 32767, 32768, 32769, 65537, 128256, 131073, 262145])
 def test_sampling_over_blocks_keeps_the_set_and_the_order_of_tokens(ops, vocab):
     """Rows of one block, of clusters of 2 and 4 and of the long kernel, vocabularies at their edges; against sums in 64 bits."""

@@ -18,7 +18,7 @@ namespace tlie {
 
 constexpr int kSampleThreads = 1024;
 
-// A thread's share of a row's maximum and the lowest index that holds it.  Rows that allow it are read 16 bytes at a
+// A thread's share of a row's maximum and the lowest index that holds it (0x7fffffff: no value in its share can be compared).  Rows that allow it are read 16 bytes at a
 // time, four loads in flight per thread: one block reads a whole row, so its time is the latency of its loads in turn.
 __device__ __forceinline__ void row_max_and_arg(const float* __restrict__ row, int vocab, float& best, int& arg) {
   auto take = [&](float v, int i) {
@@ -31,12 +31,15 @@ __device__ __forceinline__ void row_max_and_arg(const float* __restrict__ row, i
     const float4* row4 = reinterpret_cast<const float4*>(row);
     const int quads = vocab >> 2;
     constexpr int kInFlight = 4;
+    // what fills up the last loads: no value is taken from it, while -INFINITY would be the maximum of a row without any comparable value, at an index past the row
+    const float nan = __int_as_float(0x7fffffff);
+    const float4 nothing = make_float4(nan, nan, nan, nan);
     for (int q0 = threadIdx.x; q0 < quads; q0 += kInFlight * blockDim.x) {
       float4 v[kInFlight];
 #pragma unroll
       for (int u = 0; u < kInFlight; ++u) {
         const int q = q0 + u * blockDim.x;
-        v[u] = q < quads ? row4[q] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        v[u] = q < quads ? row4[q] : nothing;
       }
 #pragma unroll
       for (int u = 0; u < kInFlight; ++u) {
