@@ -55,6 +55,70 @@ def test_every_cut_gives_the_plain_logits(model_folders, monkeypatch, key):
     assert stats["reuses"] > 0 and stats["free"] == stats["pages"]
 
 
+@pytest.mark.parametrize("changed", [None, "mixer", "feed_forward", "feed_forward_norm", "block", "a method of one object", "adds_to_residual"])
+def test_last_layer_of_wanted_rows_leaves_other_forwards_alone(tmp_path, monkeypatch, changed):
+    """The last layer of a step goes on with the wanted rows alone only where block, parts and norm run the methods that this takes apart: a subclass's own
+    ``forward`` (twice its parent's here, without the parent's newer arguments) is called for all rows, as in every other layer."""
+    import tiny_configs
+    from tinyllama_inference_engine_b200 import ops
+    from tinyllama_inference_engine_b200.engine.batch import StepEntry
+    from tinyllama_inference_engine_b200.parts.attention import Attention
+    from tinyllama_inference_engine_b200.parts.block import PreNormResidualBlock
+    from tinyllama_inference_engine_b200.parts.mlp import GatedMLP
+    from tinyllama_inference_engine_b200.parts.norm import RMSNorm
+    from tinyllama_inference_engine_b200.weights import write_random_model
+
+    class Mixer(Attention):
+        def forward(self, x, ctx, cache):
+            return 2 * super().forward(x, ctx, cache)
+
+    class FeedForward(GatedMLP):
+        def forward(self, x, ctx):
+            return 2 * super().forward(x, ctx)
+
+    class Norm(RMSNorm):
+        def forward(self, residual, delta=None, rows=None):
+            return 2 * super().forward(residual, delta, rows)
+
+    class OtherBlock(PreNormResidualBlock):
+        def forward(self, residual, pending, ctx, cache, next_norm=None):
+            residual, pending = super().forward(residual, pending, ctx, cache)
+            return residual, 2 * pending
+
+    class Adding(GatedMLP):
+        def adds_to_residual(self, rows):
+            return True
+
+        def forward(self, x, ctx, accumulate_into=None):
+            accumulate_into += 3 * super().forward(x, ctx)
+
+        def rows_alone(self, rows):
+            return True   # it may say so, but it adds where the 32-bit path's wanted rows expect an output
+
+    plain_ops.install(monkeypatch)
+    monkeypatch.setattr(ops, "gather_rows", lambda x, rows, out: out.copy_(x[rows.long()]))
+    folder = write_random_model(tmp_path / "m", tiny_configs.TINY_B, seed=4)
+    tokens = trace_tools.make_requests(tiny_configs.TINY_B["vocab_size"], [40], seed=6)
+    (_, tokens), = tokens.items()
+
+    def logits(pays):
+        monkeypatch.setattr(ops, "wanted_rows_pay", lambda *_: pays)
+        runner = _runner(folder)
+        block = runner.model.blocks[-1]
+        objects = {"mixer": (block.mixer, Mixer), "feed_forward": (block.feed_forward, FeedForward), "feed_forward_norm": (block.feed_forward_norm, Norm),
+                   "block": (block, OtherBlock), "adds_to_residual": (block.feed_forward, Adding)}
+        if changed in objects:
+            objects[changed][0].__class__ = objects[changed][1]
+        elif changed is not None:
+            own = block.mixer.forward
+            block.mixer.forward = lambda *args, **kwargs: 2 * own(*args, **kwargs)
+        assert block.keeps_wanted_rows(40) == (changed is None)
+        return runner.step([StepEntry("r", tokens, [39, 7])])
+
+    want = logits(pays=False)
+    assert torch.allclose(logits(pays=True), want, atol=1e-6)
+
+
 def test_step_refuses_bad_batches(model_folders, monkeypatch):
     plain_ops.install(monkeypatch)
     from tinyllama_inference_engine_b200.engine.batch import StepEntry

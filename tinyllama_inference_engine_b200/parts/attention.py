@@ -8,7 +8,7 @@ import torch
 
 from .. import ops
 from ..errors import ConfigError
-from .base import CacheNeed, LayerCache, Mixer, build_part, register_part
+from .base import CacheNeed, LayerCache, Mixer, build_part, register_part, runs_forward_of
 from .position import rotation_frequencies
 from .spec import PartSpec, TensorSpec
 
@@ -69,8 +69,8 @@ class Attention(Mixer):
         return self.project(self.mix(x, ctx, cache), accumulate_into, prepare)
 
     def rows_alone(self, rows: int) -> bool:
-        """Whether ``project`` of a step of this many rows can be run for a few of them with the same result."""
-        return ops.rows_keep_their_bits(rows, self.w_o)
+        """Whether ``mix``, then ``project`` of a few rows of a step of this many, gives those rows what ``forward`` of the step gives them."""
+        return runs_forward_of(self, Attention) and ops.rows_keep_their_bits(rows, self.w_o)
 
     def mix(self, x, ctx, cache: LayerCache):
         """The rows' heads side by side, before the output projection; the step's keys and values are in the cache."""

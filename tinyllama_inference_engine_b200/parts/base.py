@@ -299,6 +299,12 @@ def norm_then_part(norm, part, residual, pending, fused: bool, next_norm, *args)
     return part.forward(x, *args)
 
 
+def runs_forward_of(part, cls: type) -> bool:
+    """Whether ``part.forward`` is ``cls.forward``: not where a subclass, or somebody who wrapped this object's method, put another in its place.
+    Code that calls the pieces which ``cls.forward`` is made of, in its stead, asks this first."""
+    return getattr(part.forward, "__func__", None) is cls.forward
+
+
 # --- registry of part classes -------------------------------------------------------------
 _PARTS: dict[tuple[str, str], type] = {}
 CATEGORIES = ("mixer", "feed_forward", "norm", "position", "block", "embedding", "head", "token_input", "input_filter")

@@ -3,7 +3,7 @@ from __future__ import annotations
 
 import torch
 
-from .base import Block, CacheNeed, LayerCache, build_part, norm_then_part, part_class, register_part
+from .base import Block, CacheNeed, LayerCache, build_part, norm_then_part, part_class, register_part, runs_forward_of
 from .norm import RMSNorm
 from .spec import PartSpec, TensorSpec
 
@@ -74,10 +74,13 @@ class PreNormResidualBlock(Block):
 
     def keeps_wanted_rows(self, rows: int) -> bool:
         """Whether ``forward_wanted`` can stand in for ``forward`` of a step of this many rows: the parts say where its rows stop depending on one another
-        and that a few of them get the bits that they have among all of them."""
-        parts = (self.mixer, self.feed_forward)
-        return (self.token_input is None and all(hasattr(part, "rows_alone") and part.rows_alone(rows) for part in parts)
-                and isinstance(self.feed_forward_norm, RMSNorm))
+        and that a few of them get the bits that they have among all of them; block, parts and norm run the methods that ``forward_wanted`` takes apart, and
+        the parts add into the stream exactly where it lets them."""
+        adding = self.runtime.dtype == torch.bfloat16
+        return (runs_forward_of(self, PreNormResidualBlock) and self.token_input is None and self.feed_forward is not None
+                and runs_forward_of(self.feed_forward_norm, RMSNorm)
+                and all(hasattr(part, "rows_alone") and part.rows_alone(rows) and (part.fuses_residual_add and part.adds_to_residual(rows)) == adding
+                        for part in (self.mixer, self.feed_forward)))
 
     def forward_wanted(self, residual, pending, ctx, cache: LayerCache, wanted):
         """``forward`` of a step's last layer, of which only the rows ``wanted`` are read on: every row is mixed (its keys and values belong to the

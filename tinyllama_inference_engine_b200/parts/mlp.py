@@ -5,7 +5,7 @@ import torch
 
 from .. import ops
 from ..errors import ConfigError
-from .base import FeedForward, build_part, part_class, register_part
+from .base import FeedForward, build_part, part_class, register_part, runs_forward_of
 from .spec import PartSpec, TensorSpec
 
 
@@ -58,7 +58,7 @@ class GatedMLP(FeedForward):
 
     def rows_alone(self, rows: int) -> bool:
         """Whether ``forward`` of a step of this many rows can be run for a few of them (``like_rows``) with the same result."""
-        return self.activation == "silu" and ops.rows_keep_their_bits(rows, self.w_gate_up, gated=True) and ops.rows_keep_their_bits(rows, self.w_down)
+        return runs_forward_of(self, GatedMLP) and self.activation == "silu" and ops.rows_keep_their_bits(rows, self.w_gate_up, gated=True) and ops.rows_keep_their_bits(rows, self.w_down)
 
     def forward(self, x, ctx, accumulate_into=None, prepare=None, like_rows: int | None = None):
         ws, dtype, tokens = self.runtime.workspace, self.runtime.dtype, x.shape[0]
