@@ -148,6 +148,26 @@ def test_gemm_fp32_gives_a_row_the_same_bits_in_every_kernel(ops, N, K):
     assert torch.equal(got, full[:40])
 
 
+@pytest.mark.parametrize("M", [1, 2, 4, 8, 16, 40])
+def test_gemm_fp32_takes_a_weight_that_the_kernel_before_it_writes(ops, M):
+    """A product whose weight is the result of the product before it (which lets its successor start early), over and over on the same buffer."""
+    torch.manual_seed(38)
+    N, K = 1000, 2048
+    a, b, x = torch.randn(3, N, 256).cuda(), torch.randn(K, 256).cuda(), torch.randn(M, K).cuda()
+    weight, out = torch.zeros(N, K, device="cuda"), torch.zeros(3, M, N, device="cuda")
+    want = torch.zeros_like(out)
+    for i in range(3):
+        ops.linear(a[i], b, weight)
+        torch.cuda.synchronize()
+        ops.linear(x, weight, want[i])
+        torch.cuda.synchronize()
+    for _ in range(5):
+        for i in range(3):
+            ops.linear(a[i], b, weight)
+            ops.linear(x, weight, out[i])
+        assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 256, 64), (37, 136, 80), (130, 72, 520), (64, 2048, 2048)])
 def test_linear_bf16(ops, M, N, K):
     torch.manual_seed(4)

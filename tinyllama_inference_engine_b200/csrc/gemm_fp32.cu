@@ -115,12 +115,21 @@ __global__ void __launch_bounds__(128) gemm_stream_f32_kernel(const float* __res
     const bool inside = k < K;
     for (int r = warp; r < MP; r += 4) cp_async_16(stage + r * kStreamStride, x + (long long)min(r, M - 1) * lda + (inside ? k : 0), inside);
   };
-  // the weights do not depend on the kernel before this one: its last part hides their first loads
-  for (int c = 0; c < STAGES - 1 && c < chunks; ++c) copy_w(c);
+  // While the kernel before this one runs, L2 fetches the first stages' weights.  Nothing is read: w may be what that kernel (or the one before it) writes.
+  auto ask_for_w = [&](int chunk) {
+    const int k = chunk * kStreamK + lane * 4;
+#pragma unroll
+    for (int r = 0; r < kStreamN / 4; ++r)
+      if (k < K) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(w + (long long)min(n0 + warp + 4 * r, N - 1) * K + k));
+  };
+  for (int c = 0; c < STAGES - 1 && c < chunks; ++c) ask_for_w(c);
   grid_launch_dependents();
   grid_dependency_wait();
-  for (int c = 0; c < STAGES - 1; ++c) {   // the first group also holds the weights above; empty groups keep the count
-    if (c < chunks) copy_x(c);
+  for (int c = 0; c < STAGES - 1; ++c) {   // (empty groups keep the count)
+    if (c < chunks) {
+      copy_w(c);
+      copy_x(c);
+    }
     cp_async_commit();
   }
   // a warp is 8 outputs x 4 rows (16 x 1, 16 x 2); CTAs that share an SM compute in different warps, so on different schedulers

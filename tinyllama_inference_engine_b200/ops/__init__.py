@@ -375,7 +375,10 @@ def sigmoid_gate(x, gate) -> None:
 
 
 def linear(x, weight, out) -> None:
-    """out[M, N] = x[M, K] . weight[N, K]^T in the tensors' dtype (32-bit accumulation); ``x`` may be a run of columns of wider rows."""
+    """out[M, N] = x[M, K] . weight[N, K]^T in the tensors' dtype (32-bit accumulation); ``x`` may be a run of columns of wider rows.
+
+    Up to 16 bfloat16 rows: the kernel reads ``weight`` while the kernel launched before it may still run, so ``weight`` must not be what that
+    kernel writes.  ``x`` may be, and in the 32-bit path ``weight`` too."""
     M, K = x.shape
     N = weight.shape[0]
     if weight.shape[1] != K or out.shape != (M, N):
