@@ -269,6 +269,32 @@ def test_rows_of_eight_at_a_time(ops, rows):
     assert torch.allclose(pages_gpu.cpu().float(), pages_plain.float(), atol=_tol(torch.bfloat16, 4) + 2e-4)
 
 
+@pytest.mark.parametrize("tokens", [3, 500, 1500])
+def test_rope_store_takes_positions_that_the_kernel_before_it_writes(ops, tokens):
+    """Positions, rows' requests and block table gathered by a kernel that lets its successor start early, another choice of them each time."""
+    torch.manual_seed(39)
+    held = -(-tokens // 64)
+    qkv, pages = torch.randn(tokens, 10 * 64).bfloat16(), torch.zeros(2 * held, 2, 2, 64, 64, dtype=torch.bfloat16)
+    inv_freq = torch.from_numpy(np.power(np.float32(1e4), np.float32(-2.0) * np.arange(32, dtype=np.float32) / np.float32(64)))
+    table = torch.randperm(2 * held)
+    choices = torch.stack([torch.cat([torch.arange(tokens).roll(shift), torch.full((tokens,), shift % 2), table.roll(shift)]) for shift in range(4)]).int()
+    described = torch.zeros(1, choices.shape[1], dtype=torch.int32, device="cuda")
+    cut = lambda row: (row[:tokens], row[tokens : 2 * tokens], row[2 * tokens :].view(2, held))  # noqa: E731
+    choices_gpu, freq = choices.cuda(), inv_freq.cuda()
+    index = [torch.tensor([i], dtype=torch.int32, device="cuda") for i in range(4)]
+    for i in (1, 3, 0, 2):
+        want_qkv, want_pages = qkv.clone(), pages.clone()
+        plain_ops.rope_store(want_qkv, *cut(choices[i]), inv_freq, 64, want_pages, 6, 2, 64, 64, True)
+        for _ in range(3):
+            got_qkv, got_pages = qkv.cuda(), pages.cuda()
+            torch.cuda.synchronize()
+            ops.gather_rows(choices_gpu, index[(i + 1) % 4], described)
+            ops.gather_rows(choices_gpu, index[i], described)
+            ops.rope_store(got_qkv, *cut(described[0]), freq, 64, got_pages, 6, 2, 64, 64, True)
+            assert torch.allclose(got_qkv.cpu().float(), want_qkv.float(), atol=_tol(torch.bfloat16, 4) + 2e-4)
+            assert torch.allclose(got_pages.cpu().float(), want_pages.float(), atol=_tol(torch.bfloat16, 4) + 2e-4)
+
+
 @pytest.mark.parametrize("dtype,width", [(torch.float32, 2048), (torch.bfloat16, 4096), (torch.bfloat16, 131), (torch.float32, 3)])
 def test_gather_rows(ops, dtype, width):
     x = torch.randn(40, width).to(dtype).cuda()

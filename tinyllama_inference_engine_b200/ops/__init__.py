@@ -646,7 +646,10 @@ def paged_attention(qkv, pages, positions, token_seq, block_table, out, q_heads:
 
 def attention_step(qkv, positions, token_seq, block_table, inv_freq, rotary_dim: int, pages, out, q_heads: int, kv_heads: int,
                    head_dim: int, page_size: int, window: int = 0, scale: float | None = None, write_cache: bool = True, batch=None) -> None:
-    """Rotate q and k, store k and v in the pages, and attend: ``rope_store`` then ``paged_attention``, in one kernel where one exists."""
+    """Rotate q and k, store k and v in the pages, and attend: ``rope_store`` then ``paged_attention``, in one kernel where one exists.
+
+    That one kernel (a step of one bfloat16 token per request) reads positions, block table, frequencies and every cached key but the new one while the kernel
+    launched before it may still run: of these that kernel must write none.  ``rope_store`` and ``paged_attention`` have no such condition."""
     if qkv.dtype == torch.bfloat16:
         if fast.can_fuse_rope_into_decode(batch, qkv, head_dim, q_heads, kv_heads, inv_freq, rotary_dim):
             splits = fast.decode_splits(batch.num_seqs, kv_heads, batch.max_seq_len)
