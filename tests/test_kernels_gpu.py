@@ -269,6 +269,22 @@ def test_rows_of_eight_at_a_time(ops, rows):
     assert torch.allclose(pages_gpu.cpu().float(), pages_plain.float(), atol=_tol(torch.bfloat16, 4) + 2e-4)
 
 
+@pytest.mark.parametrize("q_heads,kv_heads,head_dim,rotary_dim", [(6, 2, 64, 32), (1, 1, 16, 16), (4, 4, 64, 64), (5, 1, 64, 64), (32, 32, 128, 128), (3, 2, 48, 0), (2, 2, 128, 80)])
+@pytest.mark.parametrize("tokens", [2, 1023, 1025])
+def test_rope_store_with_one_token_per_block_and_with_four(ops, q_heads, kv_heads, head_dim, rotary_dim, tokens):
+    """Shapes on both sides of what decides between the two kernels (1,024 tokens; 64 pieces of a token), more pieces than threads, tails past the rotated part, no cache."""
+    torch.manual_seed(40)
+    qkv, pages, positions, token_seq, table = _paged_case(np.random.default_rng(40), torch.bfloat16, [tokens], [tokens], kv_heads, head_dim, 64, q_heads)
+    inv_freq = torch.from_numpy(np.power(np.float32(1e4), np.float32(-2.0) * np.arange(rotary_dim // 2, dtype=np.float32) / np.float32(max(2, rotary_dim)))) if rotary_dim else None
+    for write in (True, False):
+        want_qkv, want_pages = qkv.clone(), pages.clone()
+        plain_ops.rope_store(want_qkv, positions, token_seq, table, inv_freq, rotary_dim, want_pages, q_heads, kv_heads, head_dim, 64, write)
+        got_qkv, got_pages = qkv.cuda(), pages.cuda()
+        ops.rope_store(got_qkv, positions.cuda(), token_seq.cuda(), table.cuda(), None if inv_freq is None else inv_freq.cuda(), rotary_dim, got_pages, q_heads, kv_heads, head_dim, 64, write)
+        assert torch.allclose(got_qkv.cpu().float(), want_qkv.float(), atol=_tol(torch.bfloat16, 4) + 2e-4)
+        assert torch.allclose(got_pages.cpu().float(), want_pages.float(), atol=_tol(torch.bfloat16, 4) + 2e-4)
+
+
 @pytest.mark.parametrize("tokens", [3, 500, 1500])
 def test_rope_store_takes_positions_that_the_kernel_before_it_writes(ops, tokens):
     """Positions, rows' requests and block table gathered by a kernel that lets its successor start early, another choice of them each time."""
