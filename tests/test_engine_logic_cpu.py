@@ -191,6 +191,35 @@ def test_gemm_tile_width_prefers_full_waves():
             assert fast.gemm_tile_width(rows, cols) in fast.GEMM_TILE_WIDTHS + fast.GEMM_WIDE_TILES
 
 
+@pytest.mark.parametrize("group", [1, 3, 4, 8, 16, 32])
+def test_shared_attention_runs_cover_a_step_with_few_requests_to_a_tile(group):
+    """Random steps: every row in one tile, tiles within the kernel's 32 pairs, decoding requests alone, no tile with more than three requests, and as tall as that allows."""
+    import random
+
+    from tinyllama_inference_engine_b200.ops.fast import shared_attention_runs
+
+    def most_requests(owners, rows):
+        return max(len(set(owners[i : i + rows])) for i in range(0, len(owners), rows))
+
+    rng = random.Random(5)
+    steps = [[1], [7], [1] * 9, [1, 1, 1, 500], [500, 1], [300, 1, 1, 1, 200], [2] * 16, [5] * 8, [1, 40, 1, 40, 1]]
+    steps += [[rng.choice([1, 1, 2, 5, 31, 32, 33, 100]) for _ in range(rng.randint(1, 40))] for _ in range(200)]
+    for q_lens in steps:
+        tokens = sum(q_lens)
+        owners = [i for i, q in enumerate(q_lens) for _ in range(q)]
+        runs = shared_attention_runs(tokens, q_lens, group)
+        assert [r[0] for r in runs] == [0] + [r[1] for r in runs[:-1]] and runs[-1][1] == tokens
+        if max(q_lens) == 1:
+            assert runs == [(0, tokens, 1)]
+            continue
+        first, end, rows = runs[-1]
+        assert all(r[2] == 1 for r in runs[:-1]) and first == next(i for i, q in enumerate(q_lens) if q > 1)
+        tallest = max(1, 32 // group)
+        assert 1 <= rows <= tallest and (rows == 1 or most_requests(owners[first:], rows) <= 3)
+        assert rows == tallest or most_requests(owners[first:], next(h for h in (tallest, tallest // 2, tallest // 4, tallest // 8, tallest // 16) if h // 2 == rows)) > 3
+    assert shared_attention_runs(50, None, group) == shared_attention_runs(50, [20, 20], group) == [(0, 50, 1)]   # nobody describes the step, or not this one
+
+
 def test_decode_attention_parts_fit_one_wave():
     """requests x kv heads x parts never exceeds the SMs while a (request, kv head) has a CTA to itself: no second wave."""
     from tinyllama_inference_engine_b200.ops import fast

@@ -476,6 +476,29 @@ def test_paged_attention_f32_over_shared_keys(ops, q_heads, kv_heads, head_dim, 
     assert torch.equal(alone, got[lasts.cuda()])
 
 
+@pytest.mark.parametrize("q_heads,kv_heads,head_dim,page_size", [(8, 1, 64, 64), (4, 4, 64, 16), (6, 2, 128, 32), (24, 2, 64, 16), (32, 1, 128, 16), (9, 9, 128, 64)])
+@pytest.mark.parametrize("q_lens", [[1, 1, 1, 1, 40, 3], [2] * 9, [33, 1, 1, 1, 1, 32], [5, 5, 5, 70], [1] * 7, [64], None])
+def test_paged_attention_f32_over_shared_keys_has_the_bits_of_the_general_kernel(ops, q_heads, kv_heads, head_dim, page_size, q_lens):
+    """Described steps, whose tiles are as tall as their requests allow, and one that nobody describes."""
+    torch.manual_seed(41)
+
+    class Batch:
+        host_q_lens = q_lens
+
+    lens = q_lens or [3, 30, 1]
+    held = [q + (i * 37) % 90 for i, q in enumerate(lens)]
+    qkv, pages, positions, token_seq, table = _paged_case(np.random.default_rng(41), torch.float32, held, lens, kv_heads, head_dim, page_size, q_heads)
+    qkv, pages, positions, token_seq, table = (t.cuda() for t in (qkv, pages, positions, token_seq, table))
+    got, want = (torch.full((len(positions), q_heads * head_dim), float("nan"), device="cuda") for _ in range(2))
+    ops.paged_attention(qkv, pages, positions, token_seq, table, got, q_heads, kv_heads, head_dim, page_size, batch=Batch())
+    c_int, pointer = ops.c_int, lambda t: ops.c_void_p(t.data_ptr())  # noqa: E731
+    status = ops.core().tlie_paged_attention_generic(
+        c_int(0), pointer(qkv), c_int(qkv.shape[1]), pointer(pages), pointer(positions), pointer(token_seq), pointer(table), c_int(table.shape[1]), pointer(want),
+        c_int(len(positions)), c_int(q_heads), c_int(kv_heads), c_int(head_dim), c_int(page_size), c_int(0), ops.c_float(head_dim ** -0.5), ops._stream())
+    assert status == 0
+    assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("q_heads,kv_heads,head_dim,page_size,window", [
     (32, 4, 64, 64, 0), (8, 8, 128, 64, 0), (32, 8, 128, 16, 0), (4, 2, 16, 16, 0), (6, 2, 32, 32, 0), (3, 3, 48, 16, 0),
     (16, 1, 64, 64, 0), (8, 2, 64, 32, 100), (10, 2, 80, 16, 33),

@@ -285,20 +285,18 @@ TLIE_EXPORT int tlie_paged_attention_generic(int dtype, const void* q, int q_row
   return (int)cudaGetLastError();
 }
 
-// The same for 32-bit rows of head size 64 or 128 without a window, 16-byte aligned rows and pages, at most 32 query heads per kv head.  single_rows: every
-// row is of another request (a decode step), so a CTA takes one row.
+// The same for 32-bit rows of head size 64 or 128 without a window, 16-byte aligned pages, at most 32 query heads per kv head.  rows_per_tile: rows of a CTA
+// (times the group at most 32).  A CTA works on the requests of its rows one after the other: who calls keeps a tile to few of them.
 TLIE_EXPORT int tlie_paged_attention_shared_f32(const float* q, int q_row_stride, const float* pages, const int* positions, const int* token_seq,
                                                 const int* block_table, int table_stride, float* out, int tokens, int q_heads, int kv_heads, int head_dim,
-                                                int page_size, float scale, int single_rows, cudaStream_t stream) {
+                                                int page_size, float scale, int rows_per_tile, cudaStream_t stream) {
   if (tokens <= 0) return 0;
-  if ((head_dim != 64 && head_dim != 128) || kv_heads <= 0 || kv_heads > 65535 || q_heads % kv_heads != 0 || q_heads / kv_heads > 4 * kSharedWarps ||
-      (reinterpret_cast<uintptr_t>(pages) & 15) != 0)
+  if ((head_dim != 64 && head_dim != 128) || kv_heads <= 0 || kv_heads > 65535 || q_heads % kv_heads != 0 || rows_per_tile < 1 ||
+      (long long)rows_per_tile * (q_heads / kv_heads) > 4 * kSharedWarps || (reinterpret_cast<uintptr_t>(pages) & 15) != 0)
     return (int)cudaErrorInvalidValue;
-  const int group = q_heads / kv_heads;
-  if (single_rows && group <= kSharedWarps)
-    return head_dim == 64 ? launch_shared<64, 1>(q, q_row_stride, pages, positions, token_seq, block_table, table_stride, out, tokens, q_heads, kv_heads, page_size, scale, 1, stream)
-                          : launch_shared<128, 1>(q, q_row_stride, pages, positions, token_seq, block_table, table_stride, out, tokens, q_heads, kv_heads, page_size, scale, 1, stream);
-  const int rows = single_rows ? 1 : 4 * kSharedWarps / group;
-  return head_dim == 64 ? launch_shared<64, 4>(q, q_row_stride, pages, positions, token_seq, block_table, table_stride, out, tokens, q_heads, kv_heads, page_size, scale, rows, stream)
-                        : launch_shared<128, 4>(q, q_row_stride, pages, positions, token_seq, block_table, table_stride, out, tokens, q_heads, kv_heads, page_size, scale, rows, stream);
+  if (rows_per_tile * (q_heads / kv_heads) <= kSharedWarps)   // a pair per warp
+    return head_dim == 64 ? launch_shared<64, 1>(q, q_row_stride, pages, positions, token_seq, block_table, table_stride, out, tokens, q_heads, kv_heads, page_size, scale, rows_per_tile, stream)
+                          : launch_shared<128, 1>(q, q_row_stride, pages, positions, token_seq, block_table, table_stride, out, tokens, q_heads, kv_heads, page_size, scale, rows_per_tile, stream);
+  return head_dim == 64 ? launch_shared<64, 4>(q, q_row_stride, pages, positions, token_seq, block_table, table_stride, out, tokens, q_heads, kv_heads, page_size, scale, rows_per_tile, stream)
+                        : launch_shared<128, 4>(q, q_row_stride, pages, positions, token_seq, block_table, table_stride, out, tokens, q_heads, kv_heads, page_size, scale, rows_per_tile, stream);
 }

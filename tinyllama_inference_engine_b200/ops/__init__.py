@@ -625,14 +625,15 @@ def paged_attention(qkv, pages, positions, token_seq, block_table, out, q_heads:
         if fast.paged_attention_bf16(qkv, pages, positions, token_seq, block_table, out, q_heads, kv_heads, head_dim, page_size, window, scale, batch):
             return
     elif window <= 0 and head_dim in (64, 128) and q_heads // kv_heads <= 32 and kv_heads <= 65535 and pages.data_ptr() % 16 == 0:
-        _check(
-            core().tlie_paged_attention_shared_f32(
-                _ptr(qkv), c_int(qkv.shape[1]), _ptr(pages), _i32(positions, "positions"), _i32(token_seq, "token_seq"), _i32(block_table, "block_table"),
-                c_int(block_table.shape[1]), _ptr(out), c_int(tokens), c_int(q_heads), c_int(kv_heads), c_int(head_dim), c_int(page_size), c_float(scale),
-                c_int(1 if batch is not None and batch.decode_only else 0), _stream(),
-            ),
-            "paged_attention_shared_f32",
-        )
+        for first, end, rows in fast.shared_attention_runs(tokens, getattr(batch, "host_q_lens", None), q_heads // kv_heads):
+            _check(
+                core().tlie_paged_attention_shared_f32(
+                    _ptr(qkv[first:end]), c_int(qkv.shape[1]), _ptr(pages), _i32(positions[first:end], "positions"), _i32(token_seq[first:end], "token_seq"),
+                    _i32(block_table, "block_table"), c_int(block_table.shape[1]), _ptr(out[first:end]), c_int(end - first), c_int(q_heads), c_int(kv_heads),
+                    c_int(head_dim), c_int(page_size), c_float(scale), c_int(rows), _stream(),
+                ),
+                "paged_attention_shared_f32",
+            )
         return
     _check(
         core().tlie_paged_attention_generic(

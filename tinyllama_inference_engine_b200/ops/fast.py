@@ -9,6 +9,7 @@ import functools
 import os
 import weakref
 from ctypes import c_float, c_int, c_longlong, c_void_p
+from itertools import accumulate
 
 import torch
 
@@ -574,6 +575,29 @@ def leading_single_rows(q_lens: list[int]) -> int:
     while lead < len(q_lens) and q_lens[lead] == 1:
         lead += 1
     return lead if lead < len(q_lens) else 0
+
+
+SHARED_ATTENTION_PAIRS = 32      # (row, head) pairs of a CTA of the 32-bit kernel over shared keys (csrc/attention_generic.cu: 4 * kSharedWarps)
+SHARED_ATTENTION_REQUESTS = 3    # requests whose rows one of its tiles may hold
+
+
+def shared_attention_runs(tokens: int, q_lens: list[int] | None, group: int) -> list[tuple[int, int, int]]:
+    """The launches of the 32-bit attention kernel over shared keys for a step: (first row, end row, rows of a tile).
+
+    A tile shares its requests' keys among its rows, but walks the requests one after the other: 31 decoded tokens of 1,000 keys and a prompt
+    of 100 at 32 heads of 128, each head with keys of its own, took 5,170 us in tiles of 32 rows (the kernel with a warp per row and head: 1,266).  So the decoding
+    requests at the head of a step, and every row of a step that nobody describes (``q_lens`` None), are tiles of their own, and the other
+    tiles are only as tall as leaves each with SHARED_ATTENTION_REQUESTS requests at most (a request of 1,000 keys costs a tile 148 us at head size 128 and 91 at
+    64, the other kernel 390 us and more whatever the number)."""
+    if q_lens is None or max(q_lens) == 1 or sum(q_lens) != tokens:
+        return [(0, tokens, 1)]
+    lead = leading_single_rows(q_lens)
+    edges = list(accumulate(q_lens[lead:]))[:-1]   # first rows of the requests behind the first one
+    rows = max(1, SHARED_ATTENTION_PAIRS // group)
+    inner = SHARED_ATTENTION_REQUESTS   # this many edges inside one tile are one request too many
+    while rows > 1 and any(first % rows and first // rows == last // rows for first, last in zip(edges, edges[inner - 1 :])):
+        rows //= 2
+    return ([(0, lead, 1)] if lead else []) + [(lead, tokens, rows)]
 
 
 def attention_tiles(q_lens: list[int], first_positions: list[int], seq_starts: list[int], first_entry: int = 0, end_entry: int | None = None) -> list[int]:
