@@ -269,6 +269,20 @@ def test_rows_of_eight_at_a_time(ops, rows):
     assert torch.allclose(pages_gpu.cpu().float(), pages_plain.float(), atol=_tol(torch.bfloat16, 4) + 2e-4)
 
 
+@pytest.mark.parametrize("inter", [8, 24, 120, 128, 136, 1016, 1032, 2048, 2056])
+def test_gate_of_narrow_rows(ops, inter):
+    """Rows that share a block (two to 256 of them) and rows that a block or two take, numbers of rows that do not fill the last block, both gates."""
+    torch.manual_seed(42)
+    for rows in (1, 3, 255, 257):
+        gate_up = torch.randn(rows + 1, 2 * inter).bfloat16().cuda()
+        g, u = gate_up[:rows, :inter].double(), gate_up[:rows, inter:].double()
+        for kind, want in (("silu", g / (1 + torch.exp(-g)) * u), ("gelu_tanh", torch.nn.functional.gelu(g, approximate="tanh") * u)):
+            got = torch.full((rows + 1, inter), 7.0, dtype=torch.bfloat16, device="cuda")
+            ops.gate_mul(gate_up[:rows], got[:rows], kind)
+            # one rounding to bfloat16 (2^-9 of the value) over 32-bit arithmetic
+            assert bool(((got[:rows].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()) and bool((got[rows:] == 7.0).all())
+
+
 @pytest.mark.parametrize("q_heads,kv_heads,head_dim,rotary_dim", [(6, 2, 64, 32), (1, 1, 16, 16), (4, 4, 64, 64), (5, 1, 64, 64), (32, 32, 128, 128), (3, 2, 48, 0), (2, 2, 128, 80)])
 @pytest.mark.parametrize("tokens", [2, 1023, 1025])
 def test_rope_store_with_one_token_per_block_and_with_four(ops, q_heads, kv_heads, head_dim, rotary_dim, tokens):
