@@ -269,6 +269,24 @@ def test_rows_of_eight_at_a_time(ops, rows):
     assert torch.allclose(pages_gpu.cpu().float(), pages_plain.float(), atol=_tol(torch.bfloat16, 4) + 2e-4)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("hidden", [4, 40, 512, 516, 1024, 1028, 2048, 2050])
+def test_embedding_of_narrow_and_wide_rows(ops, dtype, hidden):
+    """Rows that share a block and rows that a block walks, numbers of rows that do not fill the last block, ids outside the table among them."""
+    torch.manual_seed(43)
+    table = torch.randn(50, hidden).to(dtype).cuda()
+    for rows in (1, 3, 255, 257):
+        ids = torch.randint(0, 50, (rows,), dtype=torch.int32)
+        got = torch.full((rows + 1, hidden), 7.0, device="cuda")
+        ops.embedding(table, ids.cuda(), got[:rows])
+        assert torch.equal(got[:rows], table[ids.cuda().long()].float()) and bool((got[rows:] == 7.0).all())
+    ids[5], ids[256] = -1, 50
+    ops.embedding(table, ids.cuda(), got[:rows])
+    with pytest.raises(Exception, match="outside the vocabulary"):
+        ops.check_device_errors(got.device)
+    assert torch.equal(got[5], table[0].float()) and torch.equal(got[256], table[0].float())
+
+
 @pytest.mark.parametrize("inter", [8, 24, 120, 128, 136, 1016, 1032, 2048, 2056])
 def test_gate_of_narrow_rows(ops, inter):
     """Rows that share a block (two to 256 of them) and rows that a block or two take, numbers of rows that do not fill the last block, both gates."""

@@ -24,37 +24,6 @@ __global__ void embedding_kernel(const T* __restrict__ table, const int* __restr
   for (int i = threadIdx.x; i < hidden; i += blockDim.x) dst[i] = to_float(src[i]);
 }
 
-// The same eight elements at a time (hidden % 8 == 0, 16-byte aligned): 8,192 rows of 4,096 took 68 us element by element, 38 so, ncu; a step of one
-// row 6.6 us and 3.1.
-__device__ __forceinline__ void load8(const float* p, float4& a, float4& b) {
-  a = reinterpret_cast<const float4*>(p)[0];
-  b = reinterpret_cast<const float4*>(p)[1];
-}
-__device__ __forceinline__ void load8(const __nv_bfloat16* p, float4& a, float4& b) {
-  const uint4 raw = *reinterpret_cast<const uint4*>(p);
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-  a = make_float4(__bfloat162float(h[0].x), __bfloat162float(h[0].y), __bfloat162float(h[1].x), __bfloat162float(h[1].y));
-  b = make_float4(__bfloat162float(h[2].x), __bfloat162float(h[2].y), __bfloat162float(h[3].x), __bfloat162float(h[3].y));
-}
-template <typename T>
-__global__ void __launch_bounds__(256) embedding_vec_kernel(const T* __restrict__ table, const int* __restrict__ ids, float* __restrict__ residual, int hidden,
-                                                            int vocab, int* __restrict__ error_flag) {
-  const int row = blockIdx.x;
-  int id = ids[row];
-  if (id < 0 || id >= vocab) {
-    if (threadIdx.x == 0 && error_flag != nullptr) atomicOr(error_flag, 2);
-    id = 0;
-  }
-  const T* src = table + (size_t)id * hidden;
-  float* dst = residual + (size_t)row * hidden;
-  for (int i = threadIdx.x * 8; i < hidden; i += 256 * 8) {
-    float4 a, b;
-    load8(src + i, a, b);
-    reinterpret_cast<float4*>(dst + i)[0] = a;
-    reinterpret_cast<float4*>(dst + i)[1] = b;
-  }
-}
-
 // Optional add, then RMSNorm.  For output row r the source row is rows ? rows[r] : r.
 //   if delta:  residual[src, :] += float(delta[src, :])        (32-bit sum, stored back)
 //   scale = 1 / sqrt(mean(residual[src]^2) + eps);  out[r, :] = (x * scale) * weight
@@ -110,6 +79,24 @@ struct Vec4<__nv_bfloat16> {
     *reinterpret_cast<uint2*>(p) = raw;
   }
 };
+
+// The embedding, four elements at a time (hidden % 4 == 0, aligned), a block a row or, of narrow rows, blockDim.y of them.  What counts is that neighbouring threads write
+// neighbouring 16 bytes.  Back to back, element by element -> so: 8,192 bfloat16 rows of 4,096 39 -> 25 us (37 with eight elements, so two writes, to a thread), 2,048 of 4,096 9.1 -> 6.8
+// (11.0 with eight), one row of 2,048 2.8 -> 1.9, 8,192 rows of 64 5.8 -> 2.0.
+template <typename T>
+__global__ void __launch_bounds__(256) embedding_vec_kernel(const T* __restrict__ table, const int* __restrict__ ids, float* __restrict__ residual, int rows, int hidden,
+                                                            int vocab, int* __restrict__ error_flag) {
+  const int row = blockIdx.x * blockDim.y + threadIdx.y;
+  if (row >= rows) return;
+  int id = ids[row];
+  if (id < 0 || id >= vocab) {
+    if (threadIdx.x == 0 && error_flag != nullptr) atomicOr(error_flag, 2);
+    id = 0;
+  }
+  const T* src = table + (size_t)id * hidden;
+  float* dst = residual + (size_t)row * hidden;
+  for (int i = threadIdx.x * 4; i < hidden; i += blockDim.x * 4) *reinterpret_cast<float4*>(dst + i) = Vec4<T>::load(src + i);
+}
 
 constexpr int kNormThreads = 256;
 constexpr int kNormChunks = 8;   // float4 chunks per thread: widths up to 256 * 8 * 4 = 8192
@@ -235,6 +222,13 @@ __global__ void silu_mul_vec_kernel(const T* __restrict__ gate_up, T* __restrict
     const float4 u = Vec4<T>::load(gate_up + row * 2 * inter + inter + col);
     Vec4<T>::store(out + row * inter + col, make_float4(gate_act(g.x, kind) * u.x, gate_act(g.y, kind) * u.y, gate_act(g.z, kind) * u.z, gate_act(g.w, kind) * u.w));
   }
+}
+
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float4& a, float4& b) {
+  const uint4 raw = *reinterpret_cast<const uint4*>(p);
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  a = make_float4(__bfloat162float(h[0].x), __bfloat162float(h[0].y), __bfloat162float(h[1].x), __bfloat162float(h[1].y));
+  b = make_float4(__bfloat162float(h[2].x), __bfloat162float(h[2].y), __bfloat162float(h[3].x), __bfloat162float(h[3].y));
 }
 
 // The same for bfloat16, eight neighbours per thread (inter % 8 == 0, 16-byte aligned), a block a run of one row's columns or, of narrow rows, blockDim.y whole rows: no
@@ -415,11 +409,15 @@ TLIE_EXPORT int tlie_embedding(int dtype, const void* table, const int* ids, flo
                                int* error_flag, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (vocab <= 0) return (int)cudaErrorInvalidValue;
-  if (hidden % 8 == 0 && ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(residual)) & 15) == 0) {
+  if (hidden % 4 == 0 && ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(residual)) & 15) == 0) {
+    const int pieces = hidden / 4;
+    int threads = 256, rows_per_block = 1;   // threads along a row; a block is 256 in all
+    while (threads > 1 && threads / 2 >= pieces) threads /= 2, rows_per_block *= 2;
+    const dim3 grid((unsigned)(((long long)rows + rows_per_block - 1) / rows_per_block)), block(threads, rows_per_block);
     if (dtype == TLIE_F32)
-      embedding_vec_kernel<float><<<rows, 256, 0, stream>>>((const float*)table, ids, residual, hidden, vocab, error_flag);
+      embedding_vec_kernel<float><<<grid, block, 0, stream>>>((const float*)table, ids, residual, rows, hidden, vocab, error_flag);
     else
-      embedding_vec_kernel<__nv_bfloat16><<<rows, 256, 0, stream>>>((const __nv_bfloat16*)table, ids, residual, hidden, vocab, error_flag);
+      embedding_vec_kernel<__nv_bfloat16><<<grid, block, 0, stream>>>((const __nv_bfloat16*)table, ids, residual, rows, hidden, vocab, error_flag);
     return (int)cudaGetLastError();
   }
   if (dtype == TLIE_F32)
