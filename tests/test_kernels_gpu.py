@@ -431,6 +431,28 @@ def test_sampling_over_blocks_keeps_the_set_and_the_order_of_tokens(ops, vocab):
             assert before - slack <= target <= float(kept[token]) + slack, (r, token)
 
 
+@pytest.mark.parametrize("vocab", [3073, 20000, 32768, 40001, 65536, 100000, 131069])
+def test_sampling_kernels_draw_what_the_simple_one_draws(ops, vocab):
+    """More rows than clusters run at once, greedy ones among them, flat tails (where another order of sums shows) and peaked rows: every draw as the simple kernel's, which
+    works with one block and one order of sums at any length."""
+    torch.manual_seed(44)
+    rows = 161
+    logits = (torch.randn(rows, vocab) * torch.tensor([0.3, 1.0, 3.0])[torch.arange(rows) % 3, None]).cuda()
+    logits[7], logits[8] = float("nan"), 0.0
+    temperature = torch.tensor([0.8, 1.3, 0.0, 0.5, 1.0])[torch.arange(rows) % 5].cuda()
+    top_p = torch.tensor([0.95, 0.5, 1.0, 0.999])[torch.arange(rows) % 4].cuda()
+    counters = torch.arange(rows, dtype=torch.int64, device="cuda")
+    for seed in range(3):
+        got, want = (torch.full((rows,), -7, dtype=torch.int32, device="cuda") for _ in range(2))
+        seeds = torch.full((rows,), seed, dtype=torch.int64, device="cuda")
+        ops.sample(logits, temperature, top_p, seeds, counters, got)
+        pointer = lambda t: ops.c_void_p(t.data_ptr())  # noqa: E731
+        assert ops.core().tlie_sample_simple(pointer(logits), ops.c_int(rows), ops.c_int(vocab), pointer(temperature), pointer(top_p), pointer(seeds), pointer(counters),
+                                             pointer(want), ops._stream()) == 0
+        assert torch.equal(got, want)
+        assert int(got.min()) >= 0 and int(got.max()) < vocab
+
+
 def test_argmax_and_sampling(ops):
     torch.manual_seed(7)
     logits = torch.randn(6, 1000)

@@ -102,9 +102,9 @@ __host__ __device__ inline float uniform_from(unsigned long long seed, unsigned 
   return (float)(z >> 40) * (1.0f / 16777216.0f);  // 24 bits -> [0, 1)
 }
 
-// Rows too long for sample_kernel: one block per row that works every probability out again in each pass.  temperature <= 0 means greedy for that row.
+// Rows too long for sample_kernel, and rows so short that most of its registers would hold nothing: one block per row that works every probability out again in each pass.  temperature <= 0 means greedy for that row.
 __global__ void __launch_bounds__(kSampleThreads)
-    sample_long_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
+    sample_simple_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
                   const float* __restrict__ top_p, const long long* __restrict__ seeds,
                   const long long* __restrict__ counters, int* __restrict__ out) {
   __shared__ float scratch[32];
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kSampleThreads)
 // probabilities stay in registers, 32 * CTAS per thread, so a question is that many comparisons and one sum over the block (and over the cluster through
 // distributed shared memory).  Read and exponentiated again for every question by one block, 64 rows of 32,000 took 550 us and 4 rows of
 // 128,256 took 800.
-// Every sum keeps the long kernel's order: 1,024 runs of consecutive tokens, one per thread of the cluster, added run by run, then 32 runs at a time, then
+// Every sum keeps the simple kernel's order: 1,024 runs of consecutive tokens, one per thread of the cluster, added run by run, then 32 runs at a time, then
 // those.  A token far down the tail has a probability near the rounding of the sums before it, so in another order one draw in a hundred that falls
 // into a flat tail would be another token.
 template <int CTAS>
@@ -416,15 +416,24 @@ TLIE_EXPORT int tlie_argmax(const float* logits, int rows, int vocab, int* out, 
   return (int)cudaGetLastError();
 }
 
+// By the simple kernel, whatever the rows' length: the order of sums that the other kernels keep.
+TLIE_EXPORT int tlie_sample_simple(const float* logits, int rows, int vocab, const float* temperature, const float* top_p,
+                                   const long long* seeds, const long long* counters, int* out, cudaStream_t stream) {
+  if (rows <= 0) return 0;
+  sample_simple_kernel<<<rows, kSampleThreads, 0, stream>>>(logits, vocab, temperature, top_p, seeds, counters, out);
+  return (int)cudaGetLastError();
+}
+
 TLIE_EXPORT int tlie_sample(const float* logits, int rows, int vocab, const float* temperature, const float* top_p,
                             const long long* seeds, const long long* counters, int* out, cudaStream_t stream) {
   if (rows <= 0) return 0;
   constexpr int kHeld = 32 * kSampleThreads;   // what a block's registers hold
+  constexpr int kShort = 3 * kSampleThreads;   // (1,000 tokens: 25 us, 30 by the kernel with 32 places per thread; 3,000: 30 and 30.4; 4,096: 32 and 30)
+  if (vocab <= kShort) return tlie_sample_simple(logits, rows, vocab, temperature, top_p, seeds, counters, out, stream);
   if (vocab <= kHeld) return launch_sample<1>(logits, rows, vocab, temperature, top_p, seeds, counters, out, stream);
   if (vocab <= 2 * kHeld) return launch_sample<2>(logits, rows, vocab, temperature, top_p, seeds, counters, out, stream);
   if (vocab <= 4 * kHeld) return launch_sample<4>(logits, rows, vocab, temperature, top_p, seeds, counters, out, stream);
-  sample_long_kernel<<<rows, kSampleThreads, 0, stream>>>(logits, vocab, temperature, top_p, seeds, counters, out);
-  return (int)cudaGetLastError();
+  return tlie_sample_simple(logits, rows, vocab, temperature, top_p, seeds, counters, out, stream);
 }
 
 TLIE_EXPORT float tlie_uniform_from(long long seed, long long counter) {
