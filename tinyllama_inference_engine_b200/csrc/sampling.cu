@@ -19,7 +19,8 @@ namespace tlie {
 constexpr int kSampleThreads = 1024;
 
 // A thread's share of a row's maximum and the lowest index that holds it (0x7fffffff: no value in its share can be compared).  Rows that allow it are read 16 bytes at a
-// time, four loads in flight per thread: one block reads a whole row, so its time is the latency of its loads in turn.
+// time, kInFlight loads in flight per thread: one block reads a whole row, so its time is the latency of its loads in turn.
+template <int kInFlight = 4>
 __device__ __forceinline__ void row_max_and_arg(const float* __restrict__ row, int vocab, float& best, int& arg) {
   auto take = [&](float v, int i) {
     if (v > best || (v == best && i < arg)) {
@@ -27,12 +28,11 @@ __device__ __forceinline__ void row_max_and_arg(const float* __restrict__ row, i
       arg = i;
     }
   };
+  // what fills up the last loads: no value is taken from it, while -INFINITY would be the maximum of a row without any comparable value, at an index past the row
+  const float nan = __int_as_float(0x7fffffff);
   if ((vocab & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
     const float4* row4 = reinterpret_cast<const float4*>(row);
     const int quads = vocab >> 2;
-    constexpr int kInFlight = 4;
-    // what fills up the last loads: no value is taken from it, while -INFINITY would be the maximum of a row without any comparable value, at an index past the row
-    const float nan = __int_as_float(0x7fffffff);
     const float4 nothing = make_float4(nan, nan, nan, nan);
     for (int q0 = threadIdx.x; q0 < quads; q0 += kInFlight * blockDim.x) {
       float4 v[kInFlight];
@@ -51,14 +51,26 @@ __device__ __forceinline__ void row_max_and_arg(const float* __restrict__ row, i
       }
     }
   } else {
-    for (int i = threadIdx.x; i < vocab; i += blockDim.x) take(row[i], i);
+    for (int i0 = threadIdx.x; i0 < vocab; i0 += kInFlight * blockDim.x) {
+      float v[kInFlight];
+#pragma unroll
+      for (int u = 0; u < kInFlight; ++u) v[u] = i0 + u * blockDim.x < vocab ? row[i0 + u * blockDim.x] : nan;
+#pragma unroll
+      for (int u = 0; u < kInFlight; ++u) take(v[u], i0 + u * blockDim.x);
+    }
   }
 }
 
-__global__ void __launch_bounds__(kSampleThreads) argmax_kernel(const float* __restrict__ logits, int vocab,
+// The lowest index of a row's maximum, by one block; token 0 for a row without any comparable value.
+// `temperature` (optional): rows above 0 are somebody else's; the kernel behind this one may then start early.
+__global__ void __launch_bounds__(kSampleThreads) argmax_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
                                                                 int* __restrict__ out) {
   __shared__ float best_value[32];
   __shared__ int best_index[32];
+  if (temperature != nullptr) {
+    grid_launch_dependents();
+    if (temperature[blockIdx.x] > 0.0f) return;
+  }
   const float* row = logits + (size_t)blockIdx.x * vocab;
   float value = -INFINITY;
   int index = 0x7fffffff;
@@ -214,20 +226,26 @@ __global__ void __launch_bounds__(kSampleThreads)
 // Every sum keeps the simple kernel's order: 1,024 runs of consecutive tokens, one per thread of the cluster, added run by run, then 32 runs at a time, then
 // those.  A token far down the tail has a probability near the rounding of the sums before it, so in another order one draw in a hundred that falls
 // into a flat tail would be another token.
+struct SampleShared {
+  float exchange[2][32];                    // the warps' partial results of the whole cluster, double buffered: one barrier per exchange
+  int arg_exchange[2][32];
+  __align__(16) float prefix[kSampleThreads];
+  float kept_total;
+  int chosen, last_kept;                    // the first block's are the row's
+};
+
+// One row.  `parity`: which half of the exchange buffers comes next (from row to row).
 template <int CTAS>
-__global__ void __launch_bounds__(kSampleThreads / CTAS)
-    sample_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature, const float* __restrict__ top_p,
-                  const long long* __restrict__ seeds, const long long* __restrict__ counters, int* __restrict__ out) {
+__device__ __forceinline__ void sample_row(SampleShared& shared, int& parity, int row_index, const float* __restrict__ logits, int vocab,
+                                           const float* __restrict__ temperature, const float* __restrict__ top_p, const long long* __restrict__ seeds,
+                                           const long long* __restrict__ counters, int* __restrict__ out) {
   namespace cg = cooperative_groups;
   constexpr int kThreads = kSampleThreads / CTAS, kWarps = kThreads / 32, kHeld = 32 * CTAS;
-  __shared__ float exchange[2][32];         // the warps' partial results of the whole cluster, double buffered: one barrier per exchange
-  __shared__ int arg_exchange[32];
-  __shared__ __align__(16) float prefix[kSampleThreads];
-  __shared__ float kept_total_smem;
-  __shared__ int chosen, last_kept;         // the first block's are the row's
+  auto& exchange = shared.exchange;
+  auto& arg_exchange = shared.arg_exchange;
+  auto& prefix = shared.prefix;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = CTAS > 1 ? (int)cluster.block_rank() : 0;
-  const int row_index = blockIdx.x / CTAS;
   const float* row = logits + (size_t)row_index * vocab;
   const float temp = temperature[row_index];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -236,12 +254,9 @@ __global__ void __launch_bounds__(kSampleThreads / CTAS)
     if (CTAS > 1) cluster.sync();
     else __syncthreads();
   };
-  if (CTAS > 1) cluster.sync();   // a block's shared memory may be written once the block runs
-
-  int parity = 0;
   // this thread's view of all 32 warps' values, lane w holds warp w's
   auto all_warps = [&](float mine) {
-    if (lane < CTAS) *(CTAS > 1 ? cluster.map_shared_rank(&exchange[parity][rank * kWarps + warp], lane) : &exchange[0][warp] + parity * 32) = mine;
+    if (lane < CTAS) *(CTAS > 1 ? cluster.map_shared_rank(&exchange[parity][rank * kWarps + warp], lane) : &exchange[parity][warp]) = mine;
     sync_all();
     const float value = exchange[parity][lane];
     parity ^= 1;
@@ -254,7 +269,7 @@ __global__ void __launch_bounds__(kSampleThreads / CTAS)
     const int first_id = min(vocab, rank * each), end_id = min(vocab, first_id + each);
     float value = -INFINITY;
     int index = 0x7fffffff;
-    row_max_and_arg(row + first_id, end_id - first_id, value, index);
+    row_max_and_arg<4 * CTAS>(row + first_id, end_id - first_id, value, index);   // as many in flight per row as one block of all the threads has
     if (index != 0x7fffffff) index += first_id;
 #pragma unroll
     for (int offset = 16; offset > 0; offset >>= 1) {
@@ -265,9 +280,9 @@ __global__ void __launch_bounds__(kSampleThreads / CTAS)
         index = oi;
       }
     }
-    if (lane < CTAS) *(CTAS > 1 ? cluster.map_shared_rank(&arg_exchange[rank * kWarps + warp], lane) : &arg_exchange[warp]) = index;
+    if (lane < CTAS) *(CTAS > 1 ? cluster.map_shared_rank(&arg_exchange[parity][rank * kWarps + warp], lane) : &arg_exchange[parity][warp]) = index;
     value = all_warps(value);
-    index = arg_exchange[lane];
+    index = arg_exchange[parity ^ 1][lane];
 #pragma unroll
     for (int offset = 16; offset > 0; offset >>= 1) {
       const float ov = __shfl_xor_sync(0xffffffffu, value, offset);
@@ -338,7 +353,7 @@ __global__ void __launch_bounds__(kSampleThreads / CTAS)
       kept += p[i];
       last = begin + i;
     }
-  if (threadIdx.x == 0) chosen = last_kept = -1;
+  if (threadIdx.x == 0) shared.chosen = shared.last_kept = -1;
 #pragma unroll
   for (int c = 0; c < CTAS; ++c) *(CTAS > 1 ? cluster.map_shared_rank(&prefix[run], c) : &prefix[run]) = kept;
   sync_all();
@@ -358,14 +373,14 @@ __global__ void __launch_bounds__(kSampleThreads / CTAS)
       running += v.w;
       *reinterpret_cast<float4*>(prefix + i) = start;
     }
-    kept_total_smem = running;
+    shared.kept_total = running;
   }
   __syncthreads();
-  const float target = uniform_from((unsigned long long)seeds[row_index], (unsigned long long)counters[row_index]) * kept_total_smem;
+  const float target = uniform_from((unsigned long long)seeds[row_index], (unsigned long long)counters[row_index]) * shared.kept_total;
   // the run whose [start, start + kept) holds the target walks its tokens
   const float start = prefix[run];
-  int* row_chosen = CTAS > 1 ? cluster.map_shared_rank(&chosen, 0) : &chosen;
-  int* row_last = CTAS > 1 ? cluster.map_shared_rank(&last_kept, 0) : &last_kept;
+  int* row_chosen = CTAS > 1 ? cluster.map_shared_rank(&shared.chosen, 0) : &shared.chosen;
+  int* row_last = CTAS > 1 ? cluster.map_shared_rank(&shared.last_kept, 0) : &shared.last_kept;
   if (kept > 0.0f && target >= start && target < start + kept) {
     float cursor = start;
     int pick = -1;
@@ -385,25 +400,67 @@ __global__ void __launch_bounds__(kSampleThreads / CTAS)
   if (rank == 0 && threadIdx.x == 0) {
     // rounding can put the target past the last kept token: take the last kept one; non-finite logits can leave nothing kept at all: the answer must
     // still be a token of the vocabulary
-    const int pick = chosen < 0 ? last_kept : chosen;
+    const int pick = shared.chosen < 0 ? shared.last_kept : shared.chosen;
     out[row_index] = (pick < 0 || pick >= vocab) ? 0 : pick;
   }
 }
 
+// A cluster takes rows until there are none: its registers let one block run per SM, and of more clusters than the SMs hold each would start anew, ask for its
+// row's temperature and wait.  What a row leaves in shared memory has been read when its cluster passes the next row's first barrier, and is written again behind that.
+// sampled_only: the greedy rows are argmax_kernel's.
+template <int CTAS>
+__global__ void __launch_bounds__(kSampleThreads / CTAS)
+    sample_kernel(const float* __restrict__ logits, int rows, int vocab, const float* __restrict__ temperature, const float* __restrict__ top_p,
+                  const long long* __restrict__ seeds, const long long* __restrict__ counters, int* __restrict__ out, int sampled_only) {
+  __shared__ SampleShared shared;
+  int parity = 0;
+  if (CTAS == 1) {
+    sample_row<1>(shared, parity, blockIdx.x, logits, vocab, temperature, top_p, seeds, counters, out);
+    return;
+  }
+  grid_dependency_wait();
+  cooperative_groups::this_cluster().sync();   // a block's shared memory may be written once the block runs
+  const int clusters = gridDim.x / CTAS, lane = threadIdx.x & 31;
+  for (int first = blockIdx.x / CTAS; first < rows; first += 32 * clusters) {
+    const int mine = first + lane * clusters;
+    unsigned todo = __ballot_sync(0xffffffffu, mine < rows && (!sampled_only || temperature[mine] > 0.0f));
+    for (; todo != 0u; todo &= todo - 1u)
+      sample_row<CTAS>(shared, parity, first + (__ffs(todo) - 1) * clusters, logits, vocab, temperature, top_p, seeds, counters, out);
+  }
+}
+
+// With more rows than clusters run at once, greedy ones go to argmax_kernel in front: a cluster's barriers cost as much as its part of such a row (us, all rows greedy, by the simple
+// kernel, by a cluster each, so: 64 rows of 128,256 10.1, 10.9, 9.0; 256 rows 24.8, 66, 23.9; 100 rows of 50,304 5.6, about 7, 6.6; none greedy, 256 rows of 128,256: 1,405, 390, 370).
 template <int CTAS>
 static int launch_sample(const float* logits, int rows, int vocab, const float* temperature, const float* top_p, const long long* seeds, const long long* counters,
                          int* out, cudaStream_t stream) {
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(rows * CTAS);
   config.blockDim = dim3(kSampleThreads / CTAS);
   config.stream = stream;
-  cudaLaunchAttribute attribute[1];
+  if (CTAS == 1) {
+    config.gridDim = dim3(rows);
+    return (int)cudaLaunchKernelEx(&config, sample_kernel<CTAS>, logits, rows, vocab, temperature, top_p, seeds, counters, out, 0);
+  }
+  cudaLaunchAttribute attribute[2];
   attribute[0].id = cudaLaunchAttributeClusterDimension;
   attribute[0].val.clusterDim.x = CTAS;
   attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
+  attribute[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
   config.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&config, sample_kernel<CTAS>, logits, vocab, temperature, top_p, seeds, counters, out);
+  config.gridDim = dim3(CTAS);   // (asked for a cluster's needs)
+  static const int resident = [&config] {
+    int clusters = 0;
+    return cudaOccupancyMaxActiveClusters(&clusters, sample_kernel<CTAS>, &config) == cudaSuccess && clusters > 0 ? clusters : 1;
+  }();
+  const int sampled_only = rows > resident;
+  if (sampled_only) {
+    argmax_kernel<<<rows, kSampleThreads, 0, stream>>>(logits, vocab, temperature, out);
+    config.numAttrs = 2;
+  }
+  config.gridDim = dim3((sampled_only ? resident : rows) * CTAS);
+  return (int)cudaLaunchKernelEx(&config, sample_kernel<CTAS>, logits, rows, vocab, temperature, top_p, seeds, counters, out, sampled_only);
 }
 
 }  // namespace tlie
@@ -412,7 +469,7 @@ using namespace tlie;
 
 TLIE_EXPORT int tlie_argmax(const float* logits, int rows, int vocab, int* out, cudaStream_t stream) {
   if (rows <= 0) return 0;
-  argmax_kernel<<<rows, kSampleThreads, 0, stream>>>(logits, vocab, out);
+  argmax_kernel<<<rows, kSampleThreads, 0, stream>>>(logits, vocab, nullptr, out);
   return (int)cudaGetLastError();
 }
 
