@@ -301,6 +301,43 @@ def test_steps_of_one_shape_queued_without_waiting_keep_their_own_descriptions(m
         assert torch.equal(a, b), index
 
 
+@pytest.mark.parametrize("publish", [True, False])
+def test_decode_steps_queued_without_reading_keep_their_own_tokens(model_folders, publish):
+    """A program that gives a session its tokens and reads none back runs ahead of the device: neither the next step's tokens, nor a new page, nor the requests loaded
+    next may be written under a copy that is still queued."""
+    from tinyllama_inference_engine_b200.engine.decode_session import DecodeSession
+
+    runner = ModelRunner(model_folders["b"], EngineConfig(dtype="float32", page_size=16, max_cache_tokens=1024, max_requests=8, max_batch_tokens=256))
+    vocab, steps = runner.spec.vocab_size, 20   # over the edge of a page
+    prompts = _prompts(vocab, [11, 5, 14, 8], seed=12)
+    following = [_prompts(vocab, [2] * steps, seed=13 + pair) for pair in range(2)]
+    session = DecodeSession(runner, 2, publish=publish)
+
+    def logits(wait):
+        got = []
+        for index, prompt in enumerate(prompts):
+            runner.step([StepEntry(f"r{index}", prompt, [])])
+        torch.cuda.synchronize()
+        if not wait:
+            torch.cuda._sleep(200_000_000)   # about a tenth of a second: the device is behind the host for the whole run
+        for pair in range(2):
+            session.load([f"r{2 * pair}", f"r{2 * pair + 1}"], following[pair][0])
+            for tokens in following[pair]:
+                session.set_tokens(tokens)
+                session.step()
+                got.append(session.logits.clone())
+                if wait:
+                    torch.cuda.synchronize()
+        for index in range(len(prompts)):
+            runner.finish(f"r{index}")
+        return got
+
+    want = logits(wait=True)
+    got = logits(wait=False)
+    for index, (a, b) in enumerate(zip(got, want)):
+        assert torch.equal(a, b), index
+
+
 @pytest.mark.parametrize("dtype,lengths", [("float32", [200, 17, 90]), ("bfloat16", [1200, 17, 831])])
 def test_last_layer_of_the_wanted_rows_alone_gives_their_logits(tmp_path, dtype, lengths):
     """Few wanted rows of many (one, several of an entry out of order, one twice, up to half of the step): the bits of a step that shows every row of every layer."""

@@ -42,6 +42,9 @@ class DecodeSession:
         view = lambda buffer, i: buffer[offsets[i] : offsets[i + 1]]  # noqa: E731
         self.h_tokens, self.h_positions = view(self._host, 0), view(self._host, 1)
         self._np = self._host.numpy()                       # the same pinned memory, for cheap host writes
+        # The host may be steps ahead of the device: pinned memory is written again only once the copies from it are done.  Those outside a step
+        # are followed by this event; a step's own copy of its input ids is done when the step has published its number.
+        self._copied = torch.cuda.Event()
         self._d_tokens = self._device[:count]               # where the step's input ids lie on the device
         # The step's result also arrives by itself: the last kernel of a step writes the tokens, the device error word and the
         # step's number into this pinned memory over the bus, and read_tokens() polls the number instead of waiting for two
@@ -77,6 +80,9 @@ class DecodeSession:
         """Bind ``count`` live requests: each one's next token (at the position its cache has reached) and sampling options."""
         if len(request_ids) != self.count or len(set(request_ids)) != self.count:
             raise BatchError(f"this decode session holds exactly {self.count} different requests")
+        self._copied.synchronize()
+        if self.publish:
+            self._wait_for_step()
         self.request_ids = list(request_ids)
         self.ctx.request_ids = self.request_ids
         self._fresh = True
@@ -97,6 +103,7 @@ class DecodeSession:
         self._fresh = False
         self._loaded = True
         self._device.copy_(self._host, non_blocking=True)
+        self._copied.record()
         if params is not None:
             self.temperature.copy_(torch.tensor([p.temperature for p in params], dtype=torch.float32))
             self.top_p.copy_(torch.tensor([p.top_p for p in params], dtype=torch.float32))
@@ -111,6 +118,8 @@ class DecodeSession:
             if self.positions[i] < self._capacity[i] and not self._fresh:
                 continue  # the position lies in a page the request already holds
             self.cache.reserve(request_id, self.positions[i] + 1)
+            if not changed:
+                self._copied.synchronize()
             record = self.cache.records[request_id]
             capacity = 1 << 60
             for g, group in enumerate(self.cache.page_groups):
@@ -139,9 +148,14 @@ class DecodeSession:
 
     def set_tokens(self, tokens: list[int]) -> None:
         """Host tokens in: the step's input ids come from pinned host memory."""
-        self._np[: self.count] = tokens
-        if not self.publish:
+        if self.publish:
+            self._wait_for_step()   # (a program that has read the last step's tokens does not wait here)
+            self._np[: self.count] = tokens
+        else:
+            self._copied.synchronize()
+            self._np[: self.count] = tokens
             self._d_tokens.copy_(self.h_tokens, non_blocking=True)
+            self._copied.record()
 
     def next_step_fits_its_pages(self) -> bool:
         """Whether every request's next position lies in a page it already holds (then the next step reserves nothing)."""
@@ -157,7 +171,15 @@ class DecodeSession:
             tokens = self.sampled.cpu()
             ops.check_device_errors(self.sampled.device)
             return tokens.tolist()
+        self._wait_for_step()
+        ops.raise_for_error_word(int(self._mail[self.count]), self._error_word.device)
+        return self._mail[: self.count].tolist()
+
+    def _wait_for_step(self) -> None:
+        """Until the last step issued has written its number into pinned memory."""
         mail, last, wanted = self._mail, self.count + 1, self._steps_issued
+        if mail[last] == wanted:
+            return
         stream = torch.cuda.current_stream()
         polls = 0
         while mail[last] != wanted:
@@ -166,8 +188,6 @@ class DecodeSession:
                 # the stream has nothing left to run and the number never came: a kernel of the step failed
                 stream.synchronize()
                 raise KernelError("a decode step ended without publishing its result")
-        ops.raise_for_error_word(int(mail[self.count]), self._error_word.device)
-        return mail[: self.count].tolist()
 
     def step(self) -> torch.Tensor:
         """One decode step for every request; returns the sampled tokens (device, int32).
@@ -178,6 +198,7 @@ class DecodeSession:
             if self._reserve_and_fill_tables():
                 o = self._offsets
                 self._device[o[8] :].copy_(self._host[o[8] :], non_blocking=True)
+                self._copied.record()
         self._loaded = False
         if not self.use_graph or self.graph is None and self._eager_steps < EAGER_STEPS_BEFORE_CAPTURE:
             if self._eager_steps == 0:
