@@ -19,6 +19,7 @@
 // which the CTA copies to shared memory 32 keys at a time while it works on the 32 before.
 #include "common.cuh"
 #include "mma_utils.cuh"
+#include "shared_memory_limit.cuh"
 
 namespace tlie {
 
@@ -253,8 +254,9 @@ template <int HEAD_DIM, int SLOTS>
 static int launch_shared(const float* q, int q_row_stride, const float* pages, const int* positions, const int* token_seq, const int* block_table,
                          int table_stride, float* out, int tokens, int q_heads, int kv_heads, int page_size, float scale, int rows_per_tile, cudaStream_t stream) {
   constexpr int smem = SharedAttention<HEAD_DIM, SLOTS>::kSmem;
-  static const cudaError_t configured = cudaFuncSetAttribute(paged_attention_shared_f32_kernel<HEAD_DIM, SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (configured != cudaSuccess) return (int)configured;
+  static std::atomic<unsigned long long> devices{0};
+  const cudaError_t allowed = allow_shared_memory(paged_attention_shared_f32_kernel<HEAD_DIM, SLOTS>, smem, devices);
+  if (allowed != cudaSuccess) return (int)allowed;
   paged_attention_shared_f32_kernel<HEAD_DIM, SLOTS><<<dim3((tokens + rows_per_tile - 1) / rows_per_tile, kv_heads), kSharedWarps * 32, smem, stream>>>(
       q, q_row_stride, pages, positions, token_seq, block_table, table_stride, out, tokens, q_heads, kv_heads, page_size, scale, rows_per_tile);
   return (int)cudaGetLastError();

@@ -12,6 +12,7 @@
 //   * operands that are not 16-byte aligned: a plain tile kernel.
 #include "common.cuh"
 #include "mma_utils.cuh"
+#include "shared_memory_limit.cuh"
 
 namespace tlie {
 
@@ -196,8 +197,9 @@ __global__ void __launch_bounds__(128) gemm_stream_f32_kernel(const float* __res
 template <int MP, int MM, int STAGES>
 static int launch_stream_stages(const float* x, const float* w, float* out, int M, int N, int K, long long lda, cudaStream_t stream) {
   constexpr int smem = STAGES * (kStreamN + MP) * kStreamStride * (int)sizeof(float);
-  static const cudaError_t configured = cudaFuncSetAttribute(gemm_stream_f32_kernel<MP, MM, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (configured != cudaSuccess) return (int)configured;
+  static std::atomic<unsigned long long> devices{0};
+  const cudaError_t allowed = allow_shared_memory(gemm_stream_f32_kernel<MP, MM, STAGES>, smem, devices);
+  if (allowed != cudaSuccess) return (int)allowed;
   return (int)launch_pdl(gemm_stream_f32_kernel<MP, MM, STAGES>, dim3((N + kStreamN - 1) / kStreamN), dim3(128), smem, stream, x, w, out, M, N, K, lda, device_sm_count());
 }
 
@@ -302,8 +304,9 @@ template <int TM, int TN, int WM, int WN>
 static int launch_wide(const float* x, const float* w, float* out, int M, int N, int K, long long lda, cudaStream_t stream) {
   constexpr int BM = TM * 4 * WM, BN = TN * 8 * WN;
   constexpr int smem = kTileStages * (BM + BN) * kWideStride * (int)sizeof(float);
-  static const cudaError_t configured = cudaFuncSetAttribute(gemm_wide_f32_kernel<TM, TN, WM, WN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (configured != cudaSuccess) return (int)configured;
+  static std::atomic<unsigned long long> devices{0};
+  const cudaError_t allowed = allow_shared_memory(gemm_wide_f32_kernel<TM, TN, WM, WN>, smem, devices);
+  if (allowed != cudaSuccess) return (int)allowed;
   return (int)launch_pdl(gemm_wide_f32_kernel<TM, TN, WM, WN>, dim3((unsigned)wide_tiles(M, N, BM, BN)), dim3(WM * WN * 32), smem, stream, x, w, out, M, N, K, lda);
 }
 
