@@ -56,8 +56,8 @@ def launchers(tmp_path_factory):
         pytest.skip("no nvcc")
     folder = tmp_path_factory.mktemp("fake_runtime")
     (folder / "runtime.cpp").write_text(FAKE_RUNTIME)
-    library = folder / "launchers.so"
-    subprocess.run([nvcc, "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-cudart", "none", "-gencode", "arch=compute_100a,code=sm_100a", "-Xptxas", "-O0",
+    library = folder / "launchers.so"   # -Bsymbolic: the real runtime may be loaded in this process too
+    subprocess.run([nvcc, "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-cudart", "none", "-Xlinker", "-Bsymbolic", "-gencode", "arch=compute_100a,code=sm_100a", "-Xptxas", "-O0",
                     "-I", str(CSRC), "-o", str(library), str(CSRC / "gemm_fp32.cu"), str(CSRC / "attention_generic.cu"), str(folder / "runtime.cpp")], check=True)
     return ctypes.CDLL(str(library))
 
