@@ -338,6 +338,43 @@ def test_decode_steps_queued_without_reading_keep_their_own_tokens(model_folders
         assert torch.equal(a, b), index
 
 
+def test_decode_session_waits_for_a_step_on_another_stream(model_folders):
+    """Steps on a stream of their own that is behind, tokens set, read and requests loaded from the default stream, which has nothing to do: that is no failed step."""
+    from tinyllama_inference_engine_b200.engine.decode_session import DecodeSession
+
+    runner = ModelRunner(model_folders["b"], EngineConfig(dtype="float32", page_size=16, max_cache_tokens=1024, max_requests=8, max_batch_tokens=256))
+    prompts = _prompts(runner.spec.vocab_size, [11, 5], seed=15)
+    following = _prompts(runner.spec.vocab_size, [2] * 5, seed=16)
+    session = DecodeSession(runner, 2)
+    side = torch.cuda.Stream()
+
+    def tokens(stream):
+        got = []
+        for index, prompt in enumerate(prompts):
+            runner.step([StepEntry(f"r{index}", prompt, [])])
+        for each in following:
+            session.load(["r0", "r1"], each)
+            torch.cuda.synchronize()
+            for read in (False, True):
+                with torch.cuda.stream(stream):
+                    if stream is side:
+                        torch.cuda._sleep(20_000_000)   # about ten milliseconds
+                    session.step()
+                if read:
+                    got.append(session.read_tokens())
+                else:
+                    session.set_tokens(each[::-1])
+            with torch.cuda.stream(stream):
+                session.step()
+        torch.cuda.synchronize()
+        for index in range(len(prompts)):
+            runner.finish(f"r{index}")
+        return got
+
+    want = tokens(torch.cuda.current_stream())
+    assert tokens(side) == want
+
+
 @pytest.mark.parametrize("dtype,lengths", [("float32", [200, 17, 90]), ("bfloat16", [1200, 17, 831])])
 def test_last_layer_of_the_wanted_rows_alone_gives_their_logits(tmp_path, dtype, lengths):
     """Few wanted rows of many (one, several of an entry out of order, one twice, up to half of the step): the bits of a step that shows every row of every layer."""

@@ -53,6 +53,7 @@ class DecodeSession:
         self._mail = self._mailbox.numpy()
         self._steps_done = torch.zeros(1, dtype=torch.int32, device=device)
         self._steps_issued = 0
+        self._step_stream: torch.cuda.Stream | None = None   # where the last step was issued (who waits for it may be on another stream)
         self._error_word = ops.error_flag(device)            # what kernels of this device report without a host in the loop
         self._capacity = [0] * count                        # tokens each request's pages hold (least over the groups)
         self.h_tables = [view(self._host, 8 + g).view(count, width) for g in range(groups)]
@@ -180,7 +181,7 @@ class DecodeSession:
         mail, last, wanted = self._mail, self.count + 1, self._steps_issued
         if mail[last] == wanted:
             return
-        stream = torch.cuda.current_stream()
+        stream = self._step_stream
         polls = 0
         while mail[last] != wanted:
             polls += 1
@@ -230,6 +231,7 @@ class DecodeSession:
         else:
             self.graph.replay()
         self._steps_issued += 1
+        self._step_stream = torch.cuda.current_stream()
         advance = self.cache.advance
         for i, request_id in enumerate(self.request_ids):
             self.positions[i] += 1
