@@ -800,6 +800,32 @@ def test_decode_attention_parts_that_are_warps(ops, q_heads, kv_heads, head_dim,
         assert float((got.cpu().float() - want.float()).abs().max()) <= 1.6e-2
 
 
+@pytest.mark.parametrize("q_heads,kv_heads,head_dim", [(32, 4, 64), (16, 8, 64), (8, 2, 128), (16, 2, 32)])
+@pytest.mark.parametrize("splits", [18, 32])
+def test_decode_attention_parts_that_are_warps_have_the_bits_of_parts_that_are_ctas(ops, q_heads, kv_heads, head_dim, splits):
+    """Every request twice: as it is, and behind eight tiles of keys whose weights are exactly 0, which are too many parts for one CTA and are merged by ticket.  (Parts
+    that count for nothing leave the others' sums as they are: added in order, and in the tree over lanes a multiple of eight away.)"""
+    from tinyllama_inference_engine_b200.ops import fast
+
+    rng = np.random.default_rng(37)
+    torch.manual_seed(37)
+    lens = [1, 2, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 160, 193, 255, 256]
+    count, page_size, empty = len(lens), 64, 4   # pages of 64 keys: 256 keys without weight
+    seq_lens = lens + [empty * page_size + n for n in lens]
+    qkv, pages, positions, token_seq, table = _paged_case(rng, torch.bfloat16, seq_lens, [1] * len(seq_lens), kv_heads, head_dim, page_size, q_heads)
+    qkv.view(len(seq_lens), -1, head_dim)[:, :q_heads, 0] = 4.0
+    qkv[count:] = qkv[:count]
+    pages[:, 0, :, :, 0] = 0.0
+    for i, n in enumerate(lens):
+        held = -(-n // page_size)
+        pages[table[count + i, empty : empty + held].long()] = pages[table[i, :held].long()]
+        pages[table[count + i, :empty].long(), 0] = torch.tensor([-4000.0] + [0.0] * (head_dim - 1), dtype=torch.bfloat16)   # scores below -1,400: 2 to their power is 0
+    got = torch.full((len(seq_lens), q_heads * head_dim), float("nan"), dtype=torch.bfloat16, device="cuda")
+    fast.decode_attention(qkv.cuda(), pages.cuda(), positions.cuda(), table.cuda(), got, q_heads, kv_heads, head_dim, page_size, 0, head_dim ** -0.5, splits)
+    assert bool(got.isfinite().all())
+    assert torch.equal(got[:count], got[count:])
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 128, 64), (128, 256, 128), (2048, 2560, 2048), (300, 200, 136), (2048, 2048, 5632), (129, 1000, 2048), (1000, 131, 80),
                                    (4200, 2500, 72)])
 @pytest.mark.parametrize("tile_n,pair", [(width, pair) for width in (128, 160, 192, 256) for pair in (False, True)] + [(288, False), (320, False), (288, True), (384, True), (480, True)])   # the wide tiles: two for single SMs, three for pairs
