@@ -10,8 +10,8 @@
 //     is read from HBM once per group, not once per head;
 //   * the key range of a request is cut into SPLITS parts so that small batches still fill the 148 SMs (none is needed when
 //     SPLITS == 1; parts of a single tile are warps of one CTA where they fit it);
-//   * each of the four warps of a CTA walks its own 32-key tiles with a private multi-stage
-//     cp.async pipeline (no block-wide barrier in the loop); rows in shared memory are padded
+//   * each warp of a CTA (eight up to head size 64, four above and in the narrow build) walks its own 32-key tiles with a private
+//     multi-stage cp.async pipeline (no block-wide barrier in the loop); rows in shared memory are padded
 //     by 16 bytes so that ldmatrix reads are free of bank conflicts for any head size;
 //   * q.K^T and P.V run on the tensor cores (mma.sync m16n8k16, bf16 in, 32-bit accumulate):
 //     with at most 16 rows per tile the 128-row tcgen05 shapes would be idle weight, and the

@@ -377,8 +377,8 @@ def sigmoid_gate(x, gate) -> None:
 def linear(x, weight, out) -> None:
     """out[M, N] = x[M, K] . weight[N, K]^T in the tensors' dtype (32-bit accumulation); ``x`` may be a run of columns of wider rows.
 
-    Up to 16 bfloat16 rows: the kernel reads ``weight`` while the kernel launched before it may still run, so ``weight`` must not be what that
-    kernel writes.  ``x`` may be, and in the 32-bit path ``weight`` too."""
+    Up to 16 bfloat16 rows: the kernel reads ``weight`` while the kernel launched before it (and, where that one was launched so itself, the ones before
+    that) may still run, so ``weight`` must not be what those write.  ``x`` may be, and in the 32-bit path ``weight`` too."""
     M, K = x.shape
     N = weight.shape[0]
     if weight.shape[1] != K or out.shape != (M, N):
@@ -649,8 +649,8 @@ def attention_step(qkv, positions, token_seq, block_table, inv_freq, rotary_dim:
                    head_dim: int, page_size: int, window: int = 0, scale: float | None = None, write_cache: bool = True, batch=None) -> None:
     """Rotate q and k, store k and v in the pages, and attend: ``rope_store`` then ``paged_attention``, in one kernel where one exists.
 
-    That one kernel (a step of one bfloat16 token per request) reads positions, block table, frequencies and every cached key but the new one while the kernel
-    launched before it may still run: of these that kernel must write none.  ``rope_store`` and ``paged_attention`` have no such condition."""
+    That one kernel (a step of one bfloat16 token per request) reads positions, block table, frequencies and every cached key but the new one while the kernels
+    launched just before it may still run (see ``linear``): of these they must write none.  ``rope_store`` and ``paged_attention`` have no such condition."""
     if qkv.dtype == torch.bfloat16:
         if fast.can_fuse_rope_into_decode(batch, qkv, head_dim, q_heads, kv_heads, inv_freq, rotary_dim):
             splits = fast.decode_splits(batch.num_seqs, kv_heads, batch.max_seq_len)
