@@ -83,7 +83,8 @@ constexpr int kStreamK = 128;        // columns of a ring stage
 constexpr int kStreamStride = kStreamK + 4;   // shared-memory row stride: 8 rows' 16-byte reads fall into different banks
 constexpr int kStreamAhead = 4;      // operands are in registers this many steps before they are used
 
-// Back to back in a graph, K = 2,048, 4 rows: 2,560 / 2,048 / 11,264 columns 11.8 / 9.4 / 27 us, K = 5,632: 25 us (the plain kernel 336 / 331 / 388 / 901).
+// Back to back in a graph, weights from HBM, 4 rows, K = 2,048: 2,560 / 2,048 / 11,264 columns 13.2 / 11.1 / 25.8 us, 2,048 columns of K = 5,632: 30.4 us (the plain kernel
+// 336 / 331 / 388 / 901); every read behind the dependency wait, which costs 1 to 2 us of that against weights copied in front of it.
 // MP: rows of x, rounded up to a power of two.  One or two warps own the outputs, a thread one weight row and MM rows of x; the others only
 // copy.  STAGES: what the CTA keeps in flight.  With at most one CTA per SM that has to cover the trip to HBM by itself.
 template <int MP, int MM, int STAGES>
@@ -310,8 +311,9 @@ static int launch_wide(const float* x, const float* w, float* out, int M, int N,
   return (int)launch_pdl(gemm_wide_f32_kernel<TM, TN, WM, WN>, dim3((unsigned)wide_tiles(M, N, BM, BN)), dim3(WM * WN * 32), smem, stream, x, w, out, M, N, K, lda);
 }
 
-// Which tile: the time of a product is that of the SM with the most tiles, about linear in their number.  Fitted to measurements at K = 2,048 (us;
-// a first tile that has the SM to itself waits for its own loads, the 8 x 8 tiles most): 24 rows x 2,048 columns 119 / 87 / 57 for the three tiles,
+// Which tile: the time of a product is that of the SM with the most tiles, about linear in their number.  Fitted to measurements at K = 2,048 alone: `each` grows with K and `once` does not, so at
+// a larger K the rule weighs the first tile's wait too much, which matters where two tiles are close.
+// In us (a first tile that has the SM to itself waits for its own loads, the 8 x 8 tiles most): 24 rows x 2,048 columns 119 / 87 / 57 for the three tiles,
 // 150 x 11,264 257 / 200 / 210, 300 x 11,264 341 / 386 / 398, 760 x 11,264 853 / 934 / 927 (the plain kernel: 387, 523, 743, 1,717).
 static int wide_choice(int M, int N) {
   const int sms = device_sm_count();
