@@ -148,6 +148,52 @@ def test_gemm_fp32_gives_a_row_the_same_bits_in_every_kernel(ops, N, K):
     assert torch.equal(got, full[:40])
 
 
+@pytest.mark.parametrize("N,K", [(96, 6208), (97, 64), (200, 14404), (2048, 36), (161, 130)])
+def test_gemm_fp32_in_parts_around_tiles_and_rounds(ops, N, K):
+    """Tiles of 128 rows of x by 64 or 96 of w, chunks of 64 k, rounds of 96 chunks, 16-byte copies and 4-byte ones: against 64-bit sums, and every row with the bits it has alone."""
+    torch.manual_seed(53)
+    x, w = torch.randn(600, K).cuda(), torch.randn(N, K).cuda()
+    exact = x.double() @ w.double().T
+    bound = K * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)   # one rounding per multiply-add of a sum of K terms: what a sum in order is held to
+    alone = torch.empty(600, N, device="cuda")
+    for first in range(0, 600, 16):
+        ops.linear(x[first : first + 16], w, alone[first : first + 16])
+    assert bool(((alone.double() - exact).abs() <= bound).all())
+    for M in (17, 63, 127, 128, 129, 256, 257, 600):
+        got = torch.full((M, N), float("nan"), device="cuda")
+        ops.linear(x[:M], w, got)
+        assert torch.equal(got, alone[:M]), M
+    assert int(ops.error_flag(x.device)) == 0, "a bounded wait inside the kernel gave up"
+
+
+@pytest.mark.parametrize("M", [1, 12, 140])
+def test_gemm_fp32_of_numbers_whose_parts_fall_out_of_range(ops, M):
+    """Infinities, NaN, sums beyond the largest number, numbers near it, and results near the smallest: as one sum of multiply-adds gives them."""
+    torch.manual_seed(54)
+    N, K = 100, 132
+    x, w = torch.randn(M, K), torch.randn(N, K)
+    w[:, 1] = 1.0   # (its middle and low parts are 0)
+    x[0, 1] = float("inf")
+    w[3, 5] = float("-inf")
+    w[7, 9] = float("nan")
+    w[11] = 3.3e38                      # sums beyond the largest number
+    w[12] = 0.0
+    w[12, 20] = 3.4028234e38            # its leading part would round to infinity
+    w[13] *= 1e-38                      # parts below the smallest bfloat16
+    x[:, 20] = 0.5
+    got = torch.empty(M, N, device="cuda")
+    ops.linear(x.cuda(), w.cuda(), got)
+    want = torch.zeros(M, N)
+    for k in range(K):   # (a product is exact in 64 bits, so one rounding to 32 bits per step, as a multiply-add's, but for ties of two roundings)
+        want = (want.double() + x[:, k].double()[:, None] * w[:, k].double()[None, :]).float()
+    got = got.cpu()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[want.isinf()], want[want.isinf()])
+    finite = want.isfinite()
+    bound = K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T) + K * 2.0 ** -149
+    assert bool(((got.double() - want.double()).abs() <= bound)[finite].all())
+
+
 @pytest.mark.parametrize("M", [1, 2, 4, 8, 16, 40])
 def test_gemm_fp32_takes_a_weight_that_the_kernel_before_it_writes(ops, M):
     """A product whose weight is the result of the product before it (which lets its successor start early), over and over on the same buffer."""

@@ -1,357 +1,474 @@
-// True 32-bit matrix product for the float32 path: out[M, N] = x[M, K] . w[N, K]^T (rows of x ``lda`` elements apart).
+// 32-bit matrix product for the float32 path: out[M, N] = x[M, K] . w[N, K]^T (rows of x ``lda`` elements apart), on the tensor cores without loss of precision.
 //
-// The reference's 32-bit model computes each output as one dot product over K in index
-// order (src/model.cpp:53-78).  These kernels keep that property on the GPU: every output
-// element is accumulated by one thread with fused multiply-adds in ascending k, so its
-// value depends on neither M nor N nor the kernel or tile it falls in, and no reduced-precision
-// tensor-core mode can be involved.  Three kernels, the same bits:
-//   * up to 16 rows (decoding): bound by the weights' bytes, or, for narrow products of long rows, by the chain of K dependent
-//     multiply-adds; a CTA streams 16 weight rows through a ring in shared memory that all of its threads fill, a thread per output;
-//   * more rows: register tiles of up to 8 x 8 outputs per thread, bound by the reads of shared memory that feed the FP32 pipes, operands in shared memory as they lie in
-//     global memory (k innermost, so that 16-byte asynchronous copies fill them and one 16-byte read feeds four steps of k);
-//   * operands that are not 16-byte aligned: a plain tile kernel.
-#include "common.cuh"
-#include "mma_utils.cuh"
+// The reference's 32-bit model computes each output as one dot product over K in index order (src/model.cpp:53-78).  The FP32 pipes are bound by what shared memory
+// delivers to them (45 of 72 TFLOP/s at 2,048 rows) and a sum over k in order by the chain of its multiply-adds.  Here every number is cut into three bfloat16 parts,
+// v = high + middle + low, each the rounded rest of the ones before it: 24 bits, nothing lost.  The product of two such numbers is the sum of nine products of parts;
+// the three that are below 2^-24 of it are left out, the other six are tensor-core products with 32-bit sums.
+//
+// The order of a sum is a definition, the same for every output whatever M, N, the kernel and the tile:
+//   * chunks of 64 k; a chunk's sum starts from zero and takes, 16 k at a time, first the five small kinds of products (low high, high low, middle middle,
+//     middle high, high middle; all 64 k of them), then the large one (high high).  The tensor core cuts off what lies below the last bit of the largest number it adds, so what is
+//     small is summed while the sum is small, and only four additions of a chunk are taken at full size;
+//   * the chunks' sums are added in order, in 32-bit, rounded to nearest.
+// A tcgen05.mma and an mma.sync m16n8k16 of the same 16 k give the same bits, and the place of a k among the 16 does not matter; so both kernels below keep to the definition:
+//   * up to 16 rows (decoding): bound by the weights' bytes; warps of a CTA take chunks of 16 rows of w in turn, straight from global memory to fragments (mma.sync);
+//   * more rows: tiles of 128 rows of x by 64 or 96 rows of w on tcgen05, operands cut on their way into shared memory.  Bound by shared memory: at 96 rows of w a chunk of 64 k brings
+//     112 KB through it on the way to registers, 84 KB of parts, and 168 KB that its 24 products read: 2,850 clocks at 128 bytes each; measured 2,550.
+// Against 64-bit sums the error is a sixth to a seventh of what multiply-adds in order give (2-norms over normal numbers: K = 2,048 1.3e-7, 8.1e-7; K = 5,632 1.9e-7, 1.34e-6).
+// Back to back in a graph, weights from HBM, the register kernels before -> these, in us:
+//   rows      2,560 x 2,048    2,048 x 2,048    11,264 x 2,048    2,048 x 5,632    32,000 x 2,048
+//      1      10.9 ->  8.5     10.1 ->  8.0      23.4 ->  23.6     26.0 ->  21       52 ->  57
+//      4      13.6 ->  8.7     12.3 ->  8.1      26.6 ->  24.0     30.5 ->  21       61 ->  57
+//     16      32.5 -> 14.5     16.8 ->  8.3      65.4 ->  36.4     44.1 ->  20      156 ->  98
+//     24      51.4 -> 50.4     51.4 -> 46.7      90.1 ->  77.5      138 -> 110      157 -> 153
+//    150       125 ->  57       107 ->  47        244 -> 100        262 -> 118      541 -> 235
+//    760       233 ->  80       236 ->  46        902 -> 220        624 -> 112
+//  2,048       671 -> 134       460 -> 132       2,225 -> 571      1,232 -> 330
+// Parts of an infinity are not finite, and of numbers below 2^-110 they fall out of range: an output that comes out not finite, or nonzero below 1e-30, is
+// worked out again as one sum of multiply-adds over k in order, by the thread that holds it, whichever kernel that is.
 #include "shared_memory_limit.cuh"
+#define TLIE_WITHOUT_TENSOR_MAPS
+#include "tcgen05_utils.cuh"
 
 namespace tlie {
 
-constexpr int kTile = 64;
-constexpr int kTileK = 16;
+constexpr int kChunkK = 64;
 
-__device__ __forceinline__ float4 read_four(unsigned addr) {   // k .. k + 3
-  float4 v;
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
-  return v;
+// a and b less a part of each, two subtractions in one instruction (exact: the part is the number's own leading bits, rounded).
+__device__ __forceinline__ void take_off(float& a, float& b, uint32_t part) {
+  unsigned long long both, parts, minus;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(both) : "f"(a), "f"(b));
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(parts) : "r"(part << 16), "r"(part & 0xffff0000u));
+  asm("mov.b64 %0, {%1, %1};\n" : "=l"(minus) : "f"(-1.0f));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(both) : "l"(parts), "l"(minus), "l"(both));
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(a), "=f"(b) : "l"(both));
+}
+// Two neighbours cut into parts (the first in the lower half of every word).
+__device__ __forceinline__ void cut_pair(float a, float b, uint32_t& high, uint32_t& middle, uint32_t& low) {
+  high = pack_bf16(a, b);
+  take_off(a, b, high);
+  middle = pack_bf16(a, b);
+  take_off(a, b, middle);
+  low = pack_bf16(a, b);
 }
 
-__global__ void __launch_bounds__(256) gemm_nt_f32_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                          float* __restrict__ out, int M, int N, int K, long long lda) {
-  __shared__ float xs[kTileK][kTile + 1];
-  __shared__ float ws[kTileK][kTile + 1];
-  const int tx = threadIdx.x % 16;
-  const int ty = threadIdx.x / 16;
-  const int row0 = blockIdx.y * kTile;
-  const int col0 = blockIdx.x * kTile;
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-
-  for (int k0 = 0; k0 < K; k0 += kTileK) {
-    for (int idx = threadIdx.x; idx < kTile * kTileK; idx += 256) {
-      const int r = idx / kTileK;
-      const int k = idx % kTileK;
-      const int gk = k0 + k;
-      const int gr = row0 + r;
-      const int gc = col0 + r;
-      xs[k][r] = (gr < M && gk < K) ? x[(size_t)gr * lda + gk] : 0.0f;
-      ws[k][r] = (gc < N && gk < K) ? w[(size_t)gc * K + gk] : 0.0f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kTileK; ++k) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = xs[k][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = ws[k][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gr = row0 + ty * 4 + i;
-    if (gr >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int gc = col0 + tx * 4 + j;
-      if (gc < N) out[(size_t)gr * N + gc] = acc[i][j];
-    }
-  }
+// Four neighbours of a row of K; zeros past its end.
+template <bool ALIGNED>
+__device__ __forceinline__ float4 load_four(const float* row, int k, int K) {
+  if (ALIGNED) return k < K ? __ldg(reinterpret_cast<const float4*>(row + k)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  return make_float4(k < K ? row[k] : 0.0f, k + 1 < K ? row[k + 1] : 0.0f, k + 2 < K ? row[k + 2] : 0.0f, k + 3 < K ? row[k + 3] : 0.0f);
 }
 
+// Asynchronous copies into shared memory; nothing is read and zeros arrive where `valid` is not set.
+__device__ __forceinline__ void cp_async_16(void* to, const void* from, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(to)), "l"(from), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_4(void* to, const void* from, bool valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(smem_u32(to)), "l"(from), "r"(valid ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
+// What the parts cannot hold (see above), worked out again.
+__device__ __noinline__ float sum_in_order(const float* __restrict__ x, const float* __restrict__ w, int K) {
+  float sum = 0.0f;
+  for (int k = 0; k < K; ++k) sum = fmaf(x[k], w[k], sum);
+  return sum;
+}
+__device__ __forceinline__ bool out_of_range(float v) { return !(fabsf(v) <= 3.402823466e38f) || (v != 0.0f && fabsf(v) < 1e-30f); }
 
 // --- up to 16 rows -----------------------------------------------------------------------------------
-constexpr int kStreamN = 16;         // weight rows of a CTA
-constexpr int kStreamK = 128;        // columns of a ring stage
-constexpr int kStreamStride = kStreamK + 4;   // shared-memory row stride: 8 rows' 16-byte reads fall into different banks
-constexpr int kStreamAhead = 4;      // operands are in registers this many steps before they are used
+constexpr int kFewThreads = 256;
+constexpr int kFewRows = 16;        // rows of w of a CTA
+constexpr int kFewRound = 96;       // chunks whose sums are in shared memory at a time
 
-// Back to back in a graph, weights from HBM, 4 rows, K = 2,048: 2,560 / 2,048 / 11,264 columns 13.2 / 11.1 / 25.8 us, 2,048 columns of K = 5,632: 30.4 us (the plain kernel
-// 336 / 331 / 388 / 901); every read behind the dependency wait, which costs 1 to 2 us of that against weights copied in front of it.
-// MP: rows of x, rounded up to a power of two.  One or two warps own the outputs, a thread one weight row and MM rows of x; the others only
-// copy.  STAGES: what the CTA keeps in flight.  With at most one CTA per SM that has to cover the trip to HBM by itself.
-template <int MP, int MM, int STAGES>
-__global__ void __launch_bounds__(128) gemm_stream_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ out, int M, int N,
-                                                              int K, long long lda, int sms) {
-  extern __shared__ __align__(16) float ring[];   // [stages][kStreamN + MP][kStreamStride]
-  constexpr int kThreads = 128;
-  constexpr int kStageFloats = (kStreamN + MP) * kStreamStride;
-  constexpr int kQuads = kStreamK / 4;
-  constexpr int kRows = MP / MM;
-  static_assert(kRows == 1 || kRows == 2 || kRows == 4, "");
-  struct Operands {
-    float4 w[kStreamAhead], x[kStreamAhead][MM];
-  };
-  const int n0 = blockIdx.x * kStreamN;
-  const int chunks = (K + kStreamK - 1) / kStreamK;
-  // rows past N or M repeat the last one (their outputs are not stored); columns past K are zeros.  A warp copies whole rows of a stage.
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto copy_w = [&](int chunk) {
-    float* stage = ring + (chunk % STAGES) * kStageFloats + lane * 4;
-    const int k = chunk * kStreamK + lane * 4;
-    const bool inside = k < K;
+__device__ __forceinline__ void mma_16x8x16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// NT: blocks of 8 rows of x.  A lane (g = lane / 4, t = lane % 4) holds rows g and g + 8 of w and row g of every block of x, k 4 t ... 4 t + 3 of every 16.
+template <int NT, bool ALIGNED>
+__global__ void __launch_bounds__(kFewThreads, NT == 1 ? 2 : 1) gemm_few_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ out, int M, int N, int K,
+                                                                  long long lda) {
+  extern __shared__ __align__(16) float sums[];   // [chunk of the round][NT][rows of x][rows of w]: 8 x 16 each
+  constexpr int kWarps = kFewThreads / 32;
+  constexpr int kOutputs = 8 * kFewRows * NT;
+  static_assert(kOutputs <= kFewThreads, "a thread adds up one output");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int n0 = blockIdx.x * kFewRows;
+  const int chunks = (K + kChunkK - 1) / kChunkK;
+  const float* w_rows[2] = {w + (long long)min(n0 + g, N - 1) * K, w + (long long)min(n0 + g + 8, N - 1) * K};
+  const float* x_rows[NT];
 #pragma unroll
-    for (int r = 0; r < kStreamN / 4; ++r)
-      cp_async_16(stage + (warp + 4 * r) * kStreamStride, w + (long long)min(n0 + warp + 4 * r, N - 1) * K + (inside ? k : 0), inside);
-  };
-  auto copy_x = [&](int chunk) {
-    float* stage = ring + (chunk % STAGES) * kStageFloats + kStreamN * kStreamStride + lane * 4;
-    const int k = chunk * kStreamK + lane * 4;
-    const bool inside = k < K;
-    for (int r = warp; r < MP; r += 4) cp_async_16(stage + r * kStreamStride, x + (long long)min(r, M - 1) * lda + (inside ? k : 0), inside);
-  };
-  // While the kernel before this one runs, L2 fetches the first stages' weights.  Nothing is read: w may be what that kernel (or the one before it) writes.
-  auto ask_for_w = [&](int chunk) {
-    const int k = chunk * kStreamK + lane * 4;
-#pragma unroll
-    for (int r = 0; r < kStreamN / 4; ++r)
-      if (k < K) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(w + (long long)min(n0 + warp + 4 * r, N - 1) * K + k));
-  };
-  for (int c = 0; c < STAGES - 1 && c < chunks; ++c) ask_for_w(c);
+  for (int j = 0; j < NT; ++j) x_rows[j] = x + (long long)min(8 * j + g, M - 1) * lda;
+  // While the kernel before this one runs, L2 fetches the warps' first chunks of weights.  Nothing is read: w may be what that kernel writes.
+  for (int c = warp; c < chunks && c < 4 * kWarps; c += kWarps)
+    for (int r = lane >> 1; r < kFewRows; r += 16) {
+      const int k = c * kChunkK + (lane & 1) * 32;
+      if (k < K) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(w + (long long)min(n0 + r, N - 1) * K + k));
+    }
   grid_launch_dependents();
   grid_dependency_wait();
-  for (int c = 0; c < STAGES - 1; ++c) {   // (empty groups keep the count)
-    if (c < chunks) {
-      copy_w(c);
-      copy_x(c);
+  float4 wv[2][4], xv[NT][4];
+  auto load = [&](int chunk) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int k = chunk * kChunkK + 16 * s + 4 * t;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) wv[r][s] = load_four<ALIGNED>(w_rows[r], k, K);
+#pragma unroll
+      for (int j = 0; j < NT; ++j) xv[j][s] = load_four<ALIGNED>(x_rows[j], k, K);
     }
-    cp_async_commit();
-  }
-  // a warp is 8 outputs x 4 rows (16 x 1, 16 x 2); CTAs that share an SM compute in different warps, so on different schedulers
-  constexpr int kWarpsNeeded = kRows == 4 ? 2 : 1;
-  const int turn = (kThreads / 32 + warp - (int)((blockIdx.x / sms) * kWarpsNeeded & 3)) & 3;
-  const bool computes = turn < kWarpsNeeded && (kRows > 1 || lane < 16);
-  const int n = kRows == 4 ? turn * 8 + (lane & 7) : lane & 15;
-  const int m = kRows == 4 ? lane >> 3 : (kRows == 2 ? lane >> 4 : 0);
-  float acc[MM];
+  };
+  float total = 0.0f;
+  if (warp < chunks) load(warp);
+  for (int first = 0; first < chunks; first += kFewRound) {
+    const int here = min(kFewRound, chunks - first);
+    for (int c = first + warp; c < first + here; c += kWarps) {
+      float acc[NT][4];
+      uint32_t wh[4][4], xh[NT][4][2];
 #pragma unroll
-  for (int j = 0; j < MM; ++j) acc[j] = 0.0f;
-  for (int c = 0; c < chunks; ++c) {
-    cp_async_wait<STAGES - 2>();
-    __syncthreads();   // stage c is here for every thread, and everyone is done with the stage that is filled next
-    if (c + STAGES - 1 < chunks) {
-      copy_w(c + STAGES - 1);
-      copy_x(c + STAGES - 1);
-    }
-    cp_async_commit();
-    if (computes) {
-      const unsigned stage = (unsigned)__cvta_generic_to_shared(ring + (c % STAGES) * kStageFloats);
-      const unsigned ws = stage + n * kStreamStride * 4, xs = stage + (kStreamN + m) * kStreamStride * 4;
-      // Two sets of operands in a rolled loop, one read while the other is used: what one pass of a loop reads for the next cannot be moved down to its use
-      // (unrolled, the reads are, whatever their order in the source, and every step waited for shared memory).
-      Operands even, odd;
-      auto fetch = [&](Operands& to, int group) {
+      for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
 #pragma unroll
-        for (int i = 0; i < kStreamAhead; ++i) {
-          to.w[i] = read_four(ws + 16 * (group * kStreamAhead + i));
+      for (int s = 0; s < 4; ++s) {
+        uint32_t wm[4], wl[4], xm[NT][2], xl[NT][2];
 #pragma unroll
-          for (int j = 0; j < MM; ++j) to.x[i][j] = read_four(xs + j * kRows * kStreamStride * 4 + 16 * (group * kStreamAhead + i));
+        for (int r = 0; r < 2; ++r) {
+          cut_pair(wv[r][s].x, wv[r][s].y, wh[s][r], wm[r], wl[r]);
+          cut_pair(wv[r][s].z, wv[r][s].w, wh[s][r + 2], wm[r + 2], wl[r + 2]);
         }
-      };
-      auto use = [&](const Operands& from) {
 #pragma unroll
-        for (int i = 0; i < kStreamAhead; ++i) {
-#pragma unroll
-          for (int j = 0; j < MM; ++j) acc[j] = fmaf(from.x[i][j].x, from.w[i].x, acc[j]);
-#pragma unroll
-          for (int j = 0; j < MM; ++j) acc[j] = fmaf(from.x[i][j].y, from.w[i].y, acc[j]);
-#pragma unroll
-          for (int j = 0; j < MM; ++j) acc[j] = fmaf(from.x[i][j].z, from.w[i].z, acc[j]);
-#pragma unroll
-          for (int j = 0; j < MM; ++j) acc[j] = fmaf(from.x[i][j].w, from.w[i].w, acc[j]);
+        for (int j = 0; j < NT; ++j) {
+          cut_pair(xv[j][s].x, xv[j][s].y, xh[j][s][0], xm[j][0], xl[j][0]);
+          cut_pair(xv[j][s].z, xv[j][s].w, xh[j][s][1], xm[j][1], xl[j][1]);
         }
-      };
-      constexpr int kGroups = kQuads / kStreamAhead;
-      fetch(even, 0);
-#pragma unroll 1
-      for (int group = 0; group < kGroups; group += 2) {
-        fetch(odd, group + 1);
-        use(even);
-        fetch(even, group + 2 < kGroups ? group + 2 : 0);   // (the last pass reads something it has)
-        use(odd);
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          mma_16x8x16(acc[j], wh[s], xl[j]);
+          mma_16x8x16(acc[j], wl, xh[j][s]);
+          mma_16x8x16(acc[j], wm, xm[j]);
+          mma_16x8x16(acc[j], wh[s], xm[j]);
+          mma_16x8x16(acc[j], wm, xh[j][s]);
+        }
+      }
+      if (c + kWarps < chunks) load(c + kWarps);   // the next chunk of this warp (of this round or the next) is on its way under what follows
+#pragma unroll
+      for (int s = 0; s < 4; ++s)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) mma_16x8x16(acc[j], wh[s], xh[j][s]);
+      float* to = sums + (c - first) * kOutputs;
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        float* block = to + j * 8 * kFewRows;
+        block[(2 * t) * kFewRows + g] = acc[j][0];
+        block[(2 * t + 1) * kFewRows + g] = acc[j][1];
+        block[(2 * t) * kFewRows + g + 8] = acc[j][2];
+        block[(2 * t + 1) * kFewRows + g + 8] = acc[j][3];
       }
     }
+    __syncthreads();
+    if (threadIdx.x < kOutputs) {
+#pragma unroll 8
+      for (int c = 0; c < here; ++c) total += sums[c * kOutputs + threadIdx.x];
+    }
+    __syncthreads();
   }
-  if (!computes || n0 + n >= N) return;
-#pragma unroll
-  for (int j = 0; j < MM; ++j)
-    if (m + j * kRows < M) out[(size_t)(m + j * kRows) * N + n0 + n] = acc[j];
+  const int m = threadIdx.x / kFewRows, n = n0 + threadIdx.x % kFewRows;
+  if (threadIdx.x < kOutputs && m < M && n < N) {
+    if (out_of_range(total)) total = sum_in_order(x + (long long)m * lda, w + (long long)n * K, K);
+    out[(size_t)m * N + n] = total;
+  }
 }
 
-template <int MP, int MM, int STAGES>
-static int launch_stream_stages(const float* x, const float* w, float* out, int M, int N, int K, long long lda, cudaStream_t stream) {
-  constexpr int smem = STAGES * (kStreamN + MP) * kStreamStride * (int)sizeof(float);
+template <int NT, bool ALIGNED>
+static int launch_few(const float* x, const float* w, float* out, int M, int N, int K, long long lda, cudaStream_t stream) {
+  const int chunks = (K + kChunkK - 1) / kChunkK;
+  const int smem = (chunks < kFewRound ? chunks : kFewRound) * 8 * kFewRows * NT * (int)sizeof(float);
   static std::atomic<unsigned long long> devices{0};
-  const cudaError_t allowed = allow_shared_memory(gemm_stream_f32_kernel<MP, MM, STAGES>, smem, devices);
+  const cudaError_t allowed = allow_shared_memory(gemm_few_f32_kernel<NT, ALIGNED>, kFewRound * 8 * kFewRows * NT * (int)sizeof(float), devices);
   if (allowed != cudaSuccess) return (int)allowed;
-  return (int)launch_pdl(gemm_stream_f32_kernel<MP, MM, STAGES>, dim3((N + kStreamN - 1) / kStreamN), dim3(128), smem, stream, x, w, out, M, N, K, lda, device_sm_count());
-}
-
-// MM rows per thread where a CTA has an SM (nearly) to itself and a sum's own chain is the time; MANY where there are more tiles than that and shared
-// memory's bandwidth is (4 rows x 11,264 columns, K = 2,048: 27.4 us with one row per thread, 26 with two; x 32,000: 69 and 58; 8 rows x 11,264: 47 with two, 37 with four).
-template <int MP, int MM, int MANY>
-static int launch_stream(const float* x, const float* w, float* out, int M, int N, int K, long long lda, cudaStream_t stream) {
-  if ((N + kStreamN - 1) / kStreamN <= 2 * device_sm_count()) return launch_stream_stages<MP, MM, 10>(x, w, out, M, N, K, lda, stream);
-  return launch_stream_stages<MP, MANY, 4>(x, w, out, M, N, K, lda, stream);
+  return (int)launch_pdl(gemm_few_f32_kernel<NT, ALIGNED>, dim3((N + kFewRows - 1) / kFewRows), dim3(kFewThreads), smem, stream, x, w, out, M, N, K, lda);
 }
 
 // --- more rows ---------------------------------------------------------------------------------------
-constexpr int kTileStages = 4;
-constexpr int kWideK = 16;
-constexpr int kWideStride = kWideK + 4;   // as above: 8 rows' 16-byte reads in one pass over the banks
+// Warps 0-7 cut and store the operands of a chunk (a ring of two stages), warp 8 issues its 24 products, warps 9-16 add the chunk's sum to the ones before it in
+// registers while the next chunk's products run into the other half of tensor memory.
+constexpr int kCutWarps = 8, kAddWarps = 8;
+constexpr int kManyThreads = (kCutWarps + 1 + kAddWarps) * 32;
+constexpr int kManyStages = 2;
 
-// A warp is 4 x 8 lanes, a lane TM x TN outputs: rows lane / 8 + 4 i, columns lane % 8 + 8 j (the eight lanes of one pass over the banks read eight
-// neighbouring weight rows, and one row of x).  Held back by what shared memory delivers, 16 values of four bytes per lane and k in the time of 64
-// multiply-adds: 45 TFLOP/s at 2,048 rows with 8 x 8 outputs per lane, of 72 (the plain kernel: 22; 8 x 16 outputs in twice the registers: 44; the next step's
-// operands read into a second set of registers: 43).
-template <int TM, int TN, int WM, int WN>
-__global__ void __launch_bounds__(WM * WN * 32) gemm_wide_f32_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                                     float* __restrict__ out, int M, int N, int K, long long lda) {
-  extern __shared__ __align__(16) float ring[];   // [stages][BM + BN][kWideStride]
-  constexpr int LM = 4, LN = 8;
-  constexpr int BM = TM * LM * WM, BN = TN * LN * WN;
-  constexpr int kThreads = WM * WN * 32;
-  constexpr int kStageFloats = (BM + BN) * kWideStride;
-  constexpr int kCopies = (BM + BN) * (kWideK / 4) / kThreads;
-  static_assert((BM + BN) * (kWideK / 4) % kThreads == 0, "every thread copies as much");
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int m_blocks = (M + BM - 1) / BM;
-  const int row0 = (blockIdx.x % m_blocks) * BM, col0 = (blockIdx.x / m_blocks) * BN;   // neighbours share their weights
-  const float* source[kCopies];
-#pragma unroll
-  for (int i = 0; i < kCopies; ++i) {
-    const int r = (threadIdx.x + i * kThreads) / (kWideK / 4);
-    source[i] = r < BM ? x + (long long)min(row0 + r, M - 1) * lda : w + (long long)min(col0 + r - BM, N - 1) * K;
+template <int BN>
+struct ManyShape {
+  static constexpr int kPlaneX = kBM * 128, kPlaneW = BN * 128;           // 64 k of one part
+  static constexpr int kStage = 3 * (kPlaneX + kPlaneW);                  // [x high, middle, low | w high, middle, low]
+  static constexpr int kFours = (kBM + BN) * (kChunkK / 4) / (kCutWarps * 32);   // float4 of a thread and chunk
+  static constexpr int kBatch = kFours % 7 == 0 ? 7 : 4;
+  static constexpr int kArrivals = kFours * kCutWarps * 32 * 16;          // where they arrive: a place for each
+  static constexpr int kSmem = kManyStages * kStage + kArrivals + 1024 + 256;
+  static_assert(kSmem <= 227 * 1024, "shared memory of one CTA");
+  static constexpr int kColumns = BN / 2;                                 // columns of an adding warp
+  static_assert(kColumns == 32 || kColumns == 48, "what an adding warp reads at once");
+};
+
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t chosen;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(chosen));
+  return chosen;
+}
+// The issuing warp walks its loop as a whole and one thread of it, always the same, executes what is issued: descriptors stay in uniform registers.
+__device__ __forceinline__ void umma_bf16_if(uint32_t issue, uint32_t tmem_d, uint32_t a_low, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      ".reg .b64 da, db;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "setp.ne.b32 q, %6, 0;\n"
+      "mov.b64 da, {%1, %5};\n"
+      "mov.b64 db, {%2, %5};\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "r"(a_low), "r"(b_low), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHigh), "r"(issue)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_if(uint32_t issue, uint32_t bar) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %1, 0;\n"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+      "}\n" ::"r"(bar), "r"(issue)
+      : "memory");
+}
+
+template <int BN, bool ALIGNED>
+__global__ void __launch_bounds__(kManyThreads, 1) gemm_many_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ out, int M, int N, int K,
+                                                                       long long lda, int* __restrict__ error_flag) {
+  using Shape = ManyShape<BN>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* ring = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* arrivals = ring + kManyStages * Shape::kStage;   // [float4 of a thread][thread]
+  uint64_t* full = reinterpret_cast<uint64_t*>(arrivals + Shape::kArrivals);
+  uint64_t* empty = full + kManyStages;
+  uint64_t* summed = empty + kManyStages;   // [2]: a chunk's products are done
+  uint64_t* taken = summed + 2;             // [2]: its sum has been read
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(taken + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int m_blocks = (M + kBM - 1) / kBM;
+  const int m0 = ((int)blockIdx.x % m_blocks) * kBM, n0 = ((int)blockIdx.x / m_blocks) * BN;   // neighbours share their weights
+  const int chunks = (K + kChunkK - 1) / kChunkK;
+  constexpr int kTmemStride = BN <= 64 ? 64 : 128, kTmemCols = 2 * kTmemStride;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kManyStages; ++s) {
+      mbar_init(&full[s], kCutWarps);
+      mbar_init(&empty[s], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&summed[a], 1);
+      mbar_init(&taken[a], kAddWarps);
+    }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  const int k_of = (threadIdx.x % (kWideK / 4)) * 4;
-  auto copy = [&](int chunk) {
-    const int k = chunk * kWideK + k_of;
-    const bool inside = k < K;
-    float* stage = ring + (chunk % kTileStages) * kStageFloats + k_of;
-#pragma unroll
-    for (int i = 0; i < kCopies; ++i)
-      cp_async_16(stage + ((threadIdx.x + i * kThreads) / (kWideK / 4)) * kWideStride, source[i] + (inside ? k : 0), inside);
-  };
-  const int chunks = (K + kWideK - 1) / kWideK;
+  if (warp == kCutWarps) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_holder)), "r"(kTmemCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t tmem = *tmem_holder;
   grid_launch_dependents();
   grid_dependency_wait();
-  for (int c = 0; c < kTileStages - 1; ++c) {
-    if (c < chunks) copy(c);
-    cp_async_commit();
-  }
-  const int m_of = (warp % WM) * TM * LM + (lane >> 3);
-  const int n_of = (warp / WM) * TN * LN + (lane & 7);
-  float acc[TM][TN];
+
+  if (warp < kCutWarps) {
+    // A thread's float4 i: row (thread / 16) + 16 i of the tile (x rows, then w rows), k 4 (thread % 16) of the chunk.  Rows past M or N repeat the last one.
+    const int first_row = threadIdx.x / 16, k_of = (threadIdx.x % 16) * 4;
+    // Each is copied to a place of its own thread's and read there by that thread; as soon as it has been read, the same place is asked to take the next chunk's, which
+    // travels while the others are cut.  (Held in registers instead, the loads of a chunk began when the cutting of the one before had ended, and a chunk took 4,400
+    // clocks for 1,536 of products.)
+    const bool whole = m0 + kBM <= M && n0 + BN <= N;
+    const float* x_first = x + (long long)min(m0 + first_row, M - 1) * lda;
+    const float* w_first = w + (long long)min(n0 + first_row, N - 1) * K;
+    auto row_of = [&](int i) {
+      if (whole) return i < kBM / 16 ? x_first + 16 * i * lda : w_first + (long long)(16 * (i - kBM / 16)) * K;
+      return i < kBM / 16 ? x + (long long)min(m0 + first_row + 16 * i, M - 1) * lda : w + (long long)min(n0 + first_row + 16 * i - kBM, N - 1) * K;
+    };
+    float4* const places = reinterpret_cast<float4*>(arrivals) + threadIdx.x;
+    auto ask = [&](int chunk, int i) {
+      const int k = chunk * kChunkK + k_of;
+      if (chunk < chunks) {
+        const float* row = row_of(i);
+        float4* place = places + i * (kCutWarps * 32);
+        if (ALIGNED) {
+          cp_async_16(place, k < K ? row + k : row, k < K);
+        } else {
 #pragma unroll
-  for (int i = 0; i < TM; ++i)
+          for (int e = 0; e < 4; ++e) cp_async_4(reinterpret_cast<float*>(place) + e, k + e < K ? row + k + e : row, k + e < K);
+        }
+      }
+    };
+    // kBatch at a time, a group each (an empty one behind the last chunk keeps the count), so that the chains of one number's cuts run beside those of others
+    constexpr int kBatch = Shape::kBatch, kBatches = Shape::kFours / kBatch;
+    // 8-byte pieces of 16-byte chunks of 128-byte rows, the chunks moved by the swizzle: rows 16 apart have the same r % 8
+    const uint32_t to = (uint32_t)first_row * 128 + ((((uint32_t)(k_of / 8)) ^ (first_row & 7)) << 4) + (k_of & 4) * 2;
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
-  for (int c = 0; c < chunks; ++c) {
-    cp_async_wait<kTileStages - 2>();
-    __syncthreads();
-    if (c + kTileStages - 1 < chunks) copy(c + kTileStages - 1);
-    cp_async_commit();
-    const float* xs = ring + (c % kTileStages) * kStageFloats + m_of * kWideStride;
-    const float* ws = ring + (c % kTileStages) * kStageFloats + (BM + n_of) * kWideStride;
+    for (int g = 0; g < kBatches; ++g) {
 #pragma unroll
-    for (int q = 0; q < kWideK / 4; ++q) {
-      float4 a[TM];
+      for (int i = 0; i < kBatch; ++i) ask(0, g * kBatch + i);
+      cp_async_commit();
+    }
+    for (int c = 0; c < chunks; ++c) {
+      const int s = c % kManyStages;
+      if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ((c / kManyStages) & 1) ^ 1, abort_flag))) break;
+      uint8_t* stage = ring + s * Shape::kStage + to;
 #pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(xs + LM * i * kWideStride + 4 * q);
+      for (int g = 0; g < kBatches; ++g) {
+        cp_async_wait<kBatches - 1>();   // the oldest of the groups on their way is this one
+        float4 v[kBatch];
 #pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        const float4 b = *reinterpret_cast<const float4*>(ws + LN * j * kWideStride + 4 * q);
+        for (int i = 0; i < kBatch; ++i) v[i] = places[(g * kBatch + i) * (kCutWarps * 32)];
 #pragma unroll
-        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].x, b.x, acc[i][j]);
+        for (int i = 0; i < kBatch; ++i) ask(c + 1, g * kBatch + i);
+        cp_async_commit();
 #pragma unroll
-        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].y, b.y, acc[i][j]);
+        for (int i = 0; i < kBatch; ++i) {
+          constexpr int kXFours = kBM / 16;
+          const int row = g * kBatch + i;
+          const bool of_x = row < kXFours;
+          uint2 high, middle, low;
+          cut_pair(v[i].x, v[i].y, high.x, middle.x, low.x);
+          cut_pair(v[i].z, v[i].w, high.y, middle.y, low.y);
+          uint8_t* at = stage + (of_x ? row * 2048 : 3 * Shape::kPlaneX + (row - kXFours) * 2048);
+          const int plane = of_x ? Shape::kPlaneX : Shape::kPlaneW;
+          *reinterpret_cast<uint2*>(at) = high;
+          *reinterpret_cast<uint2*>(at + plane) = middle;
+          *reinterpret_cast<uint2*>(at + 2 * plane) = low;
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // these writes -> visible to the tensor core
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full[s]);
+    }
+    cp_async_wait<0>();
+  } else if (warp == kCutWarps) {
+    const uint32_t issue = elect_one();
+    constexpr uint32_t idesc = umma_instr_desc(kBM, BN);
+    constexpr uint32_t kX = Shape::kPlaneX >> 4, kW = Shape::kPlaneW >> 4;   // in descriptor units
+    const uint32_t ring_low = umma_desc_low(smem_u32(ring));
+    for (int c = 0; c < chunks; ++c) {
+      const int s = c % kManyStages, b = c & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (c / kManyStages) & 1, abort_flag))) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(&taken[b], ((c / 2) & 1) ^ 1, abort_flag))) break;
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const uint32_t to = tmem + b * kTmemStride, xs = ring_low + s * (Shape::kStage >> 4), ws = xs + 3 * kX;
 #pragma unroll
-        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].z, b.z, acc[i][j]);
+      for (int k = 0; k < 4; ++k) {   // 16 k: 32 bytes inside the swizzle span
+        umma_bf16_if(issue, to, xs + 2 * kX + 2 * k, ws + 2 * k, idesc, k > 0 ? 1u : 0u);   // low of x, high of w
+        umma_bf16_if(issue, to, xs + 2 * k, ws + 2 * kW + 2 * k, idesc, 1u);                // high, low
+        umma_bf16_if(issue, to, xs + kX + 2 * k, ws + kW + 2 * k, idesc, 1u);               // middle, middle
+        umma_bf16_if(issue, to, xs + kX + 2 * k, ws + 2 * k, idesc, 1u);                    // middle, high
+        umma_bf16_if(issue, to, xs + 2 * k, ws + kW + 2 * k, idesc, 1u);                    // high, middle
+      }
 #pragma unroll
-        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].w, b.w, acc[i][j]);
+      for (int k = 0; k < 4; ++k) umma_bf16_if(issue, to, xs + 2 * k, ws + 2 * k, idesc, 1u);
+      umma_commit_if(issue, smem_u32(&empty[s]));
+      umma_commit_if(issue, smem_u32(&summed[b]));
+    }
+  } else {
+    const int sub = warp & 3, half = (warp - kCutWarps - 1) / 4;   // the quarter of the lanes that this warp may read; its half of the columns
+    const uint32_t from = tmem + ((uint32_t)(sub * 32) << 16) + half * Shape::kColumns;
+    float total[Shape::kColumns];
+#pragma unroll
+    for (int i = 0; i < Shape::kColumns; ++i) total[i] = 0.0f;
+    bool ok = true;
+    for (int c = 0; c < chunks; ++c) {
+      const int b = c & 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(&summed[b], (c / 2) & 1, abort_flag));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      uint32_t v[32], rest[16];
+      tmem_load_32(from + b * kTmemStride, v);
+      if (Shape::kColumns > 32) tmem_load_16(from + b * kTmemStride + 32, rest);
+      asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&taken[b]);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) total[j] += __uint_as_float(v[j]);
+      if (Shape::kColumns > 32) {
+#pragma unroll
+        for (int j = 32; j < Shape::kColumns; ++j) total[j] += __uint_as_float(rest[j - 32]);
       }
     }
-  }
+    const int m = m0 + sub * 32 + lane, first = n0 + half * Shape::kColumns;
+    if (ok && m < M) {
+      float* dst = out + (size_t)m * N + first;
+      const bool wide = N % 4 == 0 && ((uintptr_t)out & 15) == 0;
 #pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int row = row0 + m_of + LM * i;
-    if (row >= M) break;
+      for (int i = 0; i < Shape::kColumns; i += 4) {
 #pragma unroll
-    for (int j = 0; j < TN; ++j)
-      if (col0 + n_of + LN * j < N) out[(size_t)row * N + col0 + n_of + LN * j] = acc[i][j];
-  }
-}
-
-static long long wide_tiles(int M, int N, int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn); }
-
-template <int TM, int TN, int WM, int WN>
-static int launch_wide(const float* x, const float* w, float* out, int M, int N, int K, long long lda, cudaStream_t stream) {
-  constexpr int BM = TM * 4 * WM, BN = TN * 8 * WN;
-  constexpr int smem = kTileStages * (BM + BN) * kWideStride * (int)sizeof(float);
-  static std::atomic<unsigned long long> devices{0};
-  const cudaError_t allowed = allow_shared_memory(gemm_wide_f32_kernel<TM, TN, WM, WN>, smem, devices);
-  if (allowed != cudaSuccess) return (int)allowed;
-  return (int)launch_pdl(gemm_wide_f32_kernel<TM, TN, WM, WN>, dim3((unsigned)wide_tiles(M, N, BM, BN)), dim3(WM * WN * 32), smem, stream, x, w, out, M, N, K, lda);
-}
-
-// Which tile: the time of a product is that of the SM with the most tiles, about linear in their number.  Fitted to measurements at K = 2,048 alone: `each` grows with K and `once` does not, so at
-// a larger K the rule weighs the first tile's wait too much, which matters where two tiles are close.
-// In us (a first tile that has the SM to itself waits for its own loads, the 8 x 8 tiles most): 24 rows x 2,048 columns 119 / 87 / 57 for the three tiles,
-// 150 x 11,264 257 / 200 / 210, 300 x 11,264 341 / 386 / 398, 760 x 11,264 853 / 934 / 927 (the plain kernel: 387, 523, 743, 1,717).
-static int wide_choice(int M, int N) {
-  const int sms = device_sm_count();
-  const int bm[3] = {64, 32, 32}, bn[3] = {64, 128, 64};
-  const float each[3] = {57.0f, 62.0f, 32.0f}, once[3] = {40.0f, 25.0f, 25.0f};
-  int best = 0;
-  float least = 0.0f;
-  for (int i = 0; i < 3; ++i) {
-    const float time = each[i] * (float)((wide_tiles(M, N, bm[i], bn[i]) + sms - 1) / sms) + once[i];
-    if (i == 0 || time < least) {
-      best = i;
-      least = time;
+        for (int j = 0; j < 4; ++j)
+          if (first + i + j < N && out_of_range(total[i + j])) total[i + j] = sum_in_order(x + (long long)m * lda, w + (long long)(first + i + j) * K, K);
+        if (wide && first + i < N) {
+          *reinterpret_cast<float4*>(dst + i) = make_float4(total[i], total[i + 1], total[i + 2], total[i + 3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (first + i + j < N) dst[i + j] = total[i + j];
+        }
+      }
     }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   }
-  return best;
+  if (*abort_flag && threadIdx.x == 0 && error_flag != nullptr) atomicOr(error_flag, 1);
+  __syncthreads();
+  if (warp == kCutWarps) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kTmemCols));
+}
+
+template <int BN, bool ALIGNED>
+static int launch_many(const float* x, const float* w, float* out, int M, int N, int K, long long lda, int* error_flag, cudaStream_t stream) {
+  static std::atomic<unsigned long long> devices{0};
+  const cudaError_t allowed = allow_shared_memory(gemm_many_f32_kernel<BN, ALIGNED>, ManyShape<BN>::kSmem, devices);
+  if (allowed != cudaSuccess) return (int)allowed;
+  const long long tiles = (long long)((M + kBM - 1) / kBM) * ((N + BN - 1) / BN);
+  return (int)launch_pdl(gemm_many_f32_kernel<BN, ALIGNED>, dim3((unsigned)tiles), dim3(kManyThreads), ManyShape<BN>::kSmem, stream, x, w, out, M, N, K, lda, error_flag);
+}
+
+template <bool ALIGNED>
+static int launch_f32(const float* x, const float* w, float* out, int M, int N, int K, long long lda, int* error_flag, cudaStream_t stream) {
+  if (M <= 8) return launch_few<1, ALIGNED>(x, w, out, M, N, K, lda, stream);
+  if (M <= 16) return launch_few<2, ALIGNED>(x, w, out, M, N, K, lda, stream);
+  const long long m_blocks = (M + kBM - 1) / kBM, sms = device_sm_count();
+  const long long wide = (m_blocks * ((N + 95) / 96) + sms - 1) / sms, narrow = (m_blocks * ((N + 63) / 64) + sms - 1) / sms;   // waves
+  if (wide * 9 <= narrow * 8) return launch_many<96, ALIGNED>(x, w, out, M, N, K, lda, error_flag, stream);
+  return launch_many<64, ALIGNED>(x, w, out, M, N, K, lda, error_flag, stream);
 }
 
 }  // namespace tlie
 
 using namespace tlie;
 
-TLIE_EXPORT int tlie_gemm_nt_f32(const float* x, const float* w, float* out, int M, int N, int K, long long lda,
-                                 cudaStream_t stream) {
+// error_flag (device int, may be null): bit 0 is set if a wait gave up.
+TLIE_EXPORT int tlie_gemm_nt_f32_reporting(const float* x, const float* w, float* out, int M, int N, int K, long long lda, int* error_flag, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || lda < K) return (int)cudaErrorInvalidValue;
-  if (K % 4 == 0 && lda % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0) {
-    if (M == 1) return launch_stream<1, 1, 1>(x, w, out, M, N, K, lda, stream);
-    if (M == 2) return launch_stream<2, 1, 1>(x, w, out, M, N, K, lda, stream);
-    if (M <= 4) return launch_stream<4, 1, 2>(x, w, out, M, N, K, lda, stream);
-    if (M <= 8) return launch_stream<8, 2, 4>(x, w, out, M, N, K, lda, stream);
-    if (M <= 16) return launch_stream<16, 4, 4>(x, w, out, M, N, K, lda, stream);
-    switch (wide_choice(M, N)) {
-      case 0: return launch_wide<8, 8, 2, 1>(x, w, out, M, N, K, lda, stream);    // 64 x 64
-      case 1: return launch_wide<4, 8, 2, 2>(x, w, out, M, N, K, lda, stream);    // 32 x 128
-      default: return launch_wide<4, 4, 2, 2>(x, w, out, M, N, K, lda, stream);   // 32 x 64
-    }
-  }
-  dim3 grid((N + kTile - 1) / kTile, (M + kTile - 1) / kTile);
-  gemm_nt_f32_kernel<<<grid, 256, 0, stream>>>(x, w, out, M, N, K, lda);
-  return (int)cudaGetLastError();
+  if (K % 4 == 0 && lda % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0)
+    return launch_f32<true>(x, w, out, M, N, K, lda, error_flag, stream);
+  return launch_f32<false>(x, w, out, M, N, K, lda, error_flag, stream);
+}
+
+TLIE_EXPORT int tlie_gemm_nt_f32(const float* x, const float* w, float* out, int M, int N, int K, long long lda, cudaStream_t stream) {
+  return tlie_gemm_nt_f32_reporting(x, w, out, M, N, K, lda, nullptr, stream);
 }

@@ -275,6 +275,7 @@ __device__ __forceinline__ void store_tile_direct(uint32_t tmem_acc, int row, in
   }
 }
 
+#ifndef TLIE_WITHOUT_TENSOR_MAPS   // (a kernel that copies by other means does without the driver's entry point)
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
@@ -326,5 +327,7 @@ static bool make_add_map(CUtensorMap* map, const void* base, int M, int N) {
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+
+#endif
 
 }  // namespace tlie

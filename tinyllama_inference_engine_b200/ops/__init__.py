@@ -388,7 +388,7 @@ def linear(x, weight, out) -> None:
             raise KernelError("linear: the 32-bit path takes 32-bit weights and outputs", code="invalid_dtype")
         if not x.is_cuda or x.stride(1) != 1:
             raise KernelError("linear: x must be on a CUDA device with contiguous rows")
-        _check(core().tlie_gemm_nt_f32(c_void_p(x.data_ptr()), _ptr(weight), _ptr(out), c_int(M), c_int(N), c_int(K), c_longlong(x.stride(0)), _stream()), "gemm_nt_f32")
+        _check(core().tlie_gemm_nt_f32_reporting(c_void_p(x.data_ptr()), _ptr(weight), _ptr(out), c_int(M), c_int(N), c_int(K), c_longlong(x.stride(0)), _ptr(error_flag(x.device)), _stream()), "gemm_nt_f32")
         return
     fast.linear_bf16(x, weight, out)
 
