@@ -46,6 +46,7 @@ struct GemvArgs {
   // gate_limit): g * sigmoid(gate_alpha * g) * (u + gate_shift).
   int gate_kind;
   float gate_limit, gate_alpha, gate_shift;
+  int ahead_bytes;          // what a CTA asks L2 for before it waits for the kernel before it, beyond its first round
 };
 
 __device__ __forceinline__ float gemv_activate(int kind, float z, float a, float b) {
@@ -242,6 +243,27 @@ struct GemvPhase {
       const bool valid = kb * 32 + t * 8 < K;
       wreg[u][0] = valid ? load_stream_16(r0 + (size_t)kb * 32) : make_uint4(0, 0, 0, 0);
       wreg[u][1] = valid ? load_stream_16(r1 + (size_t)kb * 32) : make_uint4(0, 0, 0, 0);
+    }
+  }
+
+  // Asks L2 for what this CTA reads after its first round: the rest of its first tile, then its next tiles, as far as a.ahead_bytes go, so that HBM works on while the CTA waits for the
+  // kernel before it (the registers hold one round).  Sixteen threads, a row of the tile each.
+  __device__ __forceinline__ void ask_ahead(const GemvArgs& a, int first_tile, int tile_step) {
+    if (threadIdx.x >= 16) return;
+    const int n_rows = (EPI == EPI_GATED) ? a.N / 2 : a.N;
+    const int tiles = (n_rows + kTileRows - 1) / kTileRows;
+    const int r = threadIdx.x;
+    int left = a.ahead_bytes;
+    int from = WARPS * UNROLL * 32;   // columns of the first round
+    for (int tile = first_tile; tile < tiles && left > 0; tile += tile_step, from = 0) {
+      if (from >= a.K) continue;
+      const int n = tile * kTileRows + (EPI == EPI_GATED ? r & 7 : r);
+      const unsigned bytes = (unsigned)(a.K - from) * 2;
+      if (n < n_rows) {
+        const __nv_bfloat16* row = a.w + (size_t)(EPI == EPI_GATED && r >= 8 ? n_rows + n : n) * a.K + from;
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(row), "r"(bytes) : "memory");
+      }
+      left -= 16 * (int)bytes;
     }
   }
 
