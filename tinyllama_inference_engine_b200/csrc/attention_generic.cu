@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(kSharedWarps * 32) paged_attention_shared_f32_
   const int t0 = blockIdx.x * rows_per_tile, t1 = min(tokens, t0 + rows_per_tile);
   const size_t plane = (size_t)kv_heads * page_size * HEAD_DIM;
   const float* head_pages = pages + (size_t)g * page_size * HEAD_DIM;
+  const int page_shift = (page_size & (page_size - 1)) == 0 ? 31 - __clz(page_size) : -1;   // pages of a power of two: no division
 
   int row[SLOTS], head[SLOTS], pos[SLOTS];
 #pragma unroll
@@ -149,18 +150,33 @@ __global__ void __launch_bounds__(kSharedWarps * 32) paged_attention_shared_f32_
     while (last + 1 < t1 && token_seq[last + 1] == entry) longest = max(longest, positions[++last]);
     const int* table = block_table + (size_t)entry * table_stride;
     const int chunks = longest / kSharedKeys + 1;
-    auto copy = [&](int chunk) {
+    // A thread's pieces of a chunk lie in pages that it has looked up a chunk before: the table's answer is a trip to L2, and a copy that waited for it held every warp up in every
+    // chunk (four requests of 250 keys, 32 heads of 64 over 4: 17.3 us a launch).
+    constexpr int kPieces = kSharedKeys * kQuads / (kSharedWarps * 32);
+    int page[kPieces];
+    auto key_of = [&](int chunk, int i) { return chunk * kSharedKeys + ((int)threadIdx.x + i * kSharedWarps * 32) / kQuads; };
+    auto look_up = [&](int chunk) {
+#pragma unroll
+      for (int i = 0; i < kPieces; ++i) {
+        const int at = key_of(chunk, i);
+        page[i] = at <= longest ? table[page_shift >= 0 ? at >> page_shift : at / page_size] : 0;
+      }
+    };
+    auto copy = [&](int chunk) {   // whose pages have been looked up; then the next one's are
       float* stage = smem + (chunk % kSharedStages) * 2 * Shape::kPlane;
-      for (int i = threadIdx.x; i < kSharedKeys * kQuads; i += kSharedWarps * 32) {
-        const int key = i / kQuads, d = (i % kQuads) * 4;
-        const int at = chunk * kSharedKeys + key;
+#pragma unroll
+      for (int i = 0; i < kPieces; ++i) {
+        const int at = key_of(chunk, i), key = at - chunk * kSharedKeys, d = ((int)threadIdx.x + i * kSharedWarps * 32) % kQuads * 4;
         const bool seen = at <= longest;   // keys past the last one are zeros: nobody wrote them
-        const float* source = seen ? head_pages + (size_t)table[at / page_size] * 2 * plane + (size_t)(at % page_size) * HEAD_DIM + d : pages;
+        const int in_page = page_shift >= 0 ? at & (page_size - 1) : at % page_size;
+        const float* source = seen ? head_pages + (size_t)page[i] * 2 * plane + (size_t)in_page * HEAD_DIM + d : pages;
         cp_async_16(stage + key * Shape::kStride + d, source, seen);
         cp_async_16(stage + Shape::kPlane + key * Shape::kStride + d, seen ? source + plane : pages, seen);
       }
+      look_up(chunk + 1);
     };
     __syncthreads();   // everyone is done with the last request's stages
+    look_up(0);
     for (int c = 0; c < kSharedStages - 1; ++c) {
       if (c < chunks) copy(c);
       cp_async_commit();

@@ -17,9 +17,9 @@
 // Against 64-bit sums the error is a sixth to a seventh of what multiply-adds in order give (2-norms over normal numbers: K = 2,048 1.3e-7, 8.1e-7; K = 5,632 1.9e-7, 1.34e-6).
 // Back to back in a graph, weights from HBM, the register kernels before -> these, in us:
 //   rows      2,560 x 2,048    2,048 x 2,048    11,264 x 2,048    2,048 x 5,632    32,000 x 2,048
-//      1      10.9 ->  8.5     10.1 ->  8.0      23.4 ->  23.6     26.0 ->  21       52 ->  57
-//      4      13.6 ->  8.7     12.3 ->  8.1      26.6 ->  24.0     30.5 ->  21       61 ->  57
-//     16      32.5 -> 14.5     16.8 ->  8.3      65.4 ->  36.4     44.1 ->  20      156 ->  98
+//      1      10.9 ->  8.7     10.1 ->  6.3      23.4 ->  22.1     26.0 ->  12       52 ->  49
+//      4      13.6 ->  8.6     12.3 ->  6.5      26.6 ->  22.1     30.5 ->  12       61 ->  49
+//     16      32.5 -> 12.2     16.8 ->  7.6      65.4 ->  28.1     44.1 ->  16      156 ->  73
 //     24      51.4 -> 50.4     51.4 -> 46.7      90.1 ->  77.5      138 -> 110      157 -> 153
 //    150       125 ->  57       107 ->  47        244 -> 100        262 -> 118      541 -> 235
 //    760       233 ->  80       236 ->  46        902 -> 220        624 -> 112
@@ -81,8 +81,8 @@ __device__ __noinline__ float sum_in_order(const float* __restrict__ x, const fl
 __device__ __forceinline__ bool out_of_range(float v) { return !(fabsf(v) <= 3.402823466e38f) || (v != 0.0f && fabsf(v) < 1e-30f); }
 
 // --- up to 16 rows -----------------------------------------------------------------------------------
-constexpr int kFewThreads = 256;
 constexpr int kFewRows = 16;        // rows of w of a CTA
+constexpr int kFewAhead = 2;        // chunks of w on their way to a warp
 constexpr int kFewRound = 96;       // chunks whose sums are in shared memory at a time
 
 __device__ __forceinline__ void mma_16x8x16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
@@ -92,107 +92,145 @@ __device__ __forceinline__ void mma_16x8x16(float (&c)[4], const uint32_t (&a)[4
 }
 
 // NT: blocks of 8 rows of x.  A lane (g = lane / 4, t = lane % 4) holds rows g and g + 8 of w and row g of every block of x, k 4 t ... 4 t + 3 of every 16.
-template <int NT, bool ALIGNED>
-__global__ void __launch_bounds__(kFewThreads, NT == 1 ? 2 : 1) gemm_few_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ out, int M, int N, int K,
-                                                                  long long lda) {
-  extern __shared__ __align__(16) float sums[];   // [chunk of the round][NT][rows of x][rows of w]: 8 x 16 each
-  constexpr int kWarps = kFewThreads / 32;
+// WARPS: sixteen where a CTA has its SM to itself, eight where two share one.  A lane copies what it will read itself (w of two chunks ahead, whichever tile they belong to), so a warp's
+// ring needs no barrier, and an SM has 128 KB on its way from HBM (with the next chunk on its way to registers it was half of that: 11,264 x 2,048 24.5 us, 2,048 x 5,632 13).
+// A CTA walks row tiles blockIdx.x, + gridDim.x, ...
+template <int NT, int WARPS, bool ALIGNED>
+__global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gemm_few_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ out,
+                                                                                                int M, int N, int K, long long lda) {
+  extern __shared__ __align__(16) float ring[];   // [warp][kFewAhead][8][lane] float4, then the sums
+  float* sums = ring + WARPS * kFewAhead * kFewRows * kChunkK;   // [chunk of the round][NT][rows of x][rows of w]: 8 x 16 each
   constexpr int kOutputs = 8 * kFewRows * NT;
-  static_assert(kOutputs <= kFewThreads, "a thread adds up one output");
+  static_assert(kOutputs <= WARPS * 32, "a thread adds up one output");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int n0 = blockIdx.x * kFewRows;
-  const int chunks = (K + kChunkK - 1) / kChunkK;
-  const float* w_rows[2] = {w + (long long)min(n0 + g, N - 1) * K, w + (long long)min(n0 + g + 8, N - 1) * K};
+  const int tiles = (N + kFewRows - 1) / kFewRows, chunks = (K + kChunkK - 1) / kChunkK;
   const float* x_rows[NT];
 #pragma unroll
   for (int j = 0; j < NT; ++j) x_rows[j] = x + (long long)min(8 * j + g, M - 1) * lda;
-  // While the kernel before this one runs, L2 fetches the warps' first chunks of weights.  Nothing is read: w may be what that kernel writes.
-  for (int c = warp; c < chunks && c < 4 * kWarps; c += kWarps)
-    for (int r = lane >> 1; r < kFewRows; r += 16) {
-      const int k = c * kChunkK + (lane & 1) * 32;
-      if (k < K) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(w + (long long)min(n0 + r, N - 1) * K + k));
-    }
+  // While the kernel before this one runs, L2 fetches the CTA's first chunks of weights.  Nothing is read: w may be what that kernel writes.
+  for (int c = warp; c < chunks && c < 4 * WARPS; c += WARPS) {
+    const int k = c * kChunkK + (lane & 1) * 32;
+    if (k < K) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(w + (long long)min((int)blockIdx.x * kFewRows + (lane >> 1), N - 1) * K + k));
+  }
   grid_launch_dependents();
   grid_dependency_wait();
-  float4 wv[2][4], xv[NT][4];
-  auto load = [&](int chunk) {
+  float4* const mine = reinterpret_cast<float4*>(ring) + warp * kFewAhead * 8 * 32 + lane;
+  int ask_tile = warp < chunks ? (int)blockIdx.x : tiles, ask_chunk = warp;
+  auto ask = [&](int slot) {   // w of the next chunk in this warp's order; a group each (an empty one behind the last keeps the count)
+    if (ask_tile < tiles) {
+      const int n = ask_tile * kFewRows + g;
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int k = chunk * kChunkK + 16 * s + 4 * t;
+      for (int r = 0; r < 2; ++r) {
+        const float* row = w + (long long)min(n + 8 * r, N - 1) * K;
 #pragma unroll
-      for (int r = 0; r < 2; ++r) wv[r][s] = load_four<ALIGNED>(w_rows[r], k, K);
+        for (int s = 0; s < 4; ++s) {
+          const int k = ask_chunk * kChunkK + 16 * s + 4 * t;
+          float4* place = mine + (slot * 8 + r * 4 + s) * 32;
+          if (ALIGNED) {
+            cp_async_16(place, k < K ? row + k : row, k < K);
+          } else {
 #pragma unroll
-      for (int j = 0; j < NT; ++j) xv[j][s] = load_four<ALIGNED>(x_rows[j], k, K);
+            for (int e = 0; e < 4; ++e) cp_async_4(reinterpret_cast<float*>(place) + e, k + e < K ? row + k + e : row, k + e < K);
+          }
+        }
+      }
+      ask_chunk += WARPS;
+      if (ask_chunk >= chunks) ask_chunk = warp, ask_tile += gridDim.x;
     }
+    cp_async_commit();
   };
-  float total = 0.0f;
-  if (warp < chunks) load(warp);
-  for (int first = 0; first < chunks; first += kFewRound) {
-    const int here = min(kFewRound, chunks - first);
-    for (int c = first + warp; c < first + here; c += kWarps) {
-      float acc[NT][4];
-      uint32_t wh[4][4], xh[NT][4][2];
+  float4 xv[NT][4];
+  auto load_x = [&](int chunk) {
 #pragma unroll
-      for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+    for (int j = 0; j < NT; ++j)
 #pragma unroll
-      for (int s = 0; s < 4; ++s) {
-        uint32_t wm[4], wl[4], xm[NT][2], xl[NT][2];
+      for (int s = 0; s < 4; ++s) xv[j][s] = load_four<ALIGNED>(x_rows[j], chunk * kChunkK + 16 * s + 4 * t, K);
+  };
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          cut_pair(wv[r][s].x, wv[r][s].y, wh[s][r], wm[r], wl[r]);
-          cut_pair(wv[r][s].z, wv[r][s].w, wh[s][r + 2], wm[r + 2], wl[r + 2]);
+  for (int s = 0; s < kFewAhead; ++s) ask(s);
+  if (warp < chunks) load_x(warp);
+  int slot = 0;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int n0 = tile * kFewRows;
+    float total = 0.0f;
+    for (int first = 0; first < chunks; first += kFewRound) {
+      const int here = min(kFewRound, chunks - first);
+      for (int c = first + warp; c < first + here; c += WARPS) {
+        float acc[NT][4];
+        uint32_t wh[4][4], xh[NT][4][2];
+        cp_async_wait<kFewAhead - 1>();
+        float4 wv[2][4];
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+          for (int s = 0; s < 4; ++s) wv[r][s] = mine[(slot * 8 + r * 4 + s) * 32];
+        ask(slot);
+        slot = slot + 1 == kFewAhead ? 0 : slot + 1;
+#pragma unroll
+        for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          uint32_t wm[4], wl[4], xm[NT][2], xl[NT][2];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            cut_pair(wv[r][s].x, wv[r][s].y, wh[s][r], wm[r], wl[r]);
+            cut_pair(wv[r][s].z, wv[r][s].w, wh[s][r + 2], wm[r + 2], wl[r + 2]);
+          }
+#pragma unroll
+          for (int j = 0; j < NT; ++j) {
+            cut_pair(xv[j][s].x, xv[j][s].y, xh[j][s][0], xm[j][0], xl[j][0]);
+            cut_pair(xv[j][s].z, xv[j][s].w, xh[j][s][1], xm[j][1], xl[j][1]);
+          }
+#pragma unroll
+          for (int j = 0; j < NT; ++j) {
+            mma_16x8x16(acc[j], wh[s], xl[j]);
+            mma_16x8x16(acc[j], wl, xh[j][s]);
+            mma_16x8x16(acc[j], wm, xm[j]);
+            mma_16x8x16(acc[j], wh[s], xm[j]);
+            mma_16x8x16(acc[j], wm, xh[j][s]);
+          }
         }
+        load_x(c + WARPS < chunks ? c + WARPS : warp);   // of the next chunk, or of the next tile's first one
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+#pragma unroll
+          for (int j = 0; j < NT; ++j) mma_16x8x16(acc[j], wh[s], xh[j][s]);
+        float* to = sums + (c - first) * kOutputs;
 #pragma unroll
         for (int j = 0; j < NT; ++j) {
-          cut_pair(xv[j][s].x, xv[j][s].y, xh[j][s][0], xm[j][0], xl[j][0]);
-          cut_pair(xv[j][s].z, xv[j][s].w, xh[j][s][1], xm[j][1], xl[j][1]);
-        }
-#pragma unroll
-        for (int j = 0; j < NT; ++j) {
-          mma_16x8x16(acc[j], wh[s], xl[j]);
-          mma_16x8x16(acc[j], wl, xh[j][s]);
-          mma_16x8x16(acc[j], wm, xm[j]);
-          mma_16x8x16(acc[j], wh[s], xm[j]);
-          mma_16x8x16(acc[j], wm, xh[j][s]);
+          float* block = to + j * 8 * kFewRows;
+          block[(2 * t) * kFewRows + g] = acc[j][0];
+          block[(2 * t + 1) * kFewRows + g] = acc[j][1];
+          block[(2 * t) * kFewRows + g + 8] = acc[j][2];
+          block[(2 * t + 1) * kFewRows + g + 8] = acc[j][3];
         }
       }
-      if (c + kWarps < chunks) load(c + kWarps);   // the next chunk of this warp (of this round or the next) is on its way under what follows
-#pragma unroll
-      for (int s = 0; s < 4; ++s)
-#pragma unroll
-        for (int j = 0; j < NT; ++j) mma_16x8x16(acc[j], wh[s], xh[j][s]);
-      float* to = sums + (c - first) * kOutputs;
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        float* block = to + j * 8 * kFewRows;
-        block[(2 * t) * kFewRows + g] = acc[j][0];
-        block[(2 * t + 1) * kFewRows + g] = acc[j][1];
-        block[(2 * t) * kFewRows + g + 8] = acc[j][2];
-        block[(2 * t + 1) * kFewRows + g + 8] = acc[j][3];
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x < kOutputs) {
+      __syncthreads();
+      if (threadIdx.x < kOutputs) {
 #pragma unroll 8
-      for (int c = 0; c < here; ++c) total += sums[c * kOutputs + threadIdx.x];
+        for (int c = 0; c < here; ++c) total += sums[c * kOutputs + threadIdx.x];
+      }
+      __syncthreads();
     }
-    __syncthreads();
+    const int m = threadIdx.x / kFewRows, n = n0 + threadIdx.x % kFewRows;
+    if (threadIdx.x < kOutputs && m < M && n < N) {
+      if (out_of_range(total)) total = sum_in_order(x + (long long)m * lda, w + (long long)n * K, K);
+      out[(size_t)m * N + n] = total;
+    }
   }
-  const int m = threadIdx.x / kFewRows, n = n0 + threadIdx.x % kFewRows;
-  if (threadIdx.x < kOutputs && m < M && n < N) {
-    if (out_of_range(total)) total = sum_in_order(x + (long long)m * lda, w + (long long)n * K, K);
-    out[(size_t)m * N + n] = total;
-  }
+  cp_async_wait<0>();
 }
 
-template <int NT, bool ALIGNED>
+template <int NT, int WARPS, bool ALIGNED>
 static int launch_few(const float* x, const float* w, float* out, int M, int N, int K, long long lda, cudaStream_t stream) {
-  const int chunks = (K + kChunkK - 1) / kChunkK;
-  const int smem = (chunks < kFewRound ? chunks : kFewRound) * 8 * kFewRows * NT * (int)sizeof(float);
+  const int chunks = (K + kChunkK - 1) / kChunkK, tiles = (N + kFewRows - 1) / kFewRows;
+  constexpr int ring = WARPS * kFewAhead * kFewRows * kChunkK * (int)sizeof(float);
+  const int smem = ring + (chunks < kFewRound ? chunks : kFewRound) * 8 * kFewRows * NT * (int)sizeof(float);
+  const int places = (NT == 1 && WARPS == 8 ? 2 : 1) * device_sm_count();
   static std::atomic<unsigned long long> devices{0};
-  const cudaError_t allowed = allow_shared_memory(gemm_few_f32_kernel<NT, ALIGNED>, kFewRound * 8 * kFewRows * NT * (int)sizeof(float), devices);
+  const cudaError_t allowed = allow_shared_memory(gemm_few_f32_kernel<NT, WARPS, ALIGNED>, ring + kFewRound * 8 * kFewRows * NT * (int)sizeof(float), devices);
   if (allowed != cudaSuccess) return (int)allowed;
-  return (int)launch_pdl(gemm_few_f32_kernel<NT, ALIGNED>, dim3((N + kFewRows - 1) / kFewRows), dim3(kFewThreads), smem, stream, x, w, out, M, N, K, lda);
+  return (int)launch_pdl(gemm_few_f32_kernel<NT, WARPS, ALIGNED>, dim3(tiles < places ? tiles : places), dim3(WARPS * 32), smem, stream, x, w, out, M, N, K, lda);
 }
 
 // --- more rows ---------------------------------------------------------------------------------------
@@ -448,8 +486,11 @@ static int launch_many(const float* x, const float* w, float* out, int M, int N,
 
 template <bool ALIGNED>
 static int launch_f32(const float* x, const float* w, float* out, int M, int N, int K, long long lda, int* error_flag, cudaStream_t stream) {
-  if (M <= 8) return launch_few<1, ALIGNED>(x, w, out, M, N, K, lda, stream);
-  if (M <= 16) return launch_few<2, ALIGNED>(x, w, out, M, N, K, lda, stream);
+  if (M <= 8) {
+    if ((N + kFewRows - 1) / kFewRows <= device_sm_count()) return launch_few<1, 16, ALIGNED>(x, w, out, M, N, K, lda, stream);
+    return launch_few<1, 8, ALIGNED>(x, w, out, M, N, K, lda, stream);
+  }
+  if (M <= 16) return launch_few<2, 8, ALIGNED>(x, w, out, M, N, K, lda, stream);
   const long long m_blocks = (M + kBM - 1) / kBM, sms = device_sm_count();
   const long long wide = (m_blocks * ((N + 95) / 96) + sms - 1) / sms, narrow = (m_blocks * ((N + 63) / 64) + sms - 1) / sms;   // waves
   if (wide * 9 <= narrow * 8) return launch_many<96, ALIGNED>(x, w, out, M, N, K, lda, error_flag, stream);
