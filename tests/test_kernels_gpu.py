@@ -148,7 +148,7 @@ def test_gemm_fp32_gives_a_row_the_same_bits_in_every_kernel(ops, N, K):
     assert torch.equal(got, full[:40])
 
 
-@pytest.mark.parametrize("N,K", [(96, 6208), (97, 64), (200, 14404), (2048, 36), (161, 130)])
+@pytest.mark.parametrize("N,K", [(96, 6208), (97, 64), (200, 14404), (2048, 36), (161, 130), (2050, 130), (2081, 6212)])   # the last two are wide enough for tiles from 129 rows on, the others mostly blocks of 16
 def test_gemm_fp32_in_parts_around_tiles_and_rounds(ops, N, K):
     """Tiles of 128 rows of x by 64 or 96 of w, chunks of 64 k, rounds of 96 chunks, 16-byte copies and 4-byte ones: against 64-bit sums, and every row with the bits it has alone."""
     torch.manual_seed(53)

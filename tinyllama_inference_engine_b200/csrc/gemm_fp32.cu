@@ -11,7 +11,7 @@
 //     small is summed while the sum is small, and only four additions of a chunk are taken at full size;
 //   * the chunks' sums are added in order, in 32-bit, rounded to nearest.
 // A tcgen05.mma and an mma.sync m16n8k16 of the same 16 k give the same bits, and the place of a k among the 16 does not matter; so both kernels below keep to the definition:
-//   * up to 16 rows (decoding): bound by the weights' bytes; warps of a CTA take chunks of 16 rows of w in turn, straight from global memory to fragments (mma.sync);
+//   * up to 16 rows (decoding), and narrow products of up to 128: bound by the weights' bytes; warps of a CTA take chunks of 16 rows of w in turn, each lane the fragments it needs (mma.sync);
 //   * more rows: tiles of 128 rows of x by 64 or 96 rows of w on tcgen05, operands cut on their way into shared memory.  Bound by shared memory: at 96 rows of w a chunk of 64 k brings
 //     112 KB through it on the way to registers, 84 KB of parts, and 168 KB that its 24 products read: 2,850 clocks at 128 bytes each; measured 2,550.
 // Against 64-bit sums the error is a sixth to a seventh of what multiply-adds in order give (2-norms over normal numbers: K = 2,048 1.3e-7, 8.1e-7; K = 5,632 1.9e-7, 1.34e-6).
@@ -20,7 +20,7 @@
 //      1      10.9 ->  8.7     10.1 ->  6.3      23.4 ->  22.1     26.0 ->  12       52 ->  49
 //      4      13.6 ->  8.6     12.3 ->  6.5      26.6 ->  22.1     30.5 ->  12       61 ->  49
 //     16      32.5 -> 12.2     16.8 ->  7.6      65.4 ->  28.1     44.1 ->  16      156 ->  73
-//     24      51.4 -> 50.4     51.4 -> 46.7      90.1 ->  77.5      138 -> 110      157 -> 153
+//     24      51.4 -> 16.4     51.4 -> 12.0      90.1 ->  51       138 ->  28      157 -> 136
 //    150       125 ->  57       107 ->  47        244 -> 100        262 -> 118      541 -> 235
 //    760       233 ->  80       236 ->  46        902 -> 220        624 -> 112
 //  2,048       671 -> 134       460 -> 132       2,225 -> 571      1,232 -> 330
@@ -80,7 +80,7 @@ __device__ __noinline__ float sum_in_order(const float* __restrict__ x, const fl
 }
 __device__ __forceinline__ bool out_of_range(float v) { return !(fabsf(v) <= 3.402823466e38f) || (v != 0.0f && fabsf(v) < 1e-30f); }
 
-// --- up to 16 rows -----------------------------------------------------------------------------------
+// --- few rows ----------------------------------------------------------------------------------------
 constexpr int kFewRows = 16;        // rows of w of a CTA
 constexpr int kFewAhead = 2;        // chunks of w on their way to a warp
 constexpr int kFewRound = 96;       // chunks whose sums are in shared memory at a time
@@ -104,9 +104,10 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gem
   static_assert(kOutputs <= WARPS * 32, "a thread adds up one output");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int tiles = (N + kFewRows - 1) / kFewRows, chunks = (K + kChunkK - 1) / kChunkK;
+  const int m0 = blockIdx.y * 8 * NT;
   const float* x_rows[NT];
 #pragma unroll
-  for (int j = 0; j < NT; ++j) x_rows[j] = x + (long long)min(8 * j + g, M - 1) * lda;
+  for (int j = 0; j < NT; ++j) x_rows[j] = x + (long long)min(m0 + 8 * j + g, M - 1) * lda;
   // While the kernel before this one runs, L2 fetches the CTA's first chunks of weights.  Nothing is read: w may be what that kernel writes.
   for (int c = warp; c < chunks && c < 4 * WARPS; c += WARPS) {
     const int k = c * kChunkK + (lane & 1) * 32;
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gem
       }
       __syncthreads();
     }
-    const int m = threadIdx.x / kFewRows, n = n0 + threadIdx.x % kFewRows;
+    const int m = m0 + threadIdx.x / kFewRows, n = n0 + threadIdx.x % kFewRows;
     if (threadIdx.x < kOutputs && m < M && n < N) {
       if (out_of_range(total)) total = sum_in_order(x + (long long)m * lda, w + (long long)n * K, K);
       out[(size_t)m * N + n] = total;
@@ -226,11 +227,12 @@ static int launch_few(const float* x, const float* w, float* out, int M, int N, 
   const int chunks = (K + kChunkK - 1) / kChunkK, tiles = (N + kFewRows - 1) / kFewRows;
   constexpr int ring = WARPS * kFewAhead * kFewRows * kChunkK * (int)sizeof(float);
   const int smem = ring + (chunks < kFewRound ? chunks : kFewRound) * 8 * kFewRows * NT * (int)sizeof(float);
-  const int places = (NT == 1 && WARPS == 8 ? 2 : 1) * device_sm_count();
+  const int places = (NT == 1 && WARPS == 8 ? 2 : 1) * device_sm_count(), blocks = (M + 8 * NT - 1) / (8 * NT);
+  const int across = places / blocks > 1 ? places / blocks : 1;   // CTAs of a block of rows
   static std::atomic<unsigned long long> devices{0};
   const cudaError_t allowed = allow_shared_memory(gemm_few_f32_kernel<NT, WARPS, ALIGNED>, ring + kFewRound * 8 * kFewRows * NT * (int)sizeof(float), devices);
   if (allowed != cudaSuccess) return (int)allowed;
-  return (int)launch_pdl(gemm_few_f32_kernel<NT, WARPS, ALIGNED>, dim3(tiles < places ? tiles : places), dim3(WARPS * 32), smem, stream, x, w, out, M, N, K, lda);
+  return (int)launch_pdl(gemm_few_f32_kernel<NT, WARPS, ALIGNED>, dim3(tiles < across ? tiles : across, blocks), dim3(WARPS * 32), smem, stream, x, w, out, M, N, K, lda);
 }
 
 // --- more rows ---------------------------------------------------------------------------------------
@@ -490,9 +492,13 @@ static int launch_f32(const float* x, const float* w, float* out, int M, int N, 
     if ((N + kFewRows - 1) / kFewRows <= device_sm_count()) return launch_few<1, 16, ALIGNED>(x, w, out, M, N, K, lda, stream);
     return launch_few<1, 8, ALIGNED>(x, w, out, M, N, K, lda, stream);
   }
-  if (M <= 16) return launch_few<2, 8, ALIGNED>(x, w, out, M, N, K, lda, stream);
   const long long m_blocks = (M + kBM - 1) / kBM, sms = device_sm_count();
   const long long wide = (m_blocks * ((N + 95) / 96) + sms - 1) / sms, narrow = (m_blocks * ((N + 63) / 64) + sms - 1) / sms;   // waves
+  // The few-rows kernel takes 4.75 us per K = 2,048 and as many blocks of 16 x 16 outputs as there are SMs, the other one 36 to 50 per wave, whatever a wave holds, and up to 86 where
+  // a tile is mostly rows that repeat the last one (all in proportion to K).  So narrow products stay with the former up to 128 rows, wide ones up to 32: 2,048 x 2,048, 24 / 64 / 128 rows:
+  // 12 / 21 / 39 us against 47 / 41 / 39; 2,048 x 5,632, 24 / 64: 28 / 52 against 108 / 101; 11,264 x 2,048, 24 / 48: 51 / 74 against 78 / 73; 32,000 x 2,048, 24 / 48: 136 / 199 against 155 / 146.
+  const long long blocks = (long long)((M + 15) / 16) * ((N + kFewRows - 1) / kFewRows), places = sms * (wide * 9 <= narrow * 8 ? wide : narrow);
+  if (M <= 16 || 10 * blocks <= (M <= 32 ? 96 : 75) * places) return launch_few<2, 8, ALIGNED>(x, w, out, M, N, K, lda, stream);
   if (wide * 9 <= narrow * 8) return launch_many<96, ALIGNED>(x, w, out, M, N, K, lda, error_flag, stream);
   return launch_many<64, ALIGNED>(x, w, out, M, N, K, lda, error_flag, stream);
 }
