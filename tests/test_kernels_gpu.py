@@ -194,6 +194,51 @@ def test_gemm_fp32_of_numbers_whose_parts_fall_out_of_range(ops, M):
     assert bool(((got.double() - want.double()).abs() <= bound)[finite].all())
 
 
+TINY_AND_LARGE = [(1e3, 1e-33), (1e5, 1e-35), (1e8, 1e-36), (1e9, 2e-38), (1e20, 2e-41), (1e10, 1e-43)]
+
+
+@pytest.mark.parametrize("K", [64, 130])
+@pytest.mark.parametrize("M", [4, 12, 300])
+@pytest.mark.parametrize("sx,sw", TINY_AND_LARGE + [pair[::-1] for pair in TINY_AND_LARGE])
+def test_gemm_fp32_of_tiny_numbers_times_large_ones(ops, sx, sw, M, K):
+    """Results far above the smallest number whose terms have an operand near it or below (of which three bfloat16 parts hold few bits or none)."""
+    torch.manual_seed(55)
+    N = 2050
+    x, w = (torch.randn(M, K, dtype=torch.float64) * sx).float().cuda(), (torch.randn(N, K, dtype=torch.float64) * sw).float().cuda()
+    x[1], w[5] = 0.0, 0.0
+    exact = x.double() @ w.double().T
+    got = torch.full((M, N), float("nan"), device="cuda")
+    ops.linear(x, w, got)
+    # a sum of K terms in order, one rounding of at most 2^-24 per step of what has grown with the root of the step, is off by 2^-24 sqrt(K / 2) at most (2-norms)
+    assert float((got.double() - exact).norm() / exact.norm()) <= 2.0 ** -24 * (K / 2) ** 0.5
+    assert bool((got[1] == 0).all()) and bool((got[:, 5] == 0).all())
+
+
+@pytest.mark.parametrize("M", [4, 12, 300])
+def test_gemm_fp32_gives_a_row_its_bits_beside_rows_of_tiny_numbers(ops, M):
+    """Whether an output is worked out again is a matter of its own two rows: neighbours in its tile change nothing, nor do other rows of its product."""
+    torch.manual_seed(56)
+    N, K = 2050, 260
+    x, w = torch.randn(M, K).cuda(), torch.randn(N, K).cuda()
+    plain = torch.empty(M, N, device="cuda")
+    ops.linear(x, w, plain)
+    w[::3] *= 1e-37
+    w[1, 7] = 1e-41   # a normal row with one number that its parts do not hold: lost in what its sums round off
+    x[3] *= 1e-30
+    got = torch.empty(M, N, device="cuda")
+    ops.linear(x, w, got)
+    kept = [m for m in range(M) if m != 3]
+    columns = [n for n in range(N) if n % 3 and n != 1]
+    assert torch.equal(got[kept][:, columns], plain[kept][:, columns])
+    alone = torch.empty(1, N, device="cuda")
+    for m in (0, 2, 3, M - 1):
+        ops.linear(x[m : m + 1], w, alone)
+        assert torch.equal(alone[0], got[m]), m
+    exact = x.double() @ w.double().T
+    bound = K * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) + K * 2.0 ** -149
+    assert bool(((got.double() - exact).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("M", [1, 2, 4, 8, 16, 40])
 def test_gemm_fp32_takes_a_weight_that_the_kernel_before_it_writes(ops, M):
     """A product whose weight is the result of the product before it (which lets its successor start early), over and over on the same buffer."""

@@ -2,7 +2,7 @@
 //
 // The reference's 32-bit model computes each output as one dot product over K in index order (src/model.cpp:53-78).  The FP32 pipes are bound by what shared memory
 // delivers to them (45 of 72 TFLOP/s at 2,048 rows) and a sum over k in order by the chain of its multiply-adds.  Here every number is cut into three bfloat16 parts,
-// v = high + middle + low, each the rounded rest of the ones before it: 24 bits, nothing lost.  The product of two such numbers is the sum of nine products of parts;
+// v = high + middle + low, each the rounded rest of the ones before it: 24 bits, nothing lost where v is not tiny (see the end).  The product of two such numbers is the sum of nine products of parts;
 // the three that are below 2^-24 of it are left out, the other six are tensor-core products with 32-bit sums.
 //
 // The order of a sum is a definition, the same for every output whatever M, N, the kernel and the tile:
@@ -24,8 +24,10 @@
 //    150       125 ->  57       107 ->  47        244 -> 100        262 -> 118      541 -> 235
 //    760       233 ->  80       236 ->  46        902 -> 220        624 -> 112
 //  2,048       671 -> 134       460 -> 132       2,225 -> 571      1,232 -> 330
-// Parts of an infinity are not finite, and of numbers below 2^-110 they fall out of range: an output that comes out not finite, or nonzero below 1e-30, is
-// worked out again as one sum of multiply-adds over k in order, by the thread that holds it, whichever kernel that is.
+// What the parts cannot hold is worked out again as one sum of multiply-adds over k in order.  Parts of an infinity, and of numbers that round to one, are not finite: nor is such an output.
+// Parts of numbers below 2^-102 (their last bits), and products of parts where the operands' product is below 2^-98, leave the range of normal numbers; what a term loses then is at
+// most 2^-124 of the largest operand, or 2^-123.  So an output is also worked out again where its rows of x and w hold such numbers (other than zeros) and it is below
+// K * 2^-98 * max(1, largest operand), 2^25 times what it may have lost.  Both are properties of the output and its two rows, whatever kernel and tile it is in.
 #include "shared_memory_limit.cuh"
 #define TLIE_WITHOUT_TENSOR_MAPS
 #include "tcgen05_utils.cuh"
@@ -72,13 +74,91 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// What the parts cannot hold (see above), worked out again.
+// --- what the parts cannot hold (see above) -----------------------------------------------------------
+constexpr float kLargest = 3.402823466e38f;
+// What a sum of K terms has to reach if nothing that may have left the range of normal numbers is to matter to it; most: the largest magnitude among its operands.
+__device__ __forceinline__ float safe_from(float most, int K) { return (float)K * 3.1554436e-30f * fmaxf(1.0f, most); }   // 2^-98
+
+// A CTA has to tell at little cost whether one of its outputs may need it: it keeps sums of squares of what it cuts, a packed multiply-add a pair (2 to 5 % of a product; smallest magnitudes
+// took 10 to 15, largest ones 7 to 15).  While they are below 2^100, no operand is above 2^50 and every output from safe_from(2^50) on stands.
+__device__ __forceinline__ void keep_squares(unsigned long long& squares, float a, float b) {
+  unsigned long long both;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(both) : "f"(a), "f"(b));
+  asm("fma.rn.f32x2 %0, %1, %1, %0;\n" : "+l"(squares) : "l"(both));
+}
+__device__ __forceinline__ bool squares_are_large(unsigned long long squares) {
+  float a, b;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(a), "=f"(b) : "l"(squares));
+  return !(a < 1.2676506e30f && b < 1.2676506e30f);   // (NaN among them)
+}
+__device__ __forceinline__ bool stands(float v, int K) { return fabsf(v) >= safe_from(1.1258999e15f, K) && fabsf(v) <= kLargest; }
+
+struct RowRange {
+  uint32_t least;   // bits of the smallest magnitude but zero, times two, less one (2^32 - 1: all zeros)
+  uint32_t most;    // bits of the largest magnitude
+};
+// Of a row of K, by a warp.
+template <bool ALIGNED>
+__device__ __forceinline__ RowRange row_range(const float* row, int K) {
+  uint32_t least = 0xffffffffu, most = 0;
+#pragma unroll 4
+  for (int k = (threadIdx.x & 31) * 4; k < K; k += 128) {
+    const float4 v = ALIGNED ? __ldcg(reinterpret_cast<const float4*>(row + k))
+                             : make_float4(__ldcg(row + k), k + 1 < K ? __ldcg(row + k + 1) : 0.0f, k + 2 < K ? __ldcg(row + k + 2) : 0.0f, k + 3 < K ? __ldcg(row + k + 3) : 0.0f);
+    const uint32_t a = __float_as_uint(v.x) * 2, b = __float_as_uint(v.y) * 2, c = __float_as_uint(v.z) * 2, d = __float_as_uint(v.w) * 2;
+    least = min(min(least, min(a - 1, b - 1)), min(c - 1, d - 1));
+    most = max(max(most, max(a, b)), max(c, d));
+  }
+  return {__reduce_min_sync(0xffffffffu, least), __reduce_max_sync(0xffffffffu, most) / 2};
+}
+// Of an output and the ranges of its two rows.
+__device__ __forceinline__ bool work_out_again(float v, RowRange x, RowRange w, int K) {
+  if (!(fabsf(v) <= kLargest)) return true;
+  if (x.most == 0 || w.most == 0 || !(fabsf(v) < safe_from(fmaxf(__uint_as_float(x.most), __uint_as_float(w.most)), K))) return false;
+  const int a = (int)((x.least + 1) >> 24), b = (int)((w.least + 1) >> 24);   // exponents, 127 too large
+  return a < 127 - 102 || b < 127 - 102 || a + b < 2 * 127 - 98;
+}
+
 __device__ __noinline__ float sum_in_order(const float* __restrict__ x, const float* __restrict__ w, int K) {
   float sum = 0.0f;
   for (int k = 0; k < K; ++k) sum = fmaf(x[k], w[k], sum);
   return sum;
 }
-__device__ __forceinline__ bool out_of_range(float v) { return !(fabsf(v) <= 3.402823466e38f) || (v != 0.0f && fabsf(v) < 1e-30f); }
+
+template <int BARRIER, int THREADS>
+__device__ __forceinline__ void barrier_of() { asm volatile("bar.sync %0, %1;\n" ::"n"(BARRIER), "n"(THREADS) : "memory"); }
+
+// A tile of a product, as what is rarely needed finds it in shared memory.  (With the kernel's own parameters used there, registers held them through the loops: 760 rows, 2,048 x 2,048
+// 46.4 -> 48.9 us.)
+struct Tile {
+  const float *x, *w;
+  float* out;
+  long long lda;
+  int M, N, K, m0, n0;
+};
+
+// Outputs of a tile that are not sure to stand, decided and stored by THREADS threads from FIRST on, which have a barrier of their own.  values: [BM][BN + 1], as they were summed; behind
+// them room for the rows' ranges.  They come from warps of 32 rows and COLUMNS columns; bit row / 32 + 4 (column / COLUMNS) of `unsure` stands for theirs (the other warps have stored theirs).
+template <int BM, int BN, int COLUMNS, int FIRST, int THREADS, int BARRIER, bool ALIGNED>
+__device__ __noinline__ void store_unsure(const Tile* tile, const float* values, uint32_t unsure) {
+  const Tile t = *tile;
+  RowRange* ranges = reinterpret_cast<RowRange*>(const_cast<float*>(values) + BM * (BN + 1));   // rows of x, rows of w
+  const int thread = (int)threadIdx.x - FIRST;
+  for (int r = thread / 32; r < BM + BN; r += THREADS / 32) {
+    const RowRange found = row_range<ALIGNED>(r < BM ? t.x + min(t.m0 + r, t.M - 1) * t.lda : t.w + (long long)min(t.n0 + r - BM, t.N - 1) * t.K, t.K);
+    if ((thread & 31) == 0) ranges[r] = found;
+  }
+  barrier_of<BARRIER, THREADS>();
+  for (int i = thread; i < BM * BN; i += THREADS) {
+    const int row = i / BN, column = i % BN, m = t.m0 + row, n = t.n0 + column;
+    if (m >= t.M || n >= t.N || !(unsure >> (row / 32 + 4 * (column / COLUMNS)) & 1)) continue;
+    float v = values[row * (BN + 1) + column];
+    if (work_out_again(v, ranges[row], ranges[BM + column], t.K)) v = sum_in_order(t.x + m * t.lda, t.w + (long long)n * t.K, t.K);
+    t.out[(size_t)m * t.N + n] = v;
+  }
+  __syncwarp();
+  barrier_of<BARRIER, THREADS>();
+}
 
 // --- few rows ----------------------------------------------------------------------------------------
 constexpr int kFewRows = 16;        // rows of w of a CTA
@@ -151,9 +231,11 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gem
   for (int s = 0; s < kFewAhead; ++s) ask(s);
   if (warp < chunks) load_x(warp);
   int slot = 0;
+  unsigned long long squares = 0;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int n0 = tile * kFewRows;
     float total = 0.0f;
+    bool unsure = false;
     for (int first = 0; first < chunks; first += kFewRound) {
       const int here = min(kFewRound, chunks - first);
       for (int c = first + warp; c < first + here; c += WARPS) {
@@ -174,11 +256,15 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gem
           uint32_t wm[4], wl[4], xm[NT][2], xl[NT][2];
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
+            keep_squares(squares, wv[r][s].x, wv[r][s].y);
+            keep_squares(squares, wv[r][s].z, wv[r][s].w);
             cut_pair(wv[r][s].x, wv[r][s].y, wh[s][r], wm[r], wl[r]);
             cut_pair(wv[r][s].z, wv[r][s].w, wh[s][r + 2], wm[r + 2], wl[r + 2]);
           }
 #pragma unroll
           for (int j = 0; j < NT; ++j) {
+            keep_squares(squares, xv[j][s].x, xv[j][s].y);
+            keep_squares(squares, xv[j][s].z, xv[j][s].w);
             cut_pair(xv[j][s].x, xv[j][s].y, xh[j][s][0], xm[j][0], xl[j][0]);
             cut_pair(xv[j][s].z, xv[j][s].w, xh[j][s][1], xm[j][1], xl[j][1]);
           }
@@ -211,13 +297,26 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gem
 #pragma unroll 8
         for (int c = 0; c < here; ++c) total += sums[c * kOutputs + threadIdx.x];
       }
-      __syncthreads();
+      unsure = __syncthreads_or(squares_are_large(squares) || (threadIdx.x < kOutputs && !stands(total, K)));   // (of the last round, all of K)
     }
     const int m = m0 + threadIdx.x / kFewRows, n = n0 + threadIdx.x % kFewRows;
-    if (threadIdx.x < kOutputs && m < M && n < N) {
-      if (out_of_range(total)) total = sum_in_order(x + (long long)m * lda, w + (long long)n * K, K);
-      out[(size_t)m * N + n] = total;
+    if (!unsure) {
+      if (threadIdx.x < kOutputs && m < M && n < N) out[(size_t)m * N + n] = total;
+      continue;
     }
+    cp_async_wait<0>();   // the ring is put to another use; what was on its way is asked for again
+    __syncthreads();
+    Tile* here = reinterpret_cast<Tile*>(ring);
+    float* values = ring + sizeof(Tile) / sizeof(float);
+    if (threadIdx.x == 0) *here = {x, w, out, lda, M, N, K, m0, n0};
+    if (threadIdx.x < kOutputs) values[threadIdx.x / kFewRows * (kFewRows + 1) + threadIdx.x % kFewRows] = total;
+    __syncthreads();
+    store_unsure<8 * NT, kFewRows, kFewRows, 0, WARPS * 32, 0, ALIGNED>(here, values, 1);
+    ask_tile = warp < chunks ? tile + (int)gridDim.x : tiles;
+    ask_chunk = warp;
+    slot = 0;
+#pragma unroll 1
+    for (int s = 0; s < kFewAhead; ++s) ask(s);
   }
   cp_async_wait<0>();
 }
@@ -304,6 +403,9 @@ __global__ void __launch_bounds__(kManyThreads, 1) gemm_many_f32_kernel(const fl
   uint64_t* taken = summed + 2;             // [2]: its sum has been read
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(taken + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
+  uint32_t* unsure = tmem_holder + 2;       // a bit per adding warp whose outputs are not stored yet
+  uint32_t* large = tmem_holder + 3;        // not 0: an operand may be above 2^50
+  Tile* this_tile = reinterpret_cast<Tile*>(tmem_holder + 4);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int m_blocks = (M + kBM - 1) / kBM;
   const int m0 = ((int)blockIdx.x % m_blocks) * kBM, n0 = ((int)blockIdx.x / m_blocks) * BN;   // neighbours share their weights
@@ -319,6 +421,8 @@ __global__ void __launch_bounds__(kManyThreads, 1) gemm_many_f32_kernel(const fl
       mbar_init(&taken[a], kAddWarps);
     }
     *abort_flag = 0;
+    *unsure = *large = 0;
+    *this_tile = {x, w, out, lda, M, N, K, m0, n0};
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == kCutWarps) {
@@ -333,6 +437,7 @@ __global__ void __launch_bounds__(kManyThreads, 1) gemm_many_f32_kernel(const fl
   grid_dependency_wait();
 
   if (warp < kCutWarps) {
+    unsigned long long squares = 0;
     // A thread's float4 i: row (thread / 16) + 16 i of the tile (x rows, then w rows), k 4 (thread % 16) of the chunk.  Rows past M or N repeat the last one.
     const int first_row = threadIdx.x / 16, k_of = (threadIdx.x % 16) * 4;
     // Each is copied to a place of its own thread's and read there by that thread; as soon as it has been read, the same place is asked to take the next chunk's, which
@@ -388,6 +493,8 @@ __global__ void __launch_bounds__(kManyThreads, 1) gemm_many_f32_kernel(const fl
           const int row = g * kBatch + i;
           const bool of_x = row < kXFours;
           uint2 high, middle, low;
+          keep_squares(squares, v[i].x, v[i].y);
+          keep_squares(squares, v[i].z, v[i].w);
           cut_pair(v[i].x, v[i].y, high.x, middle.x, low.x);
           cut_pair(v[i].z, v[i].w, high.y, middle.y, low.y);
           uint8_t* at = stage + (of_x ? row * 2048 : 3 * Shape::kPlaneX + (row - kXFours) * 2048);
@@ -402,6 +509,9 @@ __global__ void __launch_bounds__(kManyThreads, 1) gemm_many_f32_kernel(const fl
       if (lane == 0) mbar_arrive(&full[s]);
     }
     cp_async_wait<0>();
+    if (squares_are_large(squares)) atomicOr(large, 1u);
+    __syncwarp();
+    asm volatile("bar.arrive 1, %0;\n" ::"n"((kCutWarps + kAddWarps) * 32) : "memory");   // (of the word above, to the adding warps)
   } else if (warp == kCutWarps) {
     const uint32_t issue = elect_one();
     constexpr uint32_t idesc = umma_instr_desc(kBM, BN);
@@ -452,15 +562,22 @@ __global__ void __launch_bounds__(kManyThreads, 1) gemm_many_f32_kernel(const fl
         for (int j = 32; j < Shape::kColumns; ++j) total[j] += __uint_as_float(rest[j - 32]);
       }
     }
-    const int m = m0 + sub * 32 + lane, first = n0 + half * Shape::kColumns;
-    if (ok && m < M) {
+    __syncwarp();
+    asm volatile("bar.sync 1, %0;\n" ::"n"((kCutWarps + kAddWarps) * 32) : "memory");
+    const int row = sub * 32 + lane, m = m0 + row, first = n0 + half * Shape::kColumns;
+    bool sure = *reinterpret_cast<volatile uint32_t*>(large) == 0;
+#pragma unroll
+    for (int i = 0; i < Shape::kColumns; ++i) sure = sure && stands(total[i], K);
+    if (!__all_sync(0xffffffffu, sure)) {
+      float* values = reinterpret_cast<float*>(ring) + row * (BN + 1) + half * Shape::kColumns;   // every product is done with the stages
+#pragma unroll
+      for (int i = 0; i < Shape::kColumns; ++i) values[i] = total[i];
+      if (lane == 0) atomicOr(unsure, 1u << (sub + 4 * half));
+    } else if (ok && m < M) {
       float* dst = out + (size_t)m * N + first;
       const bool wide = N % 4 == 0 && ((uintptr_t)out & 15) == 0;
 #pragma unroll
       for (int i = 0; i < Shape::kColumns; i += 4) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (first + i + j < N && out_of_range(total[i + j])) total[i + j] = sum_in_order(x + (long long)m * lda, w + (long long)(first + i + j) * K, K);
         if (wide && first + i < N) {
           *reinterpret_cast<float4*>(dst + i) = make_float4(total[i], total[i + 1], total[i + 2], total[i + 3]);
         } else {
@@ -470,6 +587,10 @@ __global__ void __launch_bounds__(kManyThreads, 1) gemm_many_f32_kernel(const fl
         }
       }
     }
+    __syncwarp();
+    barrier_of<1, kAddWarps * 32>();
+    if (*reinterpret_cast<volatile uint32_t*>(unsure) != 0 && *abort_flag == 0)
+      store_unsure<kBM, BN, Shape::kColumns, (kCutWarps + 1) * 32, kAddWarps * 32, 1, ALIGNED>(this_tile, reinterpret_cast<float*>(ring), *unsure);
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   }
   if (*abort_flag && threadIdx.x == 0 && error_flag != nullptr) atomicOr(error_flag, 1);
