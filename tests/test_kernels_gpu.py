@@ -214,6 +214,24 @@ def test_gemm_fp32_of_tiny_numbers_times_large_ones(ops, sx, sw, M, K):
     assert bool((got[1] == 0).all()) and bool((got[:, 5] == 0).all())
 
 
+@pytest.mark.parametrize("M", [1, 17, 300])
+@pytest.mark.parametrize("K", [1, 2, 3, 4, 5, 6])
+def test_gemm_fp32_of_a_few_terms_is_their_sum_in_order(ops, K, M):
+    """A single product is the rounded one, and every multiply-add after it rounds once: the bits of a sum in order."""
+    torch.manual_seed(57)
+    N = 2050
+    x, w = torch.randn(M, K), torch.randn(N, K)
+    want = torch.zeros(M, N, dtype=torch.float64)
+    ties = torch.zeros(M, N, dtype=torch.bool)   # where the 64-bit sum is itself rounded, a tie of 32-bit numbers may fall on the other side
+    for k in range(K):
+        step = want + x[:, k].double()[:, None] * w[:, k].double()[None, :]
+        ties |= (step.float().double() - step).abs() == (torch.nextafter(step.float(), torch.where(step.float().double() < step, 1.0, -1.0) * float("inf")).double() - step).abs()
+        want = step.float().double()
+    got = torch.empty(M, N, device="cuda")
+    ops.linear(x.cuda(), w.cuda(), got)
+    assert int(ties.sum()) <= 4 and torch.equal(got.cpu()[~ties], want.float()[~ties])
+
+
 @pytest.mark.parametrize("M", [4, 12, 300])
 def test_gemm_fp32_gives_a_row_its_bits_beside_rows_of_tiny_numbers(ops, M):
     """Whether an output is worked out again is a matter of its own two rows: neighbours in its tile change nothing, nor do other rows of its product."""

@@ -12,6 +12,7 @@
 //   * the chunks' sums are added in order, in 32-bit, rounded to nearest.
 // A tcgen05.mma and an mma.sync m16n8k16 of the same 16 k give the same bits, and the place of a k among the 16 does not matter; so both kernels below keep to the definition:
 //   * up to 16 rows (decoding), and narrow products of up to 128: bound by the weights' bytes; warps of a CTA take chunks of 16 rows of w in turn, each lane the fragments it needs (mma.sync);
+//   * sums of up to six terms: multiply-adds in order, a thread an output;
 //   * more rows: tiles of 128 rows of x by 64 or 96 rows of w on tcgen05, operands cut on their way into shared memory.  Bound by shared memory: at 96 rows of w a chunk of 64 k brings
 //     112 KB through it on the way to registers, 84 KB of parts, and 168 KB that its 24 products read: 2,850 clocks at 128 bytes each; measured 2,550.
 // Against 64-bit sums the error is a sixth to a seventh of what multiply-adds in order give (2-norms over normal numbers: K = 2,048 1.3e-7, 8.1e-7; K = 5,632 1.9e-7, 1.34e-6).
@@ -624,6 +625,17 @@ static int launch_f32(const float* x, const float* w, float* out, int M, int N, 
   return launch_many<64, ALIGNED>(x, w, out, M, N, K, lda, error_flag, stream);
 }
 
+// --- short sums --------------------------------------------------------------------------------------
+// Six terms and fewer, in order: the parts' products that are left out, and what the tensor core cuts off, are more than the roundings of so few multiply-adds (error against 64 bits, 2-norms,
+// at 1 / 2 / 4 / 5 terms: 2.5, 3.1, 4.0, 4.3e-8; by parts 4.6e-8 at any of them.  From seven on the parts are ahead: 5.1 and 4.8, at 16 terms 7.4 and 4.8).  A thread an output: 32 columns, 8 rows.
+constexpr int kShortK = 6;
+
+__global__ void __launch_bounds__(256) gemm_short_f32_kernel(const float* x, const float* w, float* out, int M, int N, int K, long long lda) {
+  const int across = (N + 31) / 32;
+  const int m = (int)(blockIdx.x / across) * 8 + (int)threadIdx.x / 32, n = (int)(blockIdx.x % across) * 32 + (int)threadIdx.x % 32;
+  if (m < M && n < N) out[(size_t)m * N + n] = sum_in_order(x + m * lda, w + (long long)n * K, K);
+}
+
 }  // namespace tlie
 
 using namespace tlie;
@@ -632,6 +644,10 @@ using namespace tlie;
 TLIE_EXPORT int tlie_gemm_nt_f32_reporting(const float* x, const float* w, float* out, int M, int N, int K, long long lda, int* error_flag, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || lda < K) return (int)cudaErrorInvalidValue;
+  if (K <= kShortK) {
+    gemm_short_f32_kernel<<<(unsigned)((long long)((M + 7) / 8) * ((N + 31) / 32)), 256, 0, stream>>>(x, w, out, M, N, K, lda);
+    return (int)cudaGetLastError();
+  }
   if (K % 4 == 0 && lda % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0)
     return launch_f32<true>(x, w, out, M, N, K, lda, error_flag, stream);
   return launch_f32<false>(x, w, out, M, N, K, lda, error_flag, stream);
