@@ -194,6 +194,63 @@ def test_gemm_fp32_of_numbers_whose_parts_fall_out_of_range(ops, M):
     assert bool(((got.double() - want.double()).abs() <= bound)[finite].all())
 
 
+@pytest.mark.parametrize("M", [4, 12, 300])
+@pytest.mark.parametrize("K", [131, 132, 1000])
+def test_gemm_fp32_beside_infinities_and_nan(ops, M, K):
+    """Rows of x and of w with an infinity, a NaN, zeros or large numbers, in the few-rows kernel and in tiles: their outputs are sums in order, all others have the bits they have without them."""
+    torch.manual_seed(58)
+    N = 2050
+    x, w = torch.randn(M, K), torch.randn(N, K)
+    plain = torch.empty(M, N, device="cuda")
+    ops.linear(x.cuda(), w.cuda(), plain)
+    special = {"inf": (0, 3), "nan": (1, 100), "zero": (2, 1030), "large": (M - 1, 2049)}
+    for kind, (m, n) in special.items():
+        for row in (x[m], w[n]):
+            if kind == "zero":
+                row.zero_()
+            elif kind == "large":
+                row *= 1e17
+            else:
+                row[K // 2 + (n & 1)] = float(kind)
+    got = torch.full((M, N), -1.0, device="cuda")
+    ops.linear(x.cuda(), w.cuda(), got)
+    got, plain = got.cpu(), plain.cpu()
+    rows, columns = [m for m, _ in special.values()], [n for _, n in special.values()]
+    others_m, others_n = [m for m in range(M) if m not in rows], [n for n in range(N) if n not in columns]
+    assert torch.equal(got[others_m][:, others_n], plain[others_m][:, others_n])
+    exact = x.double() @ w.double().T
+    want = torch.zeros(M, N)
+    for k in range(K):
+        want = (want.double() + x[:, k].double()[:, None] * w[:, k].double()[None, :]).float()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[want.isinf()], want[want.isinf()]) and bool((got[2] == 0)[~want[2].isnan()].all())
+    bound = K * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    assert bool(((got.double() - exact).abs() <= bound)[want.isfinite()].all())
+    assert int(ops.error_flag(torch.device("cuda", 0))) == 0, "a bounded wait inside the kernel gave up"
+
+
+def test_gemm_fp32_with_a_nan_takes_a_few_times_as_long_at_most(ops):
+    """A NaN settles its outputs and an infinity's are summed by the whole tile (2.4 and 6 times the product's time, measured; one thread for a row of a tile's outputs took 80 times)."""
+    torch.manual_seed(59)
+    x, w, out = torch.randn(760, 2048).cuda(), torch.randn(2048, 2048).cuda(), torch.empty(760, 2048, device="cuda")
+
+    def fastest():
+        times = []
+        for _ in range(6):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            for _ in range(4):
+                ops.linear(x, w, out)
+            end.record()
+            torch.cuda.synchronize()
+            times.append(start.elapsed_time(end))
+        return min(times)
+
+    without = fastest()
+    for value in (float("nan"), float("inf")):
+        x[5, 7] = value
+        assert fastest() < 20 * without, value
+
+
 TINY_AND_LARGE = [(1e3, 1e-33), (1e5, 1e-35), (1e8, 1e-36), (1e9, 2e-38), (1e20, 2e-41), (1e10, 1e-43)]
 
 
