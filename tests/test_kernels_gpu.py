@@ -334,6 +334,26 @@ def test_gemm_fp32_takes_a_weight_that_the_kernel_before_it_writes(ops, M):
         assert torch.equal(out, want)
 
 
+@pytest.mark.parametrize("M,K", [(1, 2048), (4, 2048), (16, 2048), (40, 2048), (400, 2048), (4, 2046), (400, 2046)])
+def test_gemm_fp32_takes_activations_that_the_kernel_before_it_writes(ops, M, K):
+    """The same with x, the result of the product before it: every chunk of it has to be what was written last, whatever an earlier product on the same buffer left in a cache."""
+    torch.manual_seed(60)
+    N = 1100
+    a, b, w = torch.randn(3, M, 256).cuda(), torch.randn(K, 256).cuda(), torch.randn(N, K).cuda()
+    x, out = torch.zeros(M, K, device="cuda"), torch.zeros(3, M, N, device="cuda")
+    want = torch.zeros_like(out)
+    for i in range(3):
+        ops.linear(a[i], b, x)
+        torch.cuda.synchronize()
+        ops.linear(x, w, want[i])
+        torch.cuda.synchronize()
+    for _ in range(5):
+        for i in range(3):
+            ops.linear(a[i], b, x)
+            ops.linear(x, w, out[i])
+        assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 256, 64), (37, 136, 80), (130, 72, 520), (64, 2048, 2048)])
 def test_linear_bf16(ops, M, N, K):
     torch.manual_seed(4)

@@ -1,0 +1,46 @@
+"""What holds for a kernel by the way it is launched and ended, checked without a device: on the sources, and on the launchers compiled against a stand-in for the CUDA runtime."""
+from __future__ import annotations
+
+import ctypes
+import re
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+from test_second_device import CSRC, FAKE_RUNTIME
+
+
+@pytest.fixture(scope="module")
+def products(tmp_path_factory):
+    """gemm_fp32.cu's launchers; the stand-in counts the launches that may start before the kernel in front of them has ended."""
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not Path(nvcc).exists():
+        pytest.skip("no nvcc")
+    folder = tmp_path_factory.mktemp("launch_rules")
+    launch = "cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* config, const void* kernel, void**) {"
+    assert launch in FAKE_RUNTIME
+    runtime = FAKE_RUNTIME.replace(launch, "static int early = 0;\nint fake_early_launches() { return early; }\n" + launch + " early += config->numAttrs;")
+    (folder / "runtime.cpp").write_text(runtime)
+    library = folder / "products.so"
+    subprocess.run([nvcc, "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-cudart", "none", "-Xlinker", "-Bsymbolic", "-gencode", "arch=compute_100a,code=sm_100a", "-Xptxas", "-O0",
+                    "-I", str(CSRC), "-o", str(library), str(CSRC / "gemm_fp32.cu"), str(folder / "runtime.cpp")], check=True)
+    return ctypes.CDLL(str(library))
+
+
+@pytest.mark.parametrize("M", [1, 12, 40, 300])
+def test_32_bit_products_that_read_through_l1_do_not_start_early(products, M, monkeypatch):
+    """Operands that are not 16-byte aligned take 4-byte asynchronous copies, which exist through L1 only; a line of it may be older than what the kernel in front writes."""
+    monkeypatch.delenv("TLIE_PDL", raising=False)
+    for N in (100, 2050):
+        for address, K, lda, early in ((1 << 20, 2048, 2048, 1), (1 << 20, 2048, 2052, 1), ((1 << 20) + 4, 2048, 2048, 0), (1 << 20, 2047, 2048, 0), (1 << 20, 2048, 2049, 0), (1 << 20, 5, 5, 0)):
+            memory, before, launches = ctypes.c_void_p(address), products.fake_early_launches(), products.fake_launches()
+            assert products.tlie_gemm_nt_f32(memory, memory, memory, M, N, K, ctypes.c_longlong(lda), None) == 0
+            assert (products.fake_early_launches() - before, products.fake_launches() - launches) == (early, 1), (N, address, K, lda)
+
+
+def test_32_bit_products_read_operands_by_ordinary_loads():
+    """Their kernels start while the one in front may still write x or w: no read-only path, nor C++ loads of pointers to constants, which the compiler may send there."""
+    source = (CSRC / "gemm_fp32.cu").read_text()
+    kernels = source[source.index("load_four("):source.index("gemm_short_f32_kernel")]   # (that one is launched behind the kernel in front of it)
+    assert not re.search(r"__ldg\(|ld\.global\.nc|\bx_rows\[\w+\]\[|\brow\[k|\bx\[|\bw\[", kernels)
