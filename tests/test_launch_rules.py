@@ -44,3 +44,25 @@ def test_32_bit_products_read_operands_by_ordinary_loads():
     source = (CSRC / "gemm_fp32.cu").read_text()
     kernels = source[source.index("load_four("):source.index("gemm_short_f32_kernel")]   # (that one is launched behind the kernel in front of it)
     assert not re.search(r"__ldg\(|ld\.global\.nc|\bx_rows\[\w+\]\[|\brow\[k|\bx\[|\bw\[", kernels)
+
+
+WAITING = sorted(path.name for path in CSRC.glob("*.cu") if "abort_flag" in path.read_text())
+
+
+def test_the_kernels_with_bounded_waits_are_known():
+    assert WAITING == ["attention_prefill_tc.cu", "gemm_fp32.cu", "gemm_skinny.cu", "gemm_tcgen05.cu", "gemm_tcgen05_pair.cu", "moe_grouped_tc.cu"]
+
+
+@pytest.mark.parametrize("name", WAITING)
+def test_a_wait_that_gives_up_is_reported_whichever_thread_it_is(name):
+    """The report reads the CTA's flag behind the barrier that every wait has ended at; in front of it, the reporting thread may be done before another thread's wait gives up."""
+    shared = (CSRC / "tcgen05_utils.cuh").read_text()
+    closing = shared[shared.index("void close_and_report("):]
+    closing = closing[:closing.index("\n}\n")]
+    assert closing.index("__syncthreads();") < closing.index("if (*abort_flag)") < closing.index("atomicOr(error_flag, 1)") < closing.index("__nanosleep")
+    source = (CSRC / name).read_text()
+    assert "if (*abort_flag" not in source   # nobody reports by itself
+    for kernel in re.split(r"(?=__global__ )", source)[1:]:
+        if "mbar_wait(" in kernel:
+            end = kernel.index("close_and_report(abort_flag,")
+            assert "mbar_wait(" not in kernel[end:] and kernel.index("tcgen05.dealloc", end) > end   # tensor memory is given back behind it

@@ -726,11 +726,7 @@ __global__ void __launch_bounds__(kThreadsTC, 2)
     TL_END(0)
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   }
-  if (*abort_flag) {
-    if (threadIdx.x == 0) atomicOr(error_flag, 1);
-    for (int i = 0; i < 2000; ++i) __nanosleep(1000);   // copies that were issued may still be landing
-  }
-  __syncthreads();
+  close_and_report(abort_flag, error_flag);
   if (warp == 1) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kTmemCols));
   }

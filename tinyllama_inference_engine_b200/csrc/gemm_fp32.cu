@@ -720,8 +720,7 @@ __global__ void __launch_bounds__(kManyThreads, 1) gemm_many_f32_kernel(const fl
       store_unsure<kBM, BN, Shape::kColumns, 32, (kCutWarps + 1) * 32, kAddWarps * 32, 1, ALIGNED>(this_tile, reinterpret_cast<float*>(ring), *unsure, *large != 0);
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   }
-  if (*abort_flag && threadIdx.x == 0 && error_flag != nullptr) atomicOr(error_flag, 1);
-  __syncthreads();
+  close_and_report(abort_flag, error_flag);
   if (warp == kCutWarps) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kTmemCols));
 }
 

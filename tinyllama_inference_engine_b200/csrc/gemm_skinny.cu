@@ -386,12 +386,8 @@ __global__ void __launch_bounds__(kSkinnyThreads)
     }
   }
   if (threadIdx.x == 64) stamp(8);
-  if (*abort_flag) {
-    if (threadIdx.x == 0) atomicOr(a.error_flag, 1);
-    for (int i = 0; i < 2000; ++i) __nanosleep(1000);   // copies in flight may still land in this CTA's shared memory
-  }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-  __syncthreads();
+  close_and_report(abort_flag, a.error_flag);
   if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kBN));
   if (threadIdx.x == 64) stamp(9);
 }

@@ -192,12 +192,7 @@ __global__ void __launch_bounds__(kGemmThreads)
     if (lane == 0) bulk_wait_all();   // this warp's staging boxes have been read and written out
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   }
-  if (*abort_flag) {
-    if (threadIdx.x == 0) atomicOr(error_flag, 1);
-    // copies that were issued may still be landing in this CTA's shared memory: give them time before it is released
-    for (int i = 0; i < 2000; ++i) __nanosleep(1000);
-  }
-  __syncthreads();
+  close_and_report(abort_flag, error_flag);
   if (warp == 2) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols));
   }

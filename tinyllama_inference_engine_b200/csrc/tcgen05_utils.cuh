@@ -53,6 +53,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 }
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) { return mbar_wait(smem_u32(bar), parity, abort_flag); }
 
+// How a kernel with such waits ends: the barrier that closes it, and only behind that a look at whether a wait gave up (before it, a thread that is done early would miss one that gives up
+// later).  Copies and MMAs that were issued may still be on their way to and from what the CTA gives back, so it waits for them for two milliseconds then.
+__device__ __forceinline__ void close_and_report(volatile int* abort_flag, int* error_flag) {
+  __syncthreads();
+  if (*abort_flag) {
+    if (threadIdx.x == 0 && error_flag != nullptr) atomicOr(error_flag, 1);
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+  }
+}
+
 // Position in a ring of STAGES buffers: the stage and the phase bit of its barriers, advanced without a division.
 template <int STAGES>
 struct RingPosition {
