@@ -251,6 +251,35 @@ def test_gemm_fp32_with_a_nan_takes_a_few_times_as_long_at_most(ops):
         assert fastest() < 20 * without, value
 
 
+@pytest.mark.parametrize("K", [7, 63, 64, 65, 128, 130, 192, 200, 256, 260])
+def test_gemm_fp32_of_short_rows(ops, K):
+    """Warps take chunks of several tiles at a time where a row has one to four of them (and one tile at a time above): the bits of the tiles of 128 rows, also beside outputs that are worked out again."""
+    torch.manual_seed(61)
+    N = 11290   # more tiles of 16 than CTAs, the last of them and the last group of tiles not full
+    x, w = torch.randn(300, K).cuda(), torch.randn(N, K).cuda()
+    exact = x.double() @ w.double().T
+    full = torch.empty(300, N, device="cuda")
+    ops.linear(x, w, full)
+    assert bool(((full.double() - exact).abs() <= K * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)).all())
+    again = w.clone()
+    again[40], again[4800], again[11288] = float("nan"), again[4800] * 1e-37, float("inf")
+    worked = torch.empty(300, N, device="cuda")
+    ops.linear(x, again, worked)
+    plain = torch.ones(N, dtype=torch.bool)
+    plain[[40, 4800, 11288]] = False
+    assert torch.equal(worked[:, plain], full[:, plain])
+    for M in (1, 5, 8, 9, 16, 24, 40):
+        for weight, want in ((w, full), (again, worked)):
+            got = torch.full((M, N), float("nan"), device="cuda")
+            ops.linear(x[11 : 11 + M], weight, got)
+            assert torch.equal(got.view(torch.int32), want[11 : 11 + M].view(torch.int32)), M
+    wide = torch.randn(8, K + 1).cuda()
+    wide[:, :K] = x[:8]
+    got = torch.empty(8, N, device="cuda")
+    ops.linear(wide[:, :K], w, got)   # 4-byte copies
+    assert torch.equal(got, full[:8])
+
+
 TINY_AND_LARGE = [(1e3, 1e-33), (1e5, 1e-35), (1e8, 1e-36), (1e9, 2e-38), (1e20, 2e-41), (1e10, 1e-43)]
 
 

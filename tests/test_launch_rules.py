@@ -20,7 +20,8 @@ def products(tmp_path_factory):
     folder = tmp_path_factory.mktemp("launch_rules")
     launch = "cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* config, const void* kernel, void**) {"
     assert launch in FAKE_RUNTIME
-    runtime = FAKE_RUNTIME.replace(launch, "static int early = 0;\nint fake_early_launches() { return early; }\n" + launch + " early += config->numAttrs;")
+    runtime = FAKE_RUNTIME.replace(launch, "static int early = 0;\nstatic dim3 grid, block;\nint fake_early_launches() { return early; }\nint fake_threads() { return block.x; }\n" + launch
+                                   + " early += config->numAttrs; grid = config->gridDim; block = config->blockDim; if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidConfiguration;")
     (folder / "runtime.cpp").write_text(runtime)
     library = folder / "products.so"
     subprocess.run([nvcc, "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-cudart", "none", "-Xlinker", "-Bsymbolic", "-gencode", "arch=compute_100a,code=sm_100a", "-Xptxas", "-O0",

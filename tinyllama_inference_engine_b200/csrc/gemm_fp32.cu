@@ -1,4 +1,4 @@
-// 32-bit matrix product for the float32 path: out[M, N] = x[M, K] . w[N, K]^T (rows of x ``lda`` elements apart), on the tensor cores without loss of precision.
+// 32-bit matrix product for the float32 path: out[M, N] = x[M, K] . w[N, K]^T (rows of x ``lda`` elements apart), on the tensor cores, each number in three bfloat16 parts.
 //
 // The reference's 32-bit model computes each output as one dot product over K in index order (src/model.cpp:53-78).  The FP32 pipes are bound by what shared memory
 // delivers to them (45 of 72 TFLOP/s at 2,048 rows) and a sum over k in order by the chain of its multiply-adds.  Here every number is cut into three bfloat16 parts,
@@ -18,13 +18,13 @@
 // Against 64-bit sums the error is a sixth to a seventh of what multiply-adds in order give (2-norms over normal numbers: K = 2,048 1.3e-7, 8.1e-7; K = 5,632 1.9e-7, 1.34e-6).
 // Back to back in a graph, weights from HBM, the register kernels before -> these, in us:
 //   rows      2,560 x 2,048    2,048 x 2,048    11,264 x 2,048    2,048 x 5,632    32,000 x 2,048
-//      1      10.9 ->  8.7     10.1 ->  6.3      23.4 ->  22.1     26.0 ->  12       52 ->  49
-//      4      13.6 ->  8.6     12.3 ->  6.5      26.6 ->  22.1     30.5 ->  12       61 ->  49
-//     16      32.5 -> 12.2     16.8 ->  7.6      65.4 ->  28.1     44.1 ->  16      156 ->  73
-//     24      51.4 -> 16.4     51.4 -> 12.0      90.1 ->  51       138 ->  28      157 -> 136
-//    150       125 ->  57       107 ->  47        244 -> 100        262 -> 118      541 -> 235
-//    760       233 ->  80       236 ->  46        902 -> 220        624 -> 112
-//  2,048       671 -> 134       460 -> 132       2,225 -> 571      1,232 -> 330
+//      1      10.9 ->  8.7     10.0 ->  6.3      23.3 ->  21.7     25.9 -> 12.4      49 ->  48
+//      4      13.8 ->  9.1     10.4 ->  6.5      25.9 ->  21.8     31.6 -> 12.6      57 ->  48
+//     16      32.4 -> 12.6     17.7 ->  7.7      64.9 ->  27.3     43.8 -> 16.2     155 ->  71
+//     24      51.6 -> 16.8     51.3 -> 12.2       129 ->  50       139 ->  28       244 -> 135
+//    150       130 ->  54       116 ->  44        252 -> 100       321 -> 110       538 -> 241
+//    760       233 ->  88       236 ->  47        902 -> 236       627 -> 124
+//  2,048       673 -> 143       461 -> 137      2,224 -> 671     1,234 -> 355
 // What the parts cannot hold is worked out again as one sum of multiply-adds over k in order.  Parts of an infinity, and of numbers that round to one, are not finite: nor is such an output.
 // Parts of numbers below 2^-102 (their last bits), and products of parts where the operands' product is below 2^-98, leave the range of normal numbers; what a term loses then is at
 // most 2^-124 of the largest operand, or 2^-123.  So an output is also worked out again where its rows of x and w hold such numbers (other than zeros) and it is below
@@ -293,8 +293,9 @@ __device__ __forceinline__ void mma_16x8x16(float (&c)[4], const uint32_t (&a)[4
 // NT: blocks of 8 rows of x.  A lane (g = lane / 4, t = lane % 4) holds rows g and g + 8 of w and row g of every block of x, k 4 t ... 4 t + 3 of every 16.
 // WARPS: sixteen where a CTA has its SM to itself, eight where two share one.  A lane copies what it will read itself (w of two chunks ahead, whichever tile they belong to), so a warp's
 // ring needs no barrier, and an SM has 128 KB on its way from HBM (with the next chunk on its way to registers it was half of that: 11,264 x 2,048 24.5 us, 2,048 x 5,632 13).
-// A CTA walks row tiles blockIdx.x, + gridDim.x, ...
-template <int NT, int WARPS, bool ALIGNED>
+// A CTA walks row tiles blockIdx.x, + gridDim.x, ...  SHORT: a row has so few chunks that the warps take those of `together` tiles at a time (one tile after the other,
+// one to four warps of eight worked: K = 64, 16 rows x 11,264 5.6 -> 4.2 us, 128 x 2,048 8.2 -> 4.7, 600 x 256 6.4 -> 4.1).
+template <int NT, int WARPS, bool ALIGNED, bool SHORT>
 __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gemm_few_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ out,
                                                                                                 int M, int N, int K, long long lda) {
   extern __shared__ __align__(16) float ring[];   // [warp][kFewAhead][8][lane] float4, then the sums
@@ -315,7 +316,11 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gem
   grid_launch_dependents();
   grid_dependency_wait();
   float4* const mine = reinterpret_cast<float4*>(ring) + warp * kFewAhead * 8 * 32 + lane;
-  int ask_tile = warp < chunks ? (int)blockIdx.x : tiles, ask_chunk = warp;
+  const int together = SHORT ? WARPS / chunks : 1, stride = together * (int)gridDim.x;
+  const int own_chunk = SHORT ? warp % chunks : warp;                       // a warp's first chunk of a tile
+  const int own_tile = SHORT ? warp / chunks * (int)gridDim.x : 0;          // and of which tile, from the CTA's first
+  const bool works = SHORT ? warp / chunks < together : warp < chunks;
+  int ask_tile = works ? (int)blockIdx.x + own_tile : tiles, ask_chunk = own_chunk;
   auto ask = [&](int slot) {   // w of the next chunk in this warp's order; a group each (an empty one behind the last keeps the count)
     if (ask_tile < tiles) {
       const int n = ask_tile * kFewRows + g;
@@ -335,7 +340,7 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gem
         }
       }
       ask_chunk += WARPS;
-      if (ask_chunk >= chunks) ask_chunk = warp, ask_tile += gridDim.x;
+      if (ask_chunk >= chunks) ask_chunk = own_chunk, ask_tile += stride;
     }
     cp_async_commit();
   };
@@ -348,16 +353,16 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gem
   };
 #pragma unroll
   for (int s = 0; s < kFewAhead; ++s) ask(s);
-  if (warp < chunks) load_x(warp);
+  if (works) load_x(own_chunk);
   int slot = 0;
   unsigned long long squares = 0;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    const int n0 = tile * kFewRows;
+  for (int first_tile = blockIdx.x; first_tile < tiles; first_tile += stride) {
     float total = 0.0f;
     bool unsure = false;
     for (int first = 0; first < chunks; first += kFewRound) {
       const int here = min(kFewRound, chunks - first);
-      for (int c = first + warp; c < first + here; c += WARPS) {
+      const int end = SHORT ? (works && first_tile + own_tile < tiles ? warp + 1 : 0) : first + here;   // (SHORT: one chunk a warp, its sums in the warp's place)
+      for (int c = first + warp; c < end; c += WARPS) {
         float acc[NT][4];
         uint32_t wh[4][4], xh[NT][4][2];
         cp_async_wait<kFewAhead - 1>();
@@ -396,7 +401,7 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gem
             mma_16x8x16(acc[j], wm, xh[j][s]);
           }
         }
-        load_x(c + WARPS < chunks ? c + WARPS : warp);   // of the next chunk, or of the next tile's first one
+        if (!SHORT) load_x(c + WARPS < chunks ? c + WARPS : own_chunk);   // of the next chunk, or of the next tile's first one
 #pragma unroll
         for (int s = 0; s < 4; ++s)
 #pragma unroll
@@ -412,30 +417,40 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gem
         }
       }
       __syncthreads();
+      if (SHORT) break;
       if (threadIdx.x < kOutputs) {
 #pragma unroll 8
         for (int c = 0; c < here; ++c) total += sums[c * kOutputs + threadIdx.x];
       }
       unsure = __syncthreads_or(squares_are_large(squares) || (threadIdx.x < kOutputs && !stands(total, K)));   // (of the last round, all of K)
     }
-    const int m = m0 + threadIdx.x / kFewRows, n = n0 + threadIdx.x % kFewRows;
-    if (!unsure) {
-      if (threadIdx.x < kOutputs && m < M && n < N) out[(size_t)m * N + n] = total;
-      continue;
-    }
-    cp_async_wait<0>();   // the ring is put to another use; what was on its way is asked for again
-    const bool large = __syncthreads_or(squares_are_large(squares));
-    Tile* here = reinterpret_cast<Tile*>(ring);
-    float* values = ring + sizeof(Tile) / sizeof(float);
-    if (threadIdx.x == 0) *here = {x, w, out, lda, M, N, K, m0, n0};
-    if (threadIdx.x < kOutputs) values[threadIdx.x / kFewRows * (kFewRows + 1) + threadIdx.x % kFewRows] = total;
-    __syncthreads();
-    store_unsure<8 * NT, kFewRows, kFewRows, 128, 0, WARPS * 32, 0, ALIGNED>(here, values, 1, large);
-    ask_tile = warp < chunks ? tile + (int)gridDim.x : tiles;
-    ask_chunk = warp;
-    slot = 0;
+    for (int part = 0; part < together && first_tile + part * (int)gridDim.x < tiles; ++part) {
+      const int tile = first_tile + part * (int)gridDim.x, n0 = tile * kFewRows;
+      if (SHORT) {
+        total = 0.0f;
+        if (threadIdx.x < kOutputs)
+          for (int c = 0; c < chunks; ++c) total += sums[(part * chunks + c) * kOutputs + threadIdx.x];
+        unsure = __syncthreads_or(squares_are_large(squares) || (threadIdx.x < kOutputs && !stands(total, K)));
+      }
+      const int m = m0 + threadIdx.x / kFewRows, n = n0 + threadIdx.x % kFewRows;
+      if (!unsure) {
+        if (threadIdx.x < kOutputs && m < M && n < N) out[(size_t)m * N + n] = total;
+        continue;
+      }
+      cp_async_wait<0>();   // the ring is put to another use; what was on its way is asked for again
+      const bool large = __syncthreads_or(squares_are_large(squares));
+      Tile* here = reinterpret_cast<Tile*>(ring);
+      float* values = ring + sizeof(Tile) / sizeof(float);
+      if (threadIdx.x == 0) *here = {x, w, out, lda, M, N, K, m0, n0};
+      if (threadIdx.x < kOutputs) values[threadIdx.x / kFewRows * (kFewRows + 1) + threadIdx.x % kFewRows] = total;
+      __syncthreads();
+      store_unsure<8 * NT, kFewRows, kFewRows, 128, 0, WARPS * 32, 0, ALIGNED>(here, values, 1, large);
+      ask_tile = works ? first_tile + own_tile + stride : tiles;
+      ask_chunk = own_chunk;
+      slot = 0;
 #pragma unroll 1
-    for (int s = 0; s < kFewAhead; ++s) ask(s);
+      for (int s = 0; s < kFewAhead; ++s) ask(s);
+    }
   }
   cp_async_wait<0>();
 }
@@ -448,17 +463,28 @@ static int launch_product(Kernel* kernel, dim3 grid, int threads, int smem, cuda
   return (int)cudaGetLastError();
 }
 
-template <int NT, int WARPS, bool ALIGNED>
+// CTAs of a block of rows, and tiles that a CTA's eight warps take at a time.
+static long long few_across(long long places, long long blocks, long long tiles) {
+  const long long across = places / blocks > 1 ? places / blocks : 1;
+  return tiles < across ? tiles : across;
+}
+static int few_together(int K, long long tiles, long long across) {
+  const int chunks = (K + kChunkK - 1) / kChunkK;
+  return 2 * chunks <= 8 && tiles > across ? 8 / chunks : 1;
+}
+
+template <int NT, int WARPS, bool ALIGNED, bool SHORT = false>
 static int launch_few(const float* x, const float* w, float* out, int M, int N, int K, long long lda, cudaStream_t stream) {
   const int chunks = (K + kChunkK - 1) / kChunkK, tiles = (N + kFewRows - 1) / kFewRows;
-  constexpr int ring = WARPS * kFewAhead * kFewRows * kChunkK * (int)sizeof(float);
-  const int smem = ring + (chunks < kFewRound ? chunks : kFewRound) * 8 * kFewRows * NT * (int)sizeof(float);
   const int places = (NT == 1 && WARPS == 8 ? 2 : 1) * device_sm_count(), blocks = (M + 8 * NT - 1) / (8 * NT);
-  const int across = places / blocks > 1 ? places / blocks : 1;   // CTAs of a block of rows
+  const int across = (int)few_across(places, blocks, tiles);
+  if (!SHORT && WARPS == 8 && few_together(K, tiles, across) > 1) return launch_few<NT, WARPS, ALIGNED, WARPS == 8>(x, w, out, M, N, K, lda, stream);
+  constexpr int ring = WARPS * kFewAhead * kFewRows * kChunkK * (int)sizeof(float), chunk_sums = 8 * kFewRows * NT * (int)sizeof(float);
+  const int smem = ring + (SHORT ? WARPS : chunks < kFewRound ? chunks : kFewRound) * chunk_sums;
   static std::atomic<unsigned long long> devices{0};
-  const cudaError_t allowed = allow_shared_memory(gemm_few_f32_kernel<NT, WARPS, ALIGNED>, ring + kFewRound * 8 * kFewRows * NT * (int)sizeof(float), devices);
+  const cudaError_t allowed = allow_shared_memory(gemm_few_f32_kernel<NT, WARPS, ALIGNED, SHORT>, ring + (SHORT ? WARPS : kFewRound) * chunk_sums, devices);
   if (allowed != cudaSuccess) return (int)allowed;
-  return launch_product<ALIGNED>(gemm_few_f32_kernel<NT, WARPS, ALIGNED>, dim3(tiles < across ? tiles : across, blocks), WARPS * 32, smem, stream, x, w, out, M, N, K, lda);
+  return launch_product<ALIGNED>(gemm_few_f32_kernel<NT, WARPS, ALIGNED, SHORT>, dim3(across, blocks), WARPS * 32, smem, stream, x, w, out, M, N, K, lda);
 }
 
 // --- more rows ---------------------------------------------------------------------------------------
