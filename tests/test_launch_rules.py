@@ -40,6 +40,15 @@ def test_32_bit_products_that_read_through_l1_do_not_start_early(products, M, mo
             assert (products.fake_early_launches() - before, products.fake_launches() - launches) == (early, 1), (N, address, K, lda)
 
 
+@pytest.mark.parametrize("M,N,K,few", [(17, 1, 64, True), (24, 2048, 2048, True), (64, 5632, 2048, True), (96, 2048, 2048, True), (200, 2048, 2048, False), (600, 97, 2048, True),
+                                       (1280, 208, 2048, False), (24, 32000, 2048, True), (48, 11264, 2048, False), (150, 2048, 5632, False), (400, 256, 64, True), (760, 2048, 5632, False), (3000000, 1, 64, False)])
+def test_32_bit_products_take_the_kernel_that_is_cheaper(products, M, N, K, few):
+    """Blocks of 16 rows (CTAs of 256 threads) or tiles of 128: measured, one of them 1.1 to 8 times as fast; and never more blocks than a grid's second dimension has."""
+    memory = ctypes.c_void_p(1 << 20)
+    assert products.tlie_gemm_nt_f32(memory, memory, memory, M, N, K, ctypes.c_longlong(K), None) == 0
+    assert products.fake_threads() == (256 if few else 544)
+
+
 def test_32_bit_products_read_operands_by_ordinary_loads():
     """Their kernels start while the one in front may still write x or w: no read-only path, nor C++ loads of pointers to constants, which the compiler may send there."""
     source = (CSRC / "gemm_fp32.cu").read_text()

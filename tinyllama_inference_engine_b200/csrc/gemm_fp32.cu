@@ -11,10 +11,12 @@
 //     small is summed while the sum is small, and only four additions of a chunk are taken at full size;
 //   * the chunks' sums are added in order, in 32-bit, rounded to nearest.
 // A tcgen05.mma and an mma.sync m16n8k16 of the same 16 k give the same bits, and the place of a k among the 16 does not matter; so both kernels below keep to the definition:
-//   * up to 16 rows (decoding), and narrow products of up to 128: bound by the weights' bytes; warps of a CTA take chunks of 16 rows of w in turn, each lane the fragments it needs (mma.sync);
-//   * sums of up to six terms: multiply-adds in order, a thread an output;
-//   * more rows: tiles of 128 rows of x by 64 or 96 rows of w on tcgen05, operands cut on their way into shared memory.  Bound by shared memory: at 96 rows of w a chunk of 64 k brings
-//     112 KB through it on the way to registers, 84 KB of parts, and 168 KB that its 24 products read: 2,850 clocks at 128 bytes each; measured 2,550.
+//   * up to 16 rows (decoding), and more where that is cheaper (see `cheapest`): bound by the weights' bytes; warps of a CTA take chunks of 16 rows of w in turn, each lane the fragments it
+//     needs (mma.sync);
+//   * more rows: tiles of 128 rows of x by 64 or 96 rows of w on tcgen05, operands cut on their way into shared memory.  A chunk of 64 k takes 2,550 clocks at 96 rows of w, its 24 products
+//     1,150 of them.  Every number goes through shared memory raw (112 KB a chunk in and out), in parts (84 KB) and as operands (168 KB); ncu has the tensor pipe busy 37 % of the time, shared
+//     memory's wavefronts of loads, stores and copies 52 %, issue slots 39 %;
+//   * sums of up to six terms: multiply-adds in order, a thread an output.
 // Against 64-bit sums the error is a sixth to a seventh of what multiply-adds in order give (2-norms over normal numbers: K = 2,048 1.3e-7, 8.1e-7; K = 5,632 1.9e-7, 1.34e-6).
 // Back to back in a graph, weights from HBM, the register kernels before -> these, in us:
 //   rows      2,560 x 2,048    2,048 x 2,048    11,264 x 2,048    2,048 x 5,632    32,000 x 2,048
@@ -759,21 +761,38 @@ static int launch_many(const float* x, const float* w, float* out, int M, int N,
   return launch_product<ALIGNED>(gemm_many_f32_kernel<BN, ALIGNED>, dim3((unsigned)tiles), kManyThreads, ManyShape<BN>::kSmem, stream, x, w, out, M, N, K, lda, error_flag);
 }
 
+// What a product of more than 16 rows takes, in us, by the schedule that each kernel has for it.  Fitted to 1,411 products of 17 to 4,096 rows, N from 1 to 11,264 and K from 64 to 5,632, weights
+// in L2: the choice is 0.25 % slower than the best of the three in the geometric mean, and more than 10 % slower at 10 of them.
+//   * blocks of 16 rows: CTAs walk tiles of 16 columns (or as many as fit their warps, see SHORT), 5 us each at K = 2,048;
+//   * tiles of 128 x 96 and 128 x 64: waves of 46 and 39 us at K = 2,048, up to twice that where rows of a tile repeat the last one (2,048 columns of 24 / 64 / 128 rows: 47 / 40 / 38; 11,264
+//     columns of 24 rows 79, of 128 46).
+enum Kernels { FEW, TILES_OF_96, TILES_OF_64 };
+static Kernels cheapest(int M, int N, int K) {
+  auto up = [](long long a, long long b) { return (a + b - 1) / b; };
+  const long long sms = device_sm_count(), blocks = up(M, 16), columns = up(N, kFewRows), across = few_across(sms, blocks, columns);
+  const int together = few_together(K, columns, across);
+  const long long steps = up(blocks * across, sms) * up(up(columns, across), together);
+  const float few = 0.5f + (float)steps * (0.5f + 0.0022f * (float)K + (together > 1 ? 0.3f * (float)together : 0.0f));
+  const long long m_blocks = up(M, kBM);
+  const float share = (float)(m_blocks * kBM - M) / (float)(m_blocks * kBM), repeated = 1.0f + 1.1f * share * sqrtf(share);
+  const float wide = (float)up(m_blocks * up(N, 96), sms) * (5.5f + 0.02f * (float)K) * repeated;
+  const float narrow = (float)up(m_blocks * up(N, 64), sms) * (4.5f + 0.0168f * (float)K) * repeated;
+  if (few <= fminf(wide, narrow) && blocks <= 65535) return FEW;   // (blocks are the grid's second dimension)
+  return wide <= narrow ? TILES_OF_96 : TILES_OF_64;
+}
+
 template <bool ALIGNED>
 static int launch_f32(const float* x, const float* w, float* out, int M, int N, int K, long long lda, int* error_flag, cudaStream_t stream) {
   if (M <= 8) {
     if ((N + kFewRows - 1) / kFewRows <= device_sm_count()) return launch_few<1, 16, ALIGNED>(x, w, out, M, N, K, lda, stream);
     return launch_few<1, 8, ALIGNED>(x, w, out, M, N, K, lda, stream);
   }
-  const long long m_blocks = (M + kBM - 1) / kBM, sms = device_sm_count();
-  const long long wide = (m_blocks * ((N + 95) / 96) + sms - 1) / sms, narrow = (m_blocks * ((N + 63) / 64) + sms - 1) / sms;   // waves
-  // The few-rows kernel takes 4.75 us per K = 2,048 and as many blocks of 16 x 16 outputs as there are SMs, the other one 36 to 50 per wave, whatever a wave holds, and up to 86 where
-  // a tile is mostly rows that repeat the last one (all in proportion to K).  So narrow products stay with the former up to 128 rows, wide ones up to 32: 2,048 x 2,048, 24 / 64 / 128 rows:
-  // 12 / 21 / 39 us against 47 / 41 / 39; 2,048 x 5,632, 24 / 64: 28 / 52 against 108 / 101; 11,264 x 2,048, 24 / 48: 51 / 74 against 78 / 73; 32,000 x 2,048, 24 / 48: 136 / 199 against 155 / 146.
-  const long long blocks = (long long)((M + 15) / 16) * ((N + kFewRows - 1) / kFewRows), places = sms * (wide * 9 <= narrow * 8 ? wide : narrow);
-  if (M <= 16 || 10 * blocks <= (M <= 32 ? 96 : 75) * places) return launch_few<2, 8, ALIGNED>(x, w, out, M, N, K, lda, stream);
-  if (wide * 9 <= narrow * 8) return launch_many<96, ALIGNED>(x, w, out, M, N, K, lda, error_flag, stream);
-  return launch_many<64, ALIGNED>(x, w, out, M, N, K, lda, error_flag, stream);
+  if (M <= 16) return launch_few<2, 8, ALIGNED>(x, w, out, M, N, K, lda, stream);
+  switch (cheapest(M, N, K)) {
+    case FEW: return launch_few<2, 8, ALIGNED>(x, w, out, M, N, K, lda, stream);
+    case TILES_OF_96: return launch_many<96, ALIGNED>(x, w, out, M, N, K, lda, error_flag, stream);
+    default: return launch_many<64, ALIGNED>(x, w, out, M, N, K, lda, error_flag, stream);
+  }
 }
 
 // --- short sums --------------------------------------------------------------------------------------
