@@ -46,7 +46,7 @@ struct GemvArgs {
   // gate_limit): g * sigmoid(gate_alpha * g) * (u + gate_shift).
   int gate_kind;
   float gate_limit, gate_alpha, gate_shift;
-  int ahead_bytes;          // what a CTA asks L2 for before it waits for the kernel before it, beyond its first round
+  int ahead;                // 1: a CTA asks L2 for what follows its first round before it waits for the kernel before it
 };
 
 __device__ __forceinline__ float gemv_activate(int kind, float z, float a, float b) {
@@ -246,25 +246,20 @@ struct GemvPhase {
     }
   }
 
-  // Asks L2 for what this CTA reads after its first round: the rest of its first tile, then its next tiles, as far as a.ahead_bytes go, so that HBM works on while the CTA waits for the
-  // kernel before it (the registers hold one round).  Sixteen threads, a row of the tile each.
+  // Asks L2 for what this CTA reads after its first round, so that HBM works on while the CTA waits for the kernel before it (the registers hold one round): the rest of its first tile, or its next
+  // tile where the round holds all of that; 4 KB a row of the tile at most (64 KB a CTA, 19 MB over two CTAs of every SM).  Sixteen threads, a row each.
   __device__ __forceinline__ void ask_ahead(const GemvArgs& a, int first_tile, int tile_step) {
-    if (threadIdx.x >= 16) return;
+    if (threadIdx.x >= 16 || a.ahead == 0) return;
     const int n_rows = (EPI == EPI_GATED) ? a.N / 2 : a.N;
     const int tiles = (n_rows + kTileRows - 1) / kTileRows;
     const int r = threadIdx.x;
-    int left = a.ahead_bytes;
-    int from = WARPS * UNROLL * 32;   // columns of the first round
-    for (int tile = first_tile; tile < tiles && left > 0; tile += tile_step, from = 0) {
-      if (from >= a.K) continue;
-      const int n = tile * kTileRows + (EPI == EPI_GATED ? r & 7 : r);
-      const unsigned bytes = (unsigned)(a.K - from) * 2;
-      if (n < n_rows) {
-        const __nv_bfloat16* row = a.w + (size_t)(EPI == EPI_GATED && r >= 8 ? n_rows + n : n) * a.K + from;
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(row), "r"(bytes) : "memory");
-      }
-      left -= 16 * (int)bytes;
-    }
+    constexpr int kRound = WARPS * UNROLL * 32;   // columns of the first round
+    const int tile = kRound < a.K ? first_tile : first_tile + tile_step, from = kRound < a.K ? kRound : 0;
+    const int n = tile * kTileRows + (EPI == EPI_GATED ? r & 7 : r);
+    if (tile >= tiles || n >= n_rows) return;
+    const unsigned bytes = (unsigned)min(a.K - from, 2048) * 2;
+    const __nv_bfloat16* row = a.w + (size_t)(EPI == EPI_GATED && r >= 8 ? n_rows + n : n) * a.K + from;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(row), "r"(bytes) : "memory");
   }
 
   __device__ __forceinline__ void stage_x(const GemvArgs& a, __nv_bfloat16* xs, float* row_scale) { gemv_stage_x<MT, XMODE, 8, WARPS>(a, xs, row_scale); }

@@ -49,16 +49,14 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_fused_kernel(const GemvArgs a
   phase.run(a, xs, red, row_scale, blockIdx.x, gridDim.x, true);
 }
 
-constexpr int kGemvAheadBytes = 8 << 20;   // all CTAs together
-
 template <int MT, int XMODE, int EPI, int WARPS = kGemvWarps>
 static int launch_one(GemvArgs a, int grid, cudaStream_t stream) {
-  // Where asking ahead pays (us a decode step, nothing asked for -> 8 MB, 1.1B widths at 3 / 4 / 6 / 8 / 12 / 16 rows): 679 -> 654, 684 -> 660, 691 -> 675, 702 -> 677, 875 -> 872,
-  // 912 -> 910; 7B widths (8 layers) at 4 / 8: 736 -> 729, 814 -> 807; 8B widths at 4: 922 -> 914.  4 and 16 MB do the same.  Only where the operand's norm comes prepared and in the sixteen-warp adding product of
+  // Where asking ahead pays (us a decode step, without -> with it, 1.1B widths at 3 / 4 / 6 / 8 / 12 / 16 rows): 679 -> 654, 684 -> 660, 691 -> 675, 702 -> 677, 875 -> 872,
+  // 912 -> 910; 7B widths (8 layers) at 4 / 8: 736 -> 729, 814 -> 807; 8B widths at 4: 922 -> 914.  Only where the operand's norm comes prepared and in the sixteen-warp adding product of
   // three rows and more whose rest is less than its first round: with one or two rows (the norm worked out in every CTA) the step grew (650 -> 671), and the adding
   // products of longer rows lost at every width (8B widths, 4 rows: 922 -> 933).
   const bool pays = EPI == EPI_ACCUM ? WARPS == 16 && a.M > 2 && a.K < 2 * WARPS * GemvPhase<MT, XMODE, EPI, WARPS>::UNROLL * 32 : XMODE == X_PREPARED;
-  a.ahead_bytes = pays ? kGemvAheadBytes / grid : 0;
+  a.ahead = pays ? 1 : 0;
   const size_t smem = GemvPhase<MT, XMODE, EPI, WARPS>::smem_bytes(a.x_stride);
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
   static size_t configured = 0;
