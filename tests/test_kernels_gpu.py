@@ -127,9 +127,60 @@ def test_gemm_fp32_is_true_32_bit(ops, M, N, K):
     assert torch.equal(alone[0], got[M - 1])
 
 
+def _error(got, x, w) -> float:
+    """Against 64-bit sums, 2-norms."""
+    exact = x.double() @ w.double().T
+    return float((got.double() - exact).norm() / exact.norm())
+
+
+def _parts_limit(K: int) -> float:
+    """Chunks of 64 k are added in order, one rounding of at most 2^-24 each of a sum that grows with the root of their number, and 2^-24 for what happens inside a chunk.  (Measured: 0.75e-7 at one
+    chunk, 1.3e-7 at 32, 1.9e-7 at 88.  A sum of multiply-adds in order is off by 8.1e-7 at K = 2,048, parts without middle times middle by about 3e-6, bfloat16 operands by 2e-3.)"""
+    return 2.0 ** -24 * ((-(-K // 64) / 2) ** 0.5 + 1)
+
+
+@pytest.mark.parametrize("M,N", [(1, 2048), (8, 5000), (16, 2048), (64, 2048), (256, 2048), (600, 3000)])
+@pytest.mark.parametrize("K", [64, 512, 2048, 5632])
+def test_gemm_fp32_is_nearer_to_64_bits_than_a_sum_in_order(ops, M, N, K):
+    """Blocks of 8 and 16 rows, tiles of 128 x 64 and of 128 x 96."""
+    torch.manual_seed(62)
+    x, w = torch.randn(M, K).cuda(), torch.randn(N, K).cuda()
+    got = torch.empty(M, N, device="cuda")
+    ops.linear(x, w, got)
+    assert _error(got, x, w) <= _parts_limit(K)
+
+
+@pytest.mark.parametrize("K", [130, 260, 2048])
+@pytest.mark.parametrize("kind", ["spread", "cancelling", "sparse"])
+def test_gemm_fp32_gives_uneven_terms_the_same_bits_in_every_kernel(ops, kind, K):
+    """Blocks of rows run on mma.sync and tiles on tcgen05.  Terms over 2^-60 to 2^60, terms that cancel but for their last bits, and rows of mostly zeros, where an order of sums shows."""
+    torch.manual_seed(63)
+    M, N = 300, 2050
+    x, w = torch.randn(M, K), torch.randn(N, K)
+    if kind == "spread":
+        x *= 2.0 ** torch.randint(-30, 31, (M, K))
+        w *= 2.0 ** torch.randint(-30, 31, (N, K))
+    elif kind == "cancelling":
+        half = K // 2
+        order = torch.randperm(half)
+        x[:, half : 2 * half], w[:, half : 2 * half] = -x[:, order] * (1 + 2.0 ** -20), w[:, order]
+    else:
+        x *= torch.rand(M, K) < 0.1
+        w *= torch.rand(N, K) < 0.3
+    x, w = x.cuda(), w.cuda()
+    full = torch.empty(M, N, device="cuda")
+    ops.linear(x, w, full)
+    bound = K * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    assert bool(((full.double() - x.double() @ w.double().T).abs() <= bound).all())
+    for first, rows in ((0, 1), (5, 8), (17, 16), (100, 16), (250, 40), (284, 16)):
+        got = torch.empty(rows, N, device="cuda")
+        ops.linear(x[first : first + rows], w, got)
+        assert torch.equal(got, full[first : first + rows]), (first, rows)
+
+
 @pytest.mark.parametrize("N,K", [(64, 128), (130, 516), (2049, 260), (16, 4)])
 def test_gemm_fp32_gives_a_row_the_same_bits_in_every_kernel(ops, N, K):
-    """The streaming kernels (1, 2, 4, 8, 16 rows), the three register tiles and the plain one (an unaligned operand) around their edges."""
+    """Blocks of 8 and 16 rows, tiles of 128 rows and, with an operand that is not 16-byte aligned, their forms with 4-byte copies; four terms: the kernel of short sums."""
     torch.manual_seed(33)
     x, w = torch.randn(900, K).cuda(), torch.randn(N, K).cuda()
     full = torch.empty(900, N, device="cuda")
@@ -137,11 +188,12 @@ def test_gemm_fp32_gives_a_row_the_same_bits_in_every_kernel(ops, N, K):
     # one rounding per multiply-add of a sum of K terms
     bound = K * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
     assert bool(((full.double() - x.double() @ w.double().T).abs() <= bound).all())
+    assert _error(full, x, w) <= _parts_limit(K)
     for M in (1, 2, 3, 4, 5, 8, 9, 16, 17, 31, 33, 64, 65, 129, 300):
         got = torch.full((M, N), float("nan"), device="cuda")
         ops.linear(x[7 : 7 + M], w, got)
         assert torch.equal(got, full[7 : 7 + M]), M
-    wide = torch.randn(40, K + 1).cuda()   # rows one element apart from 16-byte alignment: the plain kernel
+    wide = torch.randn(40, K + 1).cuda()   # rows one element apart from 16-byte alignment: 4-byte copies
     wide[:, :K] = x[:40]
     got = torch.empty(40, N, device="cuda")
     ops.linear(wide[:, :K], w, got)
@@ -158,7 +210,7 @@ def test_gemm_fp32_in_parts_around_tiles_and_rounds(ops, N, K):
     alone = torch.empty(600, N, device="cuda")
     for first in range(0, 600, 16):
         ops.linear(x[first : first + 16], w, alone[first : first + 16])
-    assert bool(((alone.double() - exact).abs() <= bound).all())
+    assert bool(((alone.double() - exact).abs() <= bound).all()) and _error(alone, x, w) <= _parts_limit(K)
     for M in (17, 63, 127, 128, 129, 256, 257, 600):
         got = torch.full((M, N), float("nan"), device="cuda")
         ops.linear(x[:M], w, got)
