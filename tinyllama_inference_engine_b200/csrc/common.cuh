@@ -28,6 +28,12 @@ __device__ __forceinline__ float from_float<float>(float v) { return v; }
 template <>
 __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
+// Two numbers rounded to bfloat16, the first in the lower half.
+__device__ __forceinline__ uint32_t pack_bf16(float low, float high) {
+  __nv_bfloat162 v = __floats2bfloat162_rn(low, high);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+
 // 2^x in one instruction (ex2.approx: relative error about 2^-22, results below 2^-126 become zero, 2^-inf = 0).  exp2f()
 // without fast-math wraps the same instruction in a rescaling for denormal results, which a softmax weight does not need;
 // in the attention kernels' inner loops that wrapper was a third of the instructions per score.

@@ -31,6 +31,7 @@
 // Parts of numbers below 2^-102 (their last bits), and products of parts where the operands' product is below 2^-98, leave the range of normal numbers; what a term loses then is at
 // most 2^-124 of the largest operand, or 2^-123.  So an output is also worked out again where its rows of x and w hold such numbers (other than zeros) and it is below
 // K * 2^-98 * max(1, largest operand), 2^25 times what it may have lost.  Both are properties of the output and its two rows, whatever kernel and tile it is in.
+#include "mma_utils.cuh"
 #include "shared_memory_limit.cuh"
 #define TLIE_WITHOUT_TENSOR_MAPS
 #include "tcgen05_utils.cuh"
@@ -74,16 +75,17 @@ __device__ __forceinline__ float4 load_four(const float* row, int k, int K) {
   return v;
 }
 
-// Asynchronous copies into shared memory; nothing is read and zeros arrive where `valid` is not set.
-__device__ __forceinline__ void cp_async_16(void* to, const void* from, bool valid) {
+// Asynchronous copies into shared memory; nothing is read and zeros arrive where `valid` is not set.  Unlike those of mma_utils.cuh they hold the compiler to their place among plain reads and
+// writes of shared memory: a thread reads what it copied itself, without a barrier between.
+__device__ __forceinline__ void copy_16(void* to, const void* from, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(to)), "l"(from), "r"(valid ? 16 : 0) : "memory");
 }
-__device__ __forceinline__ void cp_async_4(void* to, const void* from, bool valid) {
+__device__ __forceinline__ void copy_4(void* to, const void* from, bool valid) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(smem_u32(to)), "l"(from), "r"(valid ? 4 : 0) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void copies_sent() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
-__device__ __forceinline__ void cp_async_wait() {
+__device__ __forceinline__ void wait_for_copies() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
@@ -158,17 +160,17 @@ __device__ __forceinline__ void sums_in_order(float (&sum)[TM][TN], const Tile& 
       const int r = at / (STEP / kWide), within = at % (STEP / kWide) * kWide, k = step * STEP + within;
       const float* row = r < TM * ROWS ? t.x + min(t.m0 + r, t.M - 1) * t.lda : t.w + (long long)min(t.n0 + r - TM * ROWS, t.N - 1) * t.K;
       if (ALIGNED) {
-        cp_async_16(stage + r * kStride + within, k < t.K ? row + k : row, k < t.K);
+        copy_16(stage + r * kStride + within, k < t.K ? row + k : row, k < t.K);
       } else {
-        cp_async_4(stage + r * kStride + within, k < t.K ? row + k : row, k < t.K);
+        copy_4(stage + r * kStride + within, k < t.K ? row + k : row, k < t.K);
       }
     }
-    cp_async_commit();
+    copies_sent();
   };
   const int steps = (t.K + STEP - 1) / STEP;
   copy(0);
   for (int step = 0; step < steps; ++step) {
-    cp_async_wait<0>();
+    wait_for_copies<0>();
     __syncwarp();
     barrier_of<BARRIER, THREADS>();   // this step's columns are here for every thread, and everyone is done with the other stage
     if (step + 1 < steps) copy(step + 1);
@@ -286,15 +288,10 @@ constexpr int kFewRows = 16;        // rows of w of a CTA
 constexpr int kFewAhead = 2;        // chunks of w on their way to a warp
 constexpr int kFewRound = 96;       // chunks whose sums are in shared memory at a time
 
-__device__ __forceinline__ void mma_16x8x16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-
 // NT: blocks of 8 rows of x.  A lane (g = lane / 4, t = lane % 4) holds rows g and g + 8 of w and row g of every block of x, k 4 t ... 4 t + 3 of every 16.
-// WARPS: sixteen where a CTA has its SM to itself, eight where two share one.  A lane copies what it will read itself (w of two chunks ahead, whichever tile they belong to), so a warp's
-// ring needs no barrier, and an SM has 128 KB on its way from HBM (with the next chunk on its way to registers it was half of that: 11,264 x 2,048 24.5 us, 2,048 x 5,632 13).
+// A lane copies what it will read itself (w of two chunks ahead, whichever tile they belong to), so a warp's ring needs no barrier.  WARPS: with one block sixteen where a CTA has its SM to
+// itself and eight where two share one, 128 KB an SM on their way from HBM (with the next chunk on its way to registers it was half of that: 11,264 x 2,048 24.5 us, 2,048 x 5,632 13); with
+// two blocks eight, 64 KB: registers hold no more.
 // A CTA walks row tiles blockIdx.x, + gridDim.x, ...  SHORT: a row has so few chunks that the warps take those of `together` tiles at a time (one tile after the other,
 // one to four warps of eight worked: K = 64, 16 rows x 11,264 5.6 -> 4.2 us, 128 x 2,048 8.2 -> 4.7, 600 x 256 6.4 -> 4.1).
 template <int NT, int WARPS, bool ALIGNED, bool SHORT>
@@ -334,17 +331,17 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gem
           const int k = ask_chunk * kChunkK + 16 * s + 4 * t;
           float4* place = mine + (slot * 8 + r * 4 + s) * 32;
           if (ALIGNED) {
-            cp_async_16(place, k < K ? row + k : row, k < K);
+            copy_16(place, k < K ? row + k : row, k < K);
           } else {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) cp_async_4(reinterpret_cast<float*>(place) + e, k + e < K ? row + k + e : row, k + e < K);
+            for (int e = 0; e < 4; ++e) copy_4(reinterpret_cast<float*>(place) + e, k + e < K ? row + k + e : row, k + e < K);
           }
         }
       }
       ask_chunk += WARPS;
       if (ask_chunk >= chunks) ask_chunk = own_chunk, ask_tile += stride;
     }
-    cp_async_commit();
+    copies_sent();
   };
   float4 xv[NT][4];
   auto load_x = [&](int chunk) {
@@ -367,7 +364,7 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gem
       for (int c = first + warp; c < end; c += WARPS) {
         float acc[NT][4];
         uint32_t wh[4][4], xh[NT][4][2];
-        cp_async_wait<kFewAhead - 1>();
+        wait_for_copies<kFewAhead - 1>();
         float4 wv[2][4];
 #pragma unroll
         for (int r = 0; r < 2; ++r)
@@ -396,18 +393,18 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gem
           }
 #pragma unroll
           for (int j = 0; j < NT; ++j) {
-            mma_16x8x16(acc[j], wh[s], xl[j]);
-            mma_16x8x16(acc[j], wl, xh[j][s]);
-            mma_16x8x16(acc[j], wm, xm[j]);
-            mma_16x8x16(acc[j], wh[s], xm[j]);
-            mma_16x8x16(acc[j], wm, xh[j][s]);
+            mma_bf16(acc[j], wh[s], xl[j][0], xl[j][1]);
+            mma_bf16(acc[j], wl, xh[j][s][0], xh[j][s][1]);
+            mma_bf16(acc[j], wm, xm[j][0], xm[j][1]);
+            mma_bf16(acc[j], wh[s], xm[j][0], xm[j][1]);
+            mma_bf16(acc[j], wm, xh[j][s][0], xh[j][s][1]);
           }
         }
         if (!SHORT) load_x(c + WARPS < chunks ? c + WARPS : own_chunk);   // of the next chunk, or of the next tile's first one
 #pragma unroll
         for (int s = 0; s < 4; ++s)
 #pragma unroll
-          for (int j = 0; j < NT; ++j) mma_16x8x16(acc[j], wh[s], xh[j][s]);
+          for (int j = 0; j < NT; ++j) mma_bf16(acc[j], wh[s], xh[j][s][0], xh[j][s][1]);
         float* to = sums + (c - first) * kOutputs;
 #pragma unroll
         for (int j = 0; j < NT; ++j) {
@@ -439,7 +436,7 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gem
         if (threadIdx.x < kOutputs && m < M && n < N) out[(size_t)m * N + n] = total;
         continue;
       }
-      cp_async_wait<0>();   // the ring is put to another use; what was on its way is asked for again
+      wait_for_copies<0>();   // the ring is put to another use; what was on its way is asked for again
       const bool large = __syncthreads_or(squares_are_large(squares));
       Tile* here = reinterpret_cast<Tile*>(ring);
       float* values = ring + sizeof(Tile) / sizeof(float);
@@ -454,7 +451,7 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 && WARPS == 8 ? 2 : 1) gem
       for (int s = 0; s < kFewAhead; ++s) ask(s);
     }
   }
-  cp_async_wait<0>();
+  wait_for_copies<0>();
 }
 
 // With 4-byte copies, which go through L1, a kernel starts only once the one before it is done.
@@ -612,10 +609,10 @@ __global__ void __launch_bounds__(kManyThreads, 1) gemm_many_f32_kernel(const fl
         const float* row = row_of(i);
         float4* place = places + i * (kCutWarps * 32);
         if (ALIGNED) {
-          cp_async_16(place, k < K ? row + k : row, k < K);
+          copy_16(place, k < K ? row + k : row, k < K);
         } else {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) cp_async_4(reinterpret_cast<float*>(place) + e, k + e < K ? row + k + e : row, k + e < K);
+          for (int e = 0; e < 4; ++e) copy_4(reinterpret_cast<float*>(place) + e, k + e < K ? row + k + e : row, k + e < K);
         }
       }
     };
@@ -627,7 +624,7 @@ __global__ void __launch_bounds__(kManyThreads, 1) gemm_many_f32_kernel(const fl
     for (int g = 0; g < kBatches; ++g) {
 #pragma unroll
       for (int i = 0; i < kBatch; ++i) ask(0, g * kBatch + i);
-      cp_async_commit();
+      copies_sent();
     }
     for (int c = 0; c < chunks; ++c) {
       const int s = c % kManyStages;
@@ -635,13 +632,13 @@ __global__ void __launch_bounds__(kManyThreads, 1) gemm_many_f32_kernel(const fl
       uint8_t* stage = ring + s * Shape::kStage + to;
 #pragma unroll
       for (int g = 0; g < kBatches; ++g) {
-        cp_async_wait<kBatches - 1>();   // the oldest of the groups on their way is this one
+        wait_for_copies<kBatches - 1>();   // the oldest of the groups on their way is this one
         float4 v[kBatch];
 #pragma unroll
         for (int i = 0; i < kBatch; ++i) v[i] = places[(g * kBatch + i) * (kCutWarps * 32)];
 #pragma unroll
         for (int i = 0; i < kBatch; ++i) ask(c + 1, g * kBatch + i);
-        cp_async_commit();
+        copies_sent();
 #pragma unroll
         for (int i = 0; i < kBatch; ++i) {
           constexpr int kXFours = kBM / 16;
@@ -663,7 +660,7 @@ __global__ void __launch_bounds__(kManyThreads, 1) gemm_many_f32_kernel(const fl
       __syncwarp();
       if (lane == 0) mbar_arrive(&full[s]);
     }
-    cp_async_wait<0>();
+    wait_for_copies<0>();
     if (squares_are_large(squares)) atomicOr(large, 1u);
     __syncwarp();
     asm volatile("bar.arrive 1, %0;\n" ::"n"((kCutWarps + kAddWarps) * 32) : "memory");   // (of the word above, to the adding warps)

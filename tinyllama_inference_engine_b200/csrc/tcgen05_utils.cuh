@@ -160,10 +160,6 @@ __device__ __forceinline__ float silu_gated(uint32_t gate_bits, uint32_t up_bits
   const float u = __bfloat162float(__float2bfloat16_rn(__uint_as_float(up_bits)));
   return (g / (1.0f + expf(-g))) * u;
 }
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&p);
-}
 
 // Staged: EPI 0 (bfloat16 out) or 2 (gated).  tmem_acc: the accumulator with this warp's lane offset; row0: the warp's first
 // row; n0: the tile's first output column; staging: this warp's BUFFERS boxes (1024-byte aligned); boxes: running count.
